@@ -309,6 +309,13 @@ int launch_nl_kernels(const Dev &d, cudaStream_t s, int grid_nodes, int grid_til
 }
 constexpr int NL_LAUNCHES = 8;
 
+// Centre-of-mass correction: every instance's centre, then the shift.
+void launch_com(const Dev &d, cudaStream_t s, int grid, const Prof &pf = Prof())
+{
+    k_com_centre<<<d.n_inst, 256, 0, s>>>(d); pf.mark(s, "com_centre");
+    k_com_shift<<<grid, SLOTS, 0, s>>>(d); pf.mark(s, "com_shift");
+}
+
 int launch_nl_build(cs3d_ctx *c, const Prof &pf = Prof())
 {
     return launch_nl_kernels(c->d, c->stream, c->grid_nodes, c->grid_tiles, pf);
@@ -332,7 +339,7 @@ int run_init(cs3d_ctx *c)
     k_geom<<<c->grid_cells, SLOTS, 0, s>>>(d, 0);
     // correct_com at set-up (src/GPUbounce.cu:785-805): after the first grid,
     // before the first force evaluation
-    if (c->any_com) k_com_shift<<<c->n_inst, 256, 0, s>>>(d);
+    if (c->any_com) launch_com(d, s, c->grid_s2);
     CK(cudaGetLastError());
     int rc = launch_nl_build(c);
     if (rc) return rc;
@@ -378,7 +385,7 @@ int launch_step(cs3d_ctx *c, int par, bool div, bool k1 = true, int fuse = 0, co
         if (fuse) { k_integrate_divided<<<c->grid_cells, SLOTS, 0, s>>>(d); ++n; pf.mark(s, "integrate_divided"); }
     }
     if (soften) { k_soften<<<c->n_inst, 32, 0, s>>>(d, (int)soften); ++n; pf.mark(s, "soften"); }
-    if (c->any_com) { k_com_shift<<<c->n_inst, 256, 0, s>>>(d); ++n; pf.mark(s, "com_shift"); }
+    if (c->any_com) { launch_com(d, s, c->grid_s2, pf); n += 2; }
     CK(cudaGetLastError());
     c->launches_per_step = n;
     return CS3D_OK;
@@ -1403,7 +1410,7 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     k_geom<<<sd->grid_cells, SLOTS, 0, s>>>(d, 0);
     // correct_com at set-up, as run_init (src/GPUbounce.cu:785-805): the shift
     // moves the positions the wall and contact forces see
-    if (params->correct_com) k_com_shift<<<1, 256, 0, s>>>(d);
+    if (params->correct_com) launch_com(d, s, sd->grid_cells);
     if ((rc = launch_nl_kernels(d, s, sd->grid_nodes, sd->grid_tiles))) return rc;
     k_s1<true><<<sd->grid_cells, SLOTS, sizeof(S1Smem), s>>>(d, 0);
     k_static_store<<<sd->grid_flat, 256, 0, s>>>(d, n_cells, FCX, FCY, FCZ, FDX, FDY, FDZ);

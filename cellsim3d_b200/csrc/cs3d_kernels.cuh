@@ -1320,35 +1320,56 @@ __global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par)
 // host loop does; a daughter's entry is still 0 in its first step) is
 // subtracted from every node.  The centres of mass, boxes and grid of this
 // step keep their unshifted values, as in the reference; the list anchors
-// move with the nodes (a uniform shift changes no distance).  One block per
-// instance.
-__global__ void __launch_bounds__(256) k_com_shift(Dev d)
+// move with the nodes (a uniform shift changes no distance).
+//
+// The order of the sum makes it a chain of n dependent float additions per
+// component.  The block stages the centres in shared memory, so the chain
+// waits for shared memory and the adder only; three threads take one
+// component each.  One block per instance.
+template <int NT>
+__device__ __forceinline__ void com_centre(const Dev &d, int k, float (*stage)[NT])
 {
-    const int k = blockIdx.x;
-    if (k >= d.n_inst) return;
     const InstParams &P = d.prm[k];
-    if (!P.correct_com) return;
-    __shared__ float sys[3];
-    const int n = d.st[k].n;
-    if (threadIdx.x == 0) {
-        float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-        for (int c = 0; c < n; ++c) {
-            const float4 cm = d.CM[P.base + c];
-            sx = __fadd_rn(sx, cm.x);
-            sy = __fadd_rn(sy, cm.y);
-            sz = __fadd_rn(sz, cm.z);
+    if (!P.correct_com) return;   // uniform
+    const int n = d.st[k].n, t = threadIdx.x;
+    float s = 0.0f;
+    for (int c0 = 0; c0 < n; c0 += NT) {
+        __syncthreads();
+        if (c0 + t < n) {
+            const float4 cm = d.CM[P.base + c0 + t];
+            stage[0][t] = cm.x; stage[1][t] = cm.y; stage[2][t] = cm.z;
         }
-        sys[0] = __fdiv_rn(sx, (float)n);
-        sys[1] = __fdiv_rn(sy, (float)n);
-        sys[2] = __fdiv_rn(sz, (float)n);
-        d.st[k].syscm[0] = sys[0];
-        d.st[k].syscm[1] = sys[1];
-        d.st[k].syscm[2] = sys[2];
+        __syncthreads();
+        const int m = n - c0 < NT ? n - c0 : NT;
+        if (t < 3) {
+            const float *p = stage[t];
+#pragma unroll 8
+            for (int c = 0; c < m; ++c) s = __fadd_rn(s, p[c]);
+        }
     }
-    __syncthreads();
-    const float ox = sys[0], oy = sys[1], oz = sys[2];
-    for (int q = threadIdx.x; q < n * SLOTS; q += blockDim.x) {
-        const size_t g = (size_t)P.base * SLOTS + q;
+    if (t < 3) d.st[k].syscm[t] = __fdiv_rn(s, (float)n);
+}
+
+__global__ void __launch_bounds__(256) k_com_centre(Dev d)
+{
+    __shared__ float stage[3][256];
+    if ((int)blockIdx.x < d.n_inst) com_centre<256>(d, blockIdx.x, stage);
+}
+
+// The shift of the nodes and their anchors, all 192 slots of a cell: a stream
+// over the active cells, bound by memory (64 B a node).  One block per
+// instance took 300 us a step at 1023 cells, with the centre's sum from
+// global memory.
+__global__ void __launch_bounds__(SLOTS) k_com_shift(Dev d)
+{
+    const int W = n_work(d);
+    for (int w = blockIdx.x; w < W; w += gridDim.x) {
+        const int a = cell_of(d, w);
+        const int inst = inst_of(d, a);
+        if (!d.prm[inst].correct_com) continue;
+        const float *o = d.st[inst].syscm;
+        const float ox = o[0], oy = o[1], oz = o[2];
+        const size_t g = (size_t)a * SLOTS + threadIdx.x;
         float4 x = d.X[g], b = d.Xb[g];
         x.x = __fsub_rn(x.x, ox); x.y = __fsub_rn(x.y, oy); x.z = __fsub_rn(x.z, oz);
         b.x = __fsub_rn(b.x, ox); b.y = __fsub_rn(b.y, oy); b.z = __fsub_rn(b.z, oz);
