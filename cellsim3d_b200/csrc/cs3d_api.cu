@@ -41,8 +41,8 @@ struct cs3d_ctx {
     float skin = 0.1f;
     int grid_cells = 0;            // blocks of the per-cell kernels
     int grid_flat = 0;             // blocks of the per-thread kernels
-    int grid_nodes = 0;            // blocks of the neighbour-list kernels
-    int grid_tiles = 0;            // blocks of the bucket scan
+    int grid_lists = 0;            // blocks of the neighbour lists
+    int grid_boxes = 0;            // blocks of the cell boxes (a warp per cell)
     int grid_s2 = 0;               // blocks of S2 and the integrator
     cudaGraphExec_t graph[2][2][2][3] = {};  // [parity][division][integrate first][S2 mode: 0, fused 1, fused last 2]
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -112,9 +112,51 @@ struct TopoTables {
     float4 r0[SLOTS], th[SLOTS];
     uint4 arm[SLOTS];
     uint8_t faces[CS3D_FACES * 7];
+    uint8_t patch[SLOTS];
     double2 cs0[3 * SLOTS];
     double r0i[3 * SLOTS];
 };
+
+// Nodes m[0 .. n) in the order of their distance along the bonds (within the
+// set) from its most outlying node.
+void order_along(const cs3d_topology *t, int *m, int n)
+{
+    int start = m[0];
+    std::vector<int> q;
+    for (int pass = 0; pass < 3; ++pass) {   // the last node of a search starts the next
+        std::vector<char> left(NODES, 0);
+        for (int k = 0; k < n; ++k) left[m[k]] = 1;
+        q.assign(1, start);
+        left[start] = 0;
+        for (size_t k = 0; (int)q.size() < n; ++k) {
+            if (k == q.size()) {   // a part without a bond to the rest
+                const int i = (int)(std::find(left.begin(), left.end(), 1) - left.begin());
+                left[i] = 0;
+                q.push_back(i);
+            }
+            for (int b = 0; b < 3; ++b) {
+                const int j = t->nn[b * 192 + q[k]];
+                if (left[j]) { left[j] = 0; q.push_back(j); }
+            }
+        }
+        start = q.back();
+    }
+    std::copy(q.begin(), q.end(), m);
+}
+
+// Six patches of 30 neighbouring nodes, one for each warp of a CTA: the mesh
+// cut in two, each half in three, across its longest way.
+void node_patches(const cs3d_topology *t, uint8_t *patch)
+{
+    int m[NODES];
+    for (int i = 0; i < NODES; ++i) m[i] = i;
+    order_along(t, m, NODES);
+    order_along(t, m, NODES / 2);
+    order_along(t, m + NODES / 2, NODES / 2);
+    constexpr int PER = NODES / (SLOTS / 32);
+    memset(patch, 0xff, SLOTS);
+    for (int i = 0; i < NODES; ++i) patch[32 * (i / PER) + i % PER] = (uint8_t)m[i];
+}
 
 int topo_tables(const cs3d_topology *t, TopoTables &o)
 {
@@ -150,6 +192,7 @@ int topo_tables(const cs3d_topology *t, TopoTables &o)
         if (t->faces[f] < 0 || t->faces[f] >= NODES) return CS3D_E_ARG;
         o.faces[f] = (uint8_t)t->faces[f];
     }
+    node_patches(t, o.patch);
     return CS3D_OK;
 }
 
@@ -166,6 +209,7 @@ int upload_topology(cs3d_ctx *c, const cs3d_topology *t)
     if ((rc = dalloc(c, &T.th0, SLOTS))) return rc;
     if ((rc = dalloc(c, &T.arm, SLOTS))) return rc;
     if ((rc = dalloc(c, &T.faces, CS3D_FACES * 7))) return rc;
+    if ((rc = dalloc(c, &T.patch, SLOTS))) return rc;
     CK(cudaMemcpyAsync(T.cs0, tt.cs0, sizeof tt.cs0, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.r0i, tt.r0i, sizeof tt.r0i, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.nnpack, tt.nnp, sizeof tt.nnp, cudaMemcpyHostToDevice, c->stream));
@@ -173,12 +217,13 @@ int upload_topology(cs3d_ctx *c, const cs3d_topology *t)
     CK(cudaMemcpyAsync(T.th0, tt.th, sizeof tt.th, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.arm, tt.arm, sizeof tt.arm, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.faces, tt.faces, sizeof tt.faces, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(T.patch, tt.patch, sizeof tt.patch, cudaMemcpyHostToDevice, c->stream));
     // the host tables go out of scope: the copies must have completed
     CK(cudaStreamSynchronize(c->stream));
     return CS3D_OK;
 }
 
-InstParams make_inst(const cs3d_params &p, int base, int cap, float skin)
+InstParams make_inst(const cs3d_params &p, int base, int cap, float skin, float inv_bin)
 {
     InstParams q{};
     q.mass = p.particle_mass;
@@ -209,6 +254,7 @@ InstParams make_inst(const cs3d_params &p, int base, int cap, float skin)
     q.skin = skin;
     q.skin_base = skin;
     q.rlist = p.attraction_range + skin;
+    q.inv_bin = inv_bin;
     q.check_sph = p.check_sphericity;
     q.angles = p.constrain_angles;
     q.rigid = p.use_rigid_box;
@@ -291,23 +337,17 @@ struct Prof {
     }
 };
 
-// Neighbour-list build: spatial hash of the nodes (counting sort by
-// bucket), then the per-cell lists.  Every kernel returns at once when no
-// instance rebuilds this step.
-int launch_nl_kernels(const Dev &d, cudaStream_t s, int grid_nodes, int grid_tiles, const Prof &pf = Prof())
+// Neighbour-list build: the cells' boxes and table, then the per-cell lists.
+// Both kernels return at once when no instance rebuilds this step.
+int launch_nl_kernels(const Dev &d, cudaStream_t s, int grid_lists, int grid_boxes, const Prof &pf = Prof())
 {
-    k_nh_zero<<<grid_tiles, 256, 0, s>>>(d); pf.mark(s, "nh_zero");
-    k_nh_count<<<grid_nodes, SLOTS, 0, s>>>(d); pf.mark(s, "nh_count");
-    k_nh_scan_tiles<<<grid_tiles, 256, 0, s>>>(d); pf.mark(s, "nh_scan_tiles");
-    k_nh_scan_top<<<1, 1024, 0, s>>>(d); pf.mark(s, "nh_scan_top");
-    k_nh_scan_apply<<<grid_tiles, 256, 0, s>>>(d); pf.mark(s, "nh_scan_apply");
-    k_nh_fill<<<grid_nodes, SLOTS, 0, s>>>(d); pf.mark(s, "nh_fill");
-    k_nl_cell<<<grid_nodes, SLOTS, 0, s>>>(d, 0); pf.mark(s, "nl_cell");
-    k_nl_cell<<<grid_nodes, SLOTS, 0, s>>>(d, 1); pf.mark(s, "nl_cell_nbr");
+    k_nb_boxes<<<grid_boxes, SLOTS, 0, s>>>(d); pf.mark(s, "nb_boxes");
+    k_nb_mark<<<grid_boxes, SLOTS, 0, s>>>(d); pf.mark(s, "nb_mark");
+    k_nb_lists<<<grid_lists, SLOTS, 0, s>>>(d); pf.mark(s, "nb_lists");
     CK(cudaGetLastError());
     return CS3D_OK;
 }
-constexpr int NL_LAUNCHES = 8;
+constexpr int NL_LAUNCHES = 3;
 
 // Centre-of-mass correction: every instance's centre, then the shift.
 void launch_com(const Dev &d, cudaStream_t s, int grid, const Prof &pf = Prof())
@@ -318,16 +358,26 @@ void launch_com(const Dev &d, cudaStream_t s, int grid, const Prof &pf = Prof())
 
 int launch_nl_build(cs3d_ctx *c, const Prof &pf = Prof())
 {
-    return launch_nl_kernels(c->d, c->stream, c->grid_nodes, c->grid_tiles, pf);
+    return launch_nl_kernels(c->d, c->stream, c->grid_lists, c->grid_boxes, pf);
 }
 
-// Buckets of the node hash for a capacity of `cells` cells.
-constexpr int hash_size(long long cells)
+// Bins of the list build's cell table for a capacity of `cells` cells.
+constexpr int table_size(long long cells)
 {
-    long long n = std::max<long long>(cells * SLOTS, SCAN_TILE);
-    int h = SCAN_TILE;
-    while (h < n) h <<= 1;
+    int h = 64;
+    while (h < 2 * cells) h <<= 1;
     return h;
+}
+
+// Bin edge of the cell table: six mean bond lengths, about two thirds of a
+// cell's diameter.  The box of a cell then has some five bins in reach along
+// each axis, one for every thread of its CTA, and a bin seldom holds two cells.
+float inv_bin_edge(const cs3d_topology *t)
+{
+    double sum = 0.0;
+    for (int k = 0; k < 3; ++k)
+        for (int i = 0; i < NODES; ++i) sum += t->r0[k * 192 + i];
+    return (float)(3.0 * NODES / (6.0 * sum));
 }
 
 int run_init(cs3d_ctx *c)
@@ -494,7 +544,7 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
         total += capacity[k];
     }
     if (total > (1 << 23)) return CS3D_E_ARG;  // cell ids are packed in 24 bits for pair records
-    if (total * SLOTS * 2 > (1ll << 31) - SCAN_TILE) return CS3D_E_ARG;  // int bucket offsets of the node hash
+    if (total * SLOTS * 2 > (1ll << 31) - 4096) return CS3D_E_ARG;  // node indices are ints
     cs3d_ctx *c = new (std::nothrow) cs3d_ctx();
     if (!c) return CS3D_E_NOMEM;
     c->device = device;
@@ -509,8 +559,9 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     c->cap_total = (int)total;
     c->hn.assign(n_inst, 0);
     int base = 0;
+    const float inv_bin = inv_bin_edge(topo);
     for (int k = 0; k < n_inst; ++k) {
-        c->hprm.push_back(make_inst(params[k], base, capacity[k], c->skin));
+        c->hprm.push_back(make_inst(params[k], base, capacity[k], c->skin, inv_bin));
         base += capacity[k];
         if (params[k].growth_rate > 0) c->any_growth = true;
         if (params[k].correct_com) c->any_com = true;
@@ -541,13 +592,14 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     AL(d.cell_inst, c->cap_total);
     AL(d.work, c->cap_total); AL(d.work_n, 1);
     AL(d.cand, (size_t)c->cap_total * MAXC); AL(d.ncand, c->cap_total);
-    AL(d.dlist, (size_t)c->cap_total * MAXD * SLOTS); AL(d.ndis, nodes); AL(d.dirty, c->cap_total);
+    AL(d.dlist, (size_t)c->cap_total * MAXD * SLOTS); AL(d.ndis, nodes);
     AL(d.Xb, nodes);
     AL(d.ent, (size_t)c->cap_total * MAXE * SLOTS); AL(d.nent, nodes);
-    d.hsize = hash_size(2ll * c->cap_total);  // slices: a power of two >= nodes per instance
-    AL(d.hcount, (size_t)d.hsize + SCAN_TILE); AL(d.hscan, (size_t)d.hsize / SCAN_TILE + 1); AL(d.hsz, 1);
-    AL(d.hpos, nodes); AL(d.node_rank, nodes);
-    AL(d.divtab, c->cap_total); AL(d.div_total, 1);
+    size_t bins = 0;
+    for (int k = 0; k < n_inst; ++k) bins += (size_t)table_size(capacity[k]);
+    AL(d.nbox, 2 * (size_t)c->cap_total); AL(d.bins, bins); AL(d.bnext, c->cap_total); AL(d.epoch, 1);
+    AL(d.cdisp, c->cap_total); AL(d.build, c->cap_total); AL(d.n_build, 1); AL(d.mark, c->cap_total);
+    AL(d.divtab, c->cap_total); AL(d.div_total, 1); AL(d.div_prev, 1);
     d.ev_cap = std::max(1 << 16, 2 * c->cap_total);
     AL(d.events, d.ev_cap); AL(d.n_events, 1);
     d.far_cap = d.ev_cap;
@@ -588,9 +640,9 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     c->grid_cells = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ, 1)));
     c->grid_flat = std::max(1, std::min((c->cap_total + 255) / 256 + 1, c->nsm * 8));
     int occ_nl = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_nl, k_nl_cell, SLOTS, 0);
-    c->grid_nodes = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ_nl, 1)));
-    c->grid_tiles = std::max(1, std::min(d.hsize / SCAN_TILE + 1, c->nsm * 8));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_nl, k_nb_lists, SLOTS, 0);
+    c->grid_lists = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ_nl, 1)));
+    c->grid_boxes = std::max(1, std::min((c->cap_total + NBW - 1) / NBW, c->nsm * 8));
     int occ_s2 = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s2, k_s2<true, 0>, SLOTS, 0);
     c->grid_s2 = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ_s2, 1)));
@@ -1208,7 +1260,7 @@ int cs3d_get_stats(cs3d_ctx *c, long long *stats, int n)
 namespace {
 
 constexpr int SCAP = CS3D_STATIC_MAX_CELLS;
-constexpr int SHASH = hash_size(2 * SCAP);   // bucket rule of cs3d_create_ensemble
+constexpr int SBINS = table_size(SCAP);
 constexpr int SEVENTS = 16;
 
 struct StaticScratch {
@@ -1220,18 +1272,21 @@ struct StaticScratch {
     float press[SCAP], E[SCAP], vol[SCAP], area[SCAP];
     uint8_t divflag[SCAP];
     float4 aabb0[2 * SCAP], aabb1[2 * SCAP];
-    float4 hpos[SCAP * SLOTS];
-    alignas(16) int hcount[SHASH + SCAN_TILE];
-    int hscan[SHASH / SCAN_TILE + 1], node_rank[SCAP * SLOTS], hsz;
+    float4 nbox[2 * SCAP];
+    unsigned long long bins[SBINS];
+    int bnext[SCAP];
+    unsigned epoch;
+    float cdisp[SCAP];
+    int build[SCAP], n_build;
+    uint8_t mark[SCAP];
     int cell_inst[SCAP], work[SCAP], work_n;
     int cand[SCAP * MAXC], ncand[SCAP];
     uint16_t dlist[SCAP * MAXD * SLOTS];
     uint8_t ndis[SCAP * SLOTS];
-    int dirty[SCAP];
     uint16_t ent[SCAP * MAXE * SLOTS];
     uint8_t nent[SCAP * SLOTS];
     DivEntry divtab[SCAP];
-    int div_total;
+    int div_total, div_prev;
     int4 events[SEVENTS];
     int n_events;
     int flags[4];
@@ -1240,7 +1295,7 @@ struct StaticScratch {
     uint32_t nnpack[SLOTS];
     float4 r0[SLOTS], th0[SLOTS];
     uint4 arm[SLOTS];
-    uint8_t faces[CS3D_FACES * 7];
+    uint8_t faces[CS3D_FACES * 7], patch[SLOTS];
     double2 cs0[3 * SLOTS];
     double r0i[3 * SLOTS];
 };
@@ -1253,7 +1308,7 @@ static __device__ __align__(256) unsigned char g_static_scratch[sizeof(StaticScr
 struct StaticDevice {
     bool ready = false;
     StaticScratch *base = nullptr;
-    int grid_cells = 1, grid_flat = 1, grid_nodes = 1, grid_tiles = 1;
+    int grid_cells = 1, grid_flat = 1, grid_lists = 1, grid_boxes = 1;
 };
 
 constexpr int kMaxDevices = 64;
@@ -1273,6 +1328,7 @@ Dev static_dev(StaticScratch *s)
     d.topo.th0 = s->th0;
     d.topo.arm = s->arm;
     d.topo.faces = s->faces;
+    d.topo.patch = s->patch;
     d.topo.cs0 = s->cs0;
     d.topo.r0i = s->r0i;
     d.X = s->X; d.V = s->V; d.Vb = s->Vb; d.FC = s->FC; d.FD = s->FD; d.Xb = s->Xb; d.FR = s->FR;
@@ -1282,10 +1338,11 @@ Dev static_dev(StaticScratch *s)
     d.aabb[0] = s->aabb0; d.aabb[1] = s->aabb1;
     d.cell_inst = s->cell_inst; d.work = s->work; d.work_n = &s->work_n;
     d.cand = s->cand; d.ncand = s->ncand;
-    d.dlist = s->dlist; d.ndis = s->ndis; d.dirty = s->dirty;
+    d.dlist = s->dlist; d.ndis = s->ndis;
     d.ent = s->ent; d.nent = s->nent;
-    d.hsize = SHASH; d.hsz = &s->hsz; d.hcount = s->hcount; d.hscan = s->hscan; d.hpos = s->hpos; d.node_rank = s->node_rank;
-    d.divtab = s->divtab; d.div_total = &s->div_total;
+    d.nbox = s->nbox; d.bins = s->bins; d.bnext = s->bnext; d.epoch = &s->epoch;
+    d.cdisp = s->cdisp; d.build = s->build; d.n_build = &s->n_build; d.mark = s->mark;
+    d.divtab = s->divtab; d.div_total = &s->div_total; d.div_prev = &s->div_prev;
     d.events = s->events; d.n_events = &s->n_events; d.ev_cap = SEVENTS;
     d.flags = s->flags;
     d.pairs = s->pairs; d.n_pairs = &s->n_pairs; d.pair_cap = 1; d.record_pairs = 0;
@@ -1350,8 +1407,8 @@ int static_setup(int dev, StaticDevice **out)
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_s1<true>, SLOTS, sizeof(S1Smem)));
         sd.grid_cells = std::max(1, std::min(SCAP, nsm * std::max(occ, 1)));
         sd.grid_flat = std::max(1, std::min((SCAP * SLOTS + 255) / 256, nsm * 8));
-        sd.grid_nodes = std::max(1, std::min(SCAP, nsm * 8));
-        sd.grid_tiles = std::max(1, std::min(SHASH / SCAN_TILE + 1, nsm * 8));
+        sd.grid_lists = std::max(1, std::min(SCAP, nsm * 8));
+        sd.grid_boxes = (SCAP + NBW - 1) / NBW;
         sd.ready = true;
     }
     *out = &sd;
@@ -1383,7 +1440,7 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     StaticScratch *S = sd->base;
     const Dev d = static_dev(S);
     // parameters, mesh tables and a cleared instance state
-    const InstParams ip = make_inst(*params, 0, SCAP, 0.1f);
+    const InstParams ip = make_inst(*params, 0, SCAP, 0.1f, inv_bin_edge(topo));
     InstState st0;
     memset(&st0, 0, sizeof st0);
     st0.n = n_cells;
@@ -1394,12 +1451,12 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     CK(cudaMemcpyAsync(S->th0, tt.th, sizeof tt.th, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(S->arm, tt.arm, sizeof tt.arm, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(S->faces, tt.faces, sizeof tt.faces, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(S->patch, tt.patch, sizeof tt.patch, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(S->cs0, tt.cs0, sizeof tt.cs0, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(S->r0i, tt.r0i, sizeof tt.r0i, cudaMemcpyHostToDevice, s));
     // the previous call's neighbour lists, boxes and flags must not leak in
     CK(cudaMemsetAsync(S->ncand, 0, sizeof S->ncand, s));
     CK(cudaMemsetAsync(S->nent, 0, sizeof S->nent, s));
-    CK(cudaMemsetAsync(S->dirty, 0, sizeof S->dirty, s));
     CK(cudaMemsetAsync(S->flags, 0, sizeof S->flags, s));
     CK(cudaMemsetAsync(&S->n_events, 0, sizeof S->n_events, s));
     k_static_load<<<sd->grid_flat, 256, 0, s>>>(d, n_cells, X, Y, Z, VX, VY, VZ, pressure, youngs, params->min_pressure,
@@ -1411,7 +1468,7 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     // correct_com at set-up, as run_init (src/GPUbounce.cu:785-805): the shift
     // moves the positions the wall and contact forces see
     if (params->correct_com) launch_com(d, s, sd->grid_cells);
-    if ((rc = launch_nl_kernels(d, s, sd->grid_nodes, sd->grid_tiles))) return rc;
+    if ((rc = launch_nl_kernels(d, s, sd->grid_lists, sd->grid_boxes))) return rc;
     k_s1<true><<<sd->grid_cells, SLOTS, sizeof(S1Smem), s>>>(d, 0);
     k_static_store<<<sd->grid_flat, 256, 0, s>>>(d, n_cells, FCX, FCY, FCZ, FDX, FDY, FDZ);
     CK(cudaGetLastError());

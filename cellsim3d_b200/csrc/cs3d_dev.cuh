@@ -13,7 +13,6 @@ constexpr int NODES = CS3D_NODES;      // real nodes per cell
 constexpr int MAXC = CS3D_MAX_CAND;    // contact-candidate cells per cell
 constexpr int MAXE = CS3D_MAX_ENTRIES; // contact-candidate nodes per node
 constexpr int MAXD = CS3D_MAX_DIS;     // dissipative pairs per node
-constexpr int SCAN_TILE = 4096;        // elements per block of the bucket scan
 constexpr float DL = 2.9f;             // reference grid spacing, src/GPUbounce.cu:756
 
 // Per-instance constants (uploaded once).
@@ -27,6 +26,7 @@ struct InstParams {
     float rsE;      // fl(rs*E), repulsion coefficient
     float wallk;    // fl(100*E), rigid-box wall stiffness, src/propagate.cu:481
     float rlist;    // neighbour-list radius (ra + skin)
+    float inv_bin;  // 1 / bin edge of the list build's cell table
     float skin;     // skin in use (set by the device from the schedule)
     float skin_base;            // the context's skin (CS3D_OPT_SKIN)
     int sk_n;                   // skin schedule by population: ranges in use
@@ -56,14 +56,15 @@ struct InstState {
     int step;              // number of the step in progress / last finished
     unsigned err;          // CS3D_ERRBIT_*
     int rebuild;           // list rebuild this step: 0 none, 1 around divisions, 2 whole instance
-    float rcur;            // list radius of this step's build
+    float ds;              // largest node distance from its anchor before this step's build (0 at whole builds)
     int mm[2][6];          // grid extents (ordered-int min/max) by step parity
     unsigned disp_step;    // max node displacement of the current step (float bits)
     int div_count;         // divisions in the current step
     int force_rebuild;
     int max_entries, max_cand, max_halo;
-    unsigned hbase;        // first bucket of this instance's slice of the node hash
+    unsigned hbase;        // first bin of this instance's slice of the cell table
     int hbits;             // log2 of the slice size (0: not rebuilding)
+    unsigned hmax[3];      // largest half extent of its cells' boxes at this build (float bits)
     int built;             // cells whose lists were built (cumulative)
     int rebuilds;
     int rebuilds_div;      // of those, the ones only the rule for dividing instances called for
@@ -89,6 +90,7 @@ struct Topo {
     double *r0i;        // [192*3] 1/R0 in FP64
     uint4 *arm;         // [192] x, y, z: arm-force index n*3 + k for the three neighbours n
     uint8_t *faces;     // [92*7]
+    uint8_t *patch;     // [192] node of each thread: 30 neighbouring nodes to a warp (0xff: none)
 };
 
 // Pointers of a context (passed by value to every kernel).
@@ -116,7 +118,6 @@ struct Dev {
     int *cand;          // [cell*MAXC]
     int *ncand;         // [cell]
     float4 *Xb;         // anchors of the displacement test (positions at a build)
-    int *dirty;         // [cell] 1: divided last step, 2: within the list radius of such a cell
     // contact candidates of each node: slot << 8 | node, ascending, where
     // slot indexes the cell's candidate list (cand) and node the node in
     // that cell
@@ -126,16 +127,20 @@ struct Dev {
     // order), read by S2: positions do not change in between
     uint16_t *dlist;    // [(cell*MAXD + k)*192 + node]
     uint8_t *ndis;      // [cell*192 + node]
-    // node-level spatial hash of the neighbour-list build: cubic bins of
-    // edge ~rlist hashed (with the instance) into hsize buckets
-    int hsize;          // bucket capacity (>= twice the nodes of the capacity)
-    int *hsz;           // buckets in use by the current list build (whole scan tiles, <= hsize)
-    int *hcount;        // [hsize + SCAN_TILE] bucket counts, then exclusive starts
-    int *hscan;         // [hsize / SCAN_TILE + 1] tile sums of the scan
-    float4 *hpos;       // [cap_total*192] positions sorted by bucket, w = (cell << 8 | node) bits
-    int *node_rank;     // [cap_total*192] position of the node in its bucket
+    // the list build's boxes (current positions) and cell table: per bin the
+    // last cell put in (with the build's epoch in the high word), per cell the
+    // one put in before it
+    float4 *nbox;       // [2*cell] lo, hi
+    unsigned long long *bins;
+    int *bnext;         // [cell]
+    float *cdisp;       // [cell] largest distance of its nodes from their anchors
+    int *build;         // cells of this step's partial builds
+    int *n_build;
+    uint8_t *mark;      // [cell] of them: 1 near a divided cell, 2 divided
+    unsigned *epoch;
     DivEntry *divtab;
     int *div_total;
+    int *div_prev;      // divisions of the previous step (divtab)
     int4 *events;       // (inst, step, parent, daughter)
     int4 *farlog;       // (inst, step, far cells, 0) of the internal-cells mitotic count
     int *n_far;
@@ -143,7 +148,7 @@ struct Dev {
     uint8_t *pick;      // [cap_total + n_inst] flags of the random soft-cell picks
     int *n_events;
     int ev_cap;
-    int *flags;         // [0] any rebuild, [1] any division
+    int *flags;         // [0] any rebuild, [1] any division, [2] any whole-instance rebuild
     int4 *pairs;        // (cell_a<<8 | node_i, cell_b<<8 | node_j, kind, 0)
     unsigned long long *n_pairs;
     long long pair_cap;

@@ -515,6 +515,7 @@ __device__ __forceinline__ void integrate_cell(const Dev &d, int a, float *smax)
         if (i == 0) {
             float m = smax[0];
             for (int q = 1; q < SLOTS / 32; ++q) m = fmaxf(m, smax[q]);
+            d.cdisp[a] = m;
             atomicMax(&d.st[inst].disp_step, __float_as_uint(m));
         }
         __syncthreads();
@@ -545,10 +546,9 @@ __global__ void __launch_bounds__(SLOTS) k_integrate_divided(Dev d)
 // Per-step bookkeeping (one block): step counter, rebuild decision, reset of
 // the accumulators that this step fills.
 // ---------------------------------------------------------------------------
-// Hash slices of the list build: every rebuilding instance gets its own
-// power-of-two range of buckets (at least its node count), laid out back to
-// back; *d.hsz = their total rounded up to whole scan tiles.  Whole block
-// (256 threads), after the rebuild decisions.
+// Slices of the cell table of the list build: every rebuilding instance gets
+// its own power-of-two range of bins (at least twice its cells), laid out
+// back to back.  Whole block (256 threads), after the rebuild decisions.
 __device__ void assign_hash_slices(const Dev &d)
 {
     __shared__ int wsum[32];
@@ -563,7 +563,8 @@ __device__ void assign_hash_slices(const Dev &d)
             int bits = 0;
             if (st->rebuild) {
                 bits = 6;
-                while ((1ll << bits) < (long long)st->n * NODES) ++bits;
+                while ((1ll << bits) < 2ll * st->n) ++bits;
+                for (int q = 0; q < 3; ++q) st->hmax[q] = 0u;
                 size = 1 << bits;
             }
             st->hbits = bits;
@@ -574,30 +575,34 @@ __device__ void assign_hash_slices(const Dev &d)
         if (threadIdx.x == 0) carry += (unsigned)tot;
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        unsigned h = (carry + SCAN_TILE - 1) / SCAN_TILE * SCAN_TILE;
-        *d.hsz = (int)(h < (unsigned)SCAN_TILE ? (unsigned)SCAN_TILE : h);
-    }
+    if (threadIdx.x == 0) *d.epoch += 1u;   // empties the table
 }
 
 __global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
 {
-    __shared__ int any;
-    if (threadIdx.x == 0) { any = 0; *d.div_total = 0; }
+    __shared__ int any, any_full;
+    if (threadIdx.x == 0) {
+        any = any_full = 0;
+        *d.n_build = 0;
+        *d.div_prev = *d.div_total;   // the divisions the lists are rebuilt around
+        *d.div_total = 0;
+    }
     __syncthreads();
     for (int k = threadIdx.x; k < d.n_inst; k += blockDim.x) {
         InstState *st = &d.st[k];
         const InstParams &P = d.prm[k];
         st->step += 1;
         // ds: the largest distance of any node from its anchor (Xb, its
-        // position at a build).  Every list built at time tb with radius
-        // ra + skin + 2*ds(tb) stays complete while all nodes stay within
-        // skin/2 of their anchors: a pair within ra now was within
-        // ra + 2*(skin/2 + ds(tb)) at tb.  Whole-instance builds (ds reset
-        // to 0) use ra + skin; the 1e-3 slack covers float rounding.
-        // After divisions, only the divided cells (anchors reset) and the
-        // cells within the list radius of them are rebuilt, unless ds is
-        // already large.
+        // position at a build).  A list built at time tb stays complete
+        // while all nodes stay within skin/2 of their anchors, if it holds
+        // the pairs within ra + skin + D(a) + D(b), D the largest such
+        // distance at tb among the nodes of each of the two cells: a pair
+        // within ra now was within ra + (skin/2 + D(a)) + (skin/2 + D(b)) at
+        // tb.  Whole-instance builds (D reset to 0) use ra + skin; the 1e-3
+        // slack covers float rounding.  After divisions, only the divided
+        // cells (anchors reset) and the cells within the list radius of them
+        // are rebuilt, unless many cells divided: a division concerns some
+        // dozen cells, so that from one cell in 16 on most would be built.
         const float ds = __uint_as_float(st->disp_step);
         st->disp_step = 0u;
         if (P.sk_n > 0) {
@@ -614,16 +619,16 @@ __global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
             }
         }
         const bool by_disp = st->force_rebuild || !(2.0f * ds + 1e-3f < P.skin);
-        const bool by_div = st->div_count > 0 && ds > 0.25f * P.skin;
+        const bool by_div = st->div_count > 0 && 16 * st->div_count > st->n;
         const bool full = by_disp || by_div;
         if (by_div && !by_disp) st->rebuilds_div += 1;
         const bool part = !full && st->div_count > 0;
         st->rebuild = full ? 2 : part ? 1 : 0;
-        st->rcur = full ? P.rlist : P.rlist + 2.0f * ds + 1e-3f;
+        st->ds = full ? 0.0f : ds;
         st->force_rebuild = 0;
         st->div_count = 0;
         if (full || part) {
-            if (full) st->rebuilds += 1;
+            if (full) { st->rebuilds += 1; any_full = 1; }
             any = 1;
         }
         for (int q = 0; q < 3; ++q) {
@@ -635,6 +640,7 @@ __global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
     assign_hash_slices(d);
     if (threadIdx.x == 0) {
         d.flags[0] = any;
+        d.flags[2] = any_full;
         *d.n_pairs = 0ull;
     }
 }
@@ -651,7 +657,7 @@ __global__ void __launch_bounds__(256) k_init_begin(Dev d)
     for (int k = threadIdx.x; k < d.n_inst; k += blockDim.x) {
         InstState *st = &d.st[k];
         st->rebuild = 2;
-        st->rcur = d.prm[k].rlist;
+        st->ds = 0.0f;
         st->force_rebuild = 0;
         st->disp_step = 0u;
         for (int p = 0; p < 2; ++p)
@@ -664,7 +670,10 @@ __global__ void __launch_bounds__(256) k_init_begin(Dev d)
     assign_hash_slices(d);
     if (threadIdx.x == 0) {
         d.flags[0] = 1;
+        d.flags[2] = 1;
+        *d.n_build = 0;
         *d.div_total = 0;
+        *d.div_prev = 0;
         *d.n_pairs = 0ull;
     }
 }
@@ -1079,6 +1088,7 @@ __global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
             if (FUSE && (!DIV || sm.dflag == 0)) {
                 float mx = smax[0];  // visible: cell_geom (and the division decision) synchronise the block
                 for (int q = 1; q < SLOTS / 32; ++q) mx = fmaxf(mx, smax[q]);
+                d.cdisp[a] = mx;
                 atomicMax(&st->disp_step, __float_as_uint(mx));
             }
             d.CM[a] = make_float4(cm.x, cm.y, cm.z, 0.f);
@@ -1294,8 +1304,6 @@ __global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par)
             d.press[b] = P.minp;
             d.E[b] = P.daught_same ? d.E[a] : P.stiff1;
             d.cell_inst[b] = e.inst;
-            d.dirty[a] = 1;  // lists rebuilt around the two cells next step
-            d.dirty[b] = 1;
         }
         if (i < NODES) {
             size_t ga = (size_t)a * SLOTS + i, gb = (size_t)b * SLOTS + i;
@@ -1543,352 +1551,549 @@ __global__ void k_grid_fix(Dev d, int par)
 
 // ---------------------------------------------------------------------------
 // Neighbour-list build (instances whose displacement bound reached the skin,
-// or that divided).  The nodes are binned in cubes of edge hb slightly above
-// the list radius and the bins hashed into the instance's slice of the
-// buckets; a counting sort puts the positions in bucket order (hpos).
-// Bucket of bin (ix, iy, iz): the low bits of each coordinate side by side,
-// so that the 27 bins around a node fall in 27 distinct buckets and the three
-// bins along x are (unless they wrap) three consecutive buckets.
+// or that divided): every cell's box at the current positions, a table of the
+// cells by the bin of their box centre, then one CTA per cell that collects
+// the cells whose boxes come within the list radius of its own and, of their
+// nodes, those within the list radius of its nodes.
+//
+// A form that binned the nodes instead (a counting sort of all nodes into
+// bins of the list radius, every thread walking the 27 bins around its node)
+// went at the pace of the fullest node of a warp: next to the plane of a fresh
+// division a bin holds tens of nodes, and the build of one cell there took
+// 50 to 80 us.  Boxes cut the neighbours' nodes down to a few hundred that lie
+// near the cell, the warps test those against a patch of 30 nodes each, and
+// the entries come in their final order (ascending cell, then node).  Bound by
+// the latency of one cell's chain in partial builds (11 us a cell alone on its
+// SM) and by instruction issue in whole ones.  With this form and nb_mark's
+// rule a step of 2500 to 3200 growing cells went from 350 to 237 us (all of it
+// list build), one of 301 from 98 to 69 us; a whole build of 100,000 packed
+// cells takes 1.2 ms against 1.35 with the sort.
 // ---------------------------------------------------------------------------
-struct BinGeom {
-    float inv;          // 1 / bin edge
-    int bx, by;         // bits of x, y in the bucket number
-    unsigned mask;      // slice size - 1
-    unsigned base;      // first bucket of the instance's slice
-};
-
-__device__ __forceinline__ BinGeom bin_geom(const Dev &d, int inst)
-{
-    const InstState &st = d.st[inst];
-    BinGeom b;
-    // bin edge 1% above the list radius: float rounding of x / edge cannot
-    // put two nodes closer than the radius more than one bin apart
-    b.inv = 1.0f / ((st.rcur + 1e-4f) * 1.01f);
-    const int B = st.hbits;
-    b.bx = B / 3;
-    b.by = B / 3;
-    b.mask = (1u << B) - 1u;
-    b.base = st.hbase;
-    return b;
-}
-
 __device__ __forceinline__ int bin_coord(float v, float inv)
 {
-    return (int)floorf(fminf(fmaxf(v * inv, -1.0e9f), 1.0e9f));
+    return (int)floorf(fminf(fmaxf(__fmul_rn(v, inv), -1.0e9f), 1.0e9f));
 }
 
-constexpr int CB = 4;  // hash candidates loaded together in the list build
-
-__device__ __forceinline__ unsigned bucket_of(const BinGeom &b, int ix, int iy, int iz)
+// Bin of a box along one axis: the bin of its centre.
+__device__ __forceinline__ int box_bin(float lo, float hi, float inv)
 {
-    const unsigned code = ((unsigned)ix & ((1u << b.bx) - 1u)) | (((unsigned)iy & ((1u << b.by) - 1u)) << b.bx) |
-                          ((unsigned)iz << (b.bx + b.by));
-    return b.base + (code & b.mask);
+    return bin_coord(__fmul_rn(0.5f, __fadd_rn(lo, hi)), inv);
 }
 
-// B1: zero the bucket counts (hsize + SCAN_TILE entries, the tail pads the
-// last scan tile).
-__global__ void k_nh_zero(Dev d)
+__device__ __forceinline__ unsigned bin_slot(const InstState &st, int ix, int iy, int iz)
 {
-    if (!d.flags[0]) return;
-    int4 *p = reinterpret_cast<int4 *>(d.hcount);
-    const int n4 = (*d.hsz + SCAN_TILE) / 4;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += gridDim.x * blockDim.x)
-        p[q] = make_int4(0, 0, 0, 0);
+    unsigned h = (unsigned)ix * 0x8da6b343u ^ (unsigned)iy * 0xd8163841u ^ (unsigned)iz * 0xcb1ab31fu;
+    h ^= h >> 15;
+    h *= 0x9e3779b1u;
+    return st.hbase + (h >> (32 - st.hbits));
 }
 
-// B2: count the nodes of every bucket; each node keeps its rank.
-__global__ void __launch_bounds__(SLOTS) k_nh_count(Dev d)
+__device__ __forceinline__ float warp_min(float v)
 {
-    if (!d.flags[0]) return;
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// B1: boxes at the current positions and the cell table, one warp per cell.
+__device__ __forceinline__ void nb_boxes(const Dev &d)
+{
     const int W = n_work(d);
-    const int i = threadIdx.x;
-    for (int w = blockIdx.x; w < W; w += gridDim.x) {
-        const int a = cell_of(d, w);
-        const int inst = inst_of(d, a);
-        if (!d.st[inst].rebuild || i >= NODES) continue;
-        const BinGeom b = bin_geom(d, inst);
-        const size_t g = (size_t)a * SLOTS + i;
-        const float4 x = d.X[g];
-        const unsigned k = bucket_of(b, bin_coord(x.x, b.inv), bin_coord(x.y, b.inv), bin_coord(x.z, b.inv));
-        d.node_rank[g] = atomicAdd(&d.hcount[k], 1);
-    }
-}
-
-// B3: sums of the scan tiles.
-__global__ void __launch_bounds__(256) k_nh_scan_tiles(Dev d)
-{
-    if (!d.flags[0]) return;
-    __shared__ int wsum[32];
-    const int ntile = *d.hsz / SCAN_TILE + 1;
-    for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-        const int4 *p = reinterpret_cast<const int4 *>(d.hcount + (size_t)t * SCAN_TILE);
-        int s = 0;
-#pragma unroll
-        for (int q = 0; q < SCAN_TILE / 4 / 256; ++q) {
-            const int4 v = p[threadIdx.x + q * 256];
-            s += v.x + v.y + v.z + v.w;
-        }
-        s = warp_sum(s);
-        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int tot = 0;
-            for (int q = 0; q < 8; ++q) tot += wsum[q];
-            d.hscan[t] = tot;
-        }
-        __syncthreads();
-    }
-}
-
-// B4: exclusive scan of the tile sums (one block).
-__global__ void __launch_bounds__(1024) k_nh_scan_top(Dev d)
-{
-    if (!d.flags[0]) return;
-    __shared__ int wsum[32];
-    __shared__ int carry;
-    const int ntile = *d.hsz / SCAN_TILE + 1;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int t0 = 0; t0 < ntile; t0 += 1024) {
-        const int t = t0 + threadIdx.x;
-        const int v = t < ntile ? d.hscan[t] : 0;
-        int tot;
-        const int e = block_excl_scan<1024>(v, wsum, tot);
-        if (t < ntile) d.hscan[t] = carry + e;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += tot;
-        __syncthreads();
-    }
-}
-
-// B5: bucket starts (exclusive scan of the counts, in place).
-__global__ void __launch_bounds__(256) k_nh_scan_apply(Dev d)
-{
-    if (!d.flags[0]) return;
-    __shared__ int wsum[32];
-    constexpr int PER = SCAN_TILE / 256;  // 16 consecutive buckets per thread
-    const int ntile = *d.hsz / SCAN_TILE + 1;
-    for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-        int4 *p = reinterpret_cast<int4 *>(d.hcount + (size_t)t * SCAN_TILE + threadIdx.x * PER);
-        int4 v[PER / 4];
-        int s = 0;
-#pragma unroll
-        for (int q = 0; q < PER / 4; ++q) {
-            v[q] = p[q];
-            s += v[q].x + v[q].y + v[q].z + v[q].w;
-        }
-        int tot;
-        int run = d.hscan[t] + block_excl_scan<256>(s, wsum, tot);
-#pragma unroll
-        for (int q = 0; q < PER / 4; ++q) {
-            int4 o;
-            o.x = run; run += v[q].x;
-            o.y = run; run += v[q].y;
-            o.z = run; run += v[q].z;
-            o.w = run; run += v[q].w;
-            p[q] = o;
-        }
-    }
-}
-
-// B6: positions in bucket order.
-__global__ void __launch_bounds__(SLOTS) k_nh_fill(Dev d)
-{
-    if (!d.flags[0]) return;
-    const int W = n_work(d);
-    const int i = threadIdx.x;
-    for (int w = blockIdx.x; w < W; w += gridDim.x) {
-        const int a = cell_of(d, w);
-        const int inst = inst_of(d, a);
-        if (!d.st[inst].rebuild || i >= NODES) continue;
-        const BinGeom b = bin_geom(d, inst);
-        const size_t g = (size_t)a * SLOTS + i;
-        const float4 x = d.X[g];
-        const unsigned k = bucket_of(b, bin_coord(x.x, b.inv), bin_coord(x.y, b.inv), bin_coord(x.z, b.inv));
-        // w: the node as cell << 8 | node (cells < 2^23)
-        d.hpos[d.hcount[k] + d.node_rank[g]] = make_float4(x.x, x.y, x.z, __int_as_float((a << 8) | i));
-    }
-}
-
-// B7: per cell, from the nodes of other cells within the list radius of its
-// nodes: the candidate cells (ascending id) and each node's entries
-// (slot << 8 | node, ascending: by candidate cell, then node).  Candidate
-// cells are first collected in a shared open-addressing set ("temporary
-// slots"), each node's entries kept as (temporary slot, node) and remapped
-// once the slots are sorted.
-struct BuildSmem {
-    int tkey[256];           // candidate cell of each temporary slot, -1 if free
-    uint32_t mask[256][6];   // partner nodes of each temporary slot (CS3D_OPT_HALO_STATS)
-    int comp_key[256], comp_t[256];
-    short slot_of_t[256];    // final slot of a temporary slot, -1 if dropped
-    int slot_t[MAXC];        // temporary slot of each final slot
-    int wsum[32];
-    int ncomp;
-    int flag;
-};
-
-// Phase 0 builds the cells of whole-instance rebuilds and the divided cells
-// (dirty 1) of partial ones, and marks the candidates of the divided cells
-// (dirty 2); phase 1 builds the marked cells and clears all marks.
-__global__ void __launch_bounds__(SLOTS) k_nl_cell(Dev d, int phase)
-{
-    if (!d.flags[0]) return;
-    __shared__ BuildSmem sm;
-    const int W = n_work(d);
-    const int i = threadIdx.x;
-    for (int w = blockIdx.x; w < W; w += gridDim.x) {
+    const int lane = threadIdx.x & 31, nw = SLOTS / 32;
+    const unsigned epoch = *d.epoch;
+    for (int w = blockIdx.x * nw + (threadIdx.x >> 5); w < W; w += gridDim.x * nw) {
         const int a = cell_of(d, w);
         const int inst = inst_of(d, a);
         InstState *st = &d.st[inst];
-        const int rb = st->rebuild;
-        if (!rb) continue;  // uniform across the block
-        __syncthreads();
-        if (i == 0) sm.flag = d.dirty[a];
-        __syncthreads();
-        const int mark = sm.flag;
-        if (phase == 1 && mark && i == 0) d.dirty[a] = 0;
-        const bool build = phase == 0 ? (rb == 2 || mark == 1) : (rb == 1 && mark == 2);
-        if (!build) continue;
-        const BinGeom b = bin_geom(d, inst);
-        const float rl = st->rcur + 1e-4f;
-        const float rl2 = rl * rl;
-        const bool halo = d.halo_stats != 0;   // uniform
-        for (int t = i; t < 256; t += SLOTS) sm.tkey[t] = -1;
-        if (halo)
-            for (int q = i; q < 256 * 6; q += SLOTS) (&sm.mask[0][0])[q] = 0u;
-        if (i == 0) sm.ncomp = 0;
-        __syncthreads();
-        const size_t g = (size_t)a * SLOTS + i;
-        const float4 x = (i < NODES) ? d.X[g] : make_float4(0, 0, 0, 0);
-        uint16_t *ep = d.ent + (size_t)a * MAXE * SLOTS + i;
-        int cnt = 0;
-        bool lost = false;
-        if (i < NODES) {
-            const int ix = bin_coord(x.x, b.inv), iy = bin_coord(x.y, b.inv), iz = bin_coord(x.z, b.inv);
-            int last_c = -1, last_t = -1;
-            for (int r = 0; r < 9; ++r) {
-                const int jy = iy + (r % 3) - 1, jz = iz + r / 3 - 1;
-                const unsigned k0 = bucket_of(b, ix - 1, jy, jz);
-                const unsigned k2 = bucket_of(b, ix + 1, jy, jz);
-                // three consecutive buckets unless the x bits or the table wrap
-                const int nrun = (k2 == k0 + 2u) ? 1 : 3;
-                for (int u = 0; u < nrun; ++u) {
-                    unsigned kb, ke;
-                    if (nrun == 1) { kb = k0; ke = k0 + 3u; }
-                    else { kb = bucket_of(b, ix - 1 + u, jy, jz); ke = kb + 1u; }
-                    const int p0 = d.hcount[kb], p1 = d.hcount[ke];
-                    // candidates in batches: the loads of a batch are in flight together;
-                    // past the run a far sentinel fails the distance test
-                    for (int p = p0; p < p1; p += CB) {
-                      float4 yb[CB];
+        if (!st->rebuild) continue;
+        const float4 *X = d.X + (size_t)a * SLOTS;
+        float lx = 1e30f, ly = 1e30f, lz = 1e30f, hx = -1e30f, hy = -1e30f, hz = -1e30f;
 #pragma unroll
-                      for (int q = 0; q < CB; ++q)
-                          yb[q] = p + q < p1 ? d.hpos[p + q] : make_float4(1.0e30f, 1.0e30f, 1.0e30f, 0.f);
+        for (int k = 0; k < (NODES + 31) / 32; ++k) {
+            const int i = lane + 32 * k;
+            if (i < NODES) {
+                const float4 x = X[i];
+                lx = fminf(lx, x.x); hx = fmaxf(hx, x.x);
+                ly = fminf(ly, x.y); hy = fmaxf(hy, x.y);
+                lz = fminf(lz, x.z); hz = fmaxf(hz, x.z);
+            }
+        }
+        lx = warp_min(lx); ly = warp_min(ly); lz = warp_min(lz);
+        hx = warp_max(hx); hy = warp_max(hy); hz = warp_max(hz);
+        if (lane == 0) {
+            d.nbox[2 * a] = make_float4(lx, ly, lz, 0.f);
+            d.nbox[2 * a + 1] = make_float4(hx, hy, hz, 0.f);
+            if (lx <= hx) {   // some node is a number
+                // a look first: most cells are smaller than one already in
+                const float hq[3] = {0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz)};
 #pragma unroll
-                      for (int q = 0; q < CB; ++q) {
-                        const float4 y = yb[q];
-                        // the distance first: most candidates fail it
-                        const float dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
-                        if (!(dx * dx + dy * dy + dz * dz < rl2)) continue;
-                        // the instance's own hash slice holds only its own nodes
-                        const int id = __float_as_int(y.w);
-                        const int c = id >> 8;
-                        if (c == a) continue;
-                        int t = last_t;
-                        if (c != last_c) {
-                            t = -1;
-                            unsigned q = ((unsigned)c * 2654435761u) >> 24;
-                            for (int probe = 0; probe < 256; ++probe, q = (q + 1u) & 255u) {
-                                const int old = atomicCAS(&sm.tkey[q], -1, c);
-                                if (old == -1 || old == c) { t = (int)q; break; }
-                            }
-                            if (t < 0) { lost = true; continue; }
-                            last_c = c;
-                            last_t = t;
-                        }
-                        const int j = id & 255;
-                        if (halo) atomicOr(&sm.mask[t][j >> 5], 1u << (j & 31));
-                        if (cnt < MAXE) ep[(size_t)cnt * SLOTS] = (uint16_t)((t << 8) | j);
-                        ++cnt;
-                      }
-                    }
-                }
+                for (int q = 0; q < 3; ++q)
+                    if (__float_as_uint(hq[q]) > __ldcg(&st->hmax[q])) atomicMax(&st->hmax[q], __float_as_uint(hq[q]));
+                const float inv = d.prm[inst].inv_bin;
+                const unsigned b = bin_slot(*st, box_bin(lx, hx, inv), box_bin(ly, hy, inv), box_bin(lz, hz, inv));
+                const unsigned long long old =
+                    atomicExch(&d.bins[b], ((unsigned long long)epoch << 32) | (unsigned)a);
+                d.bnext[a] = (unsigned)(old >> 32) == epoch ? (int)(unsigned)old : -1;
             }
         }
-        __syncthreads();
-        for (int t = i; t < 256; t += SLOTS) {
-            const int c = sm.tkey[t];
-            if (c >= 0) {
-                const int q = atomicAdd(&sm.ncomp, 1);
-                sm.comp_key[q] = c;
-                sm.comp_t[q] = t;
-            }
-        }
-        __syncthreads();
-        const int nct = sm.ncomp;
-        for (int q = i; q < nct; q += SLOTS) {
-            const int key = sm.comp_key[q];
-            int r = 0;
-            for (int m = 0; m < nct; ++m) r += sm.comp_key[m] < key;
-            const int t = sm.comp_t[q];
-            sm.slot_of_t[t] = (short)(r < MAXC ? r : -1);
-            if (r < MAXC) {
-                sm.slot_t[r] = t;
-                d.cand[(size_t)a * MAXC + r] = key;
-            }
-        }
-        __syncthreads();
-        const int nc = nct < MAXC ? nct : MAXC;
-        // distinct partner nodes of the cell (statistics, CS3D_OPT_HALO_STATS)
-        int nh = 0;
-        if (halo) {
-            int ns = 0;
-            if (i < nc) {
-                const int t = sm.slot_t[i];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) ns += __popc(sm.mask[t][k]);
-            }
-            block_excl_scan<SLOTS>(ns, sm.wsum, nh);
-        }
-        // entries: (temporary slot, node) -> (slot, node), ascending
-        if (i < NODES) {
-            uint16_t ord[MAXE];
-            int m = 0;
-            const int ne = cnt < MAXE ? cnt : MAXE;
-            for (int k = 0; k < ne; ++k) {
-                const unsigned e = ep[(size_t)k * SLOTS];
-                const int s = sm.slot_of_t[e >> 8];
-                if (s < 0) continue;
-                const unsigned h = ((unsigned)s << 8) | (e & 255u);
-                int pos = m;
-                while (pos > 0 && ord[pos - 1] > h) { ord[pos] = ord[pos - 1]; --pos; }
-                ord[pos] = (uint16_t)h;
-                ++m;
-            }
-            for (int k = 0; k < m; ++k) ep[(size_t)k * SLOTS] = ord[k];
-            d.nent[g] = (uint8_t)m;
-            // new anchors, except for the neighbours of divided cells: other
-            // cells' lists rely on their old anchors
-            if (phase == 0) d.Xb[g] = x;
-            if (cnt > MAXE) atomicOr(&st->err, CS3D_ERRBIT_ENTRY_OVERFLOW);
-            if (lost) atomicOr(&st->err, CS3D_ERRBIT_CAND_OVERFLOW);
-        } else {
-            d.nent[g] = 0;
-        }
-        if (phase == 0 && rb == 1 && i < nc) atomicCAS(&d.dirty[d.cand[(size_t)a * MAXC + i]], 0, 2);
-        if (i == 0) {
-            if (nct > MAXC) atomicOr(&st->err, CS3D_ERRBIT_CAND_OVERFLOW);
-            atomicAdd(&st->built, 1);
-            d.ncand[a] = nc;
-            atomicMax(&st->max_cand, nct);
-            if (halo) atomicMax(&st->max_halo, nh);
-        }
-        int wm = cnt;
-        for (int o = 16; o > 0; o >>= 1) wm = max(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-        if ((i & 31) == 0) atomicMax(&st->max_entries, wm);
-        __syncthreads();
     }
+}
+
+__global__ void __launch_bounds__(SLOTS) k_nb_boxes(Dev d)
+{
+    if (d.flags[0]) nb_boxes(d);
+}
+
+// Gap of two intervals (negative: they overlap).
+__device__ __forceinline__ float gap(float lo1, float hi1, float lo2, float hi2)
+{
+    return fmaxf(lo1 - hi2, lo2 - hi1);
+}
+
+__device__ __forceinline__ bool boxes_near(float4 l1, float4 h1, float4 l2, float4 h2, float r)
+{
+    return gap(l1.x, h1.x, l2.x, h2.x) <= r && gap(l1.y, h1.y, l2.y, h2.y) <= r && gap(l1.z, h1.z, l2.z, h2.z) <= r;
+}
+
+// List radius of two cells whose nodes are at most da and db from their
+// anchors (both 0 at whole-instance builds), and the same for the box tests,
+// which it enlarges by more than their rounding.
+__device__ __forceinline__ float list_radius(const InstParams &P, bool full, float da, float db)
+{
+    return full ? P.rlist + 1e-4f : P.rlist + da + db + 1.1e-3f;
+}
+constexpr float BOX_REACH = 1.0001f;
+
+// B2: the cells that partial builds concern (the divided ones and those whose
+// boxes come within the list radius of one) into d.build, one thread per
+// cell.  Where one of the latter has moved more than skin/4 from its anchors,
+// its radius would lengthen its lists too much (64 entries a node is the
+// limit): the instance is rebuilt whole.  Deciding this for the cells at the
+// divisions and not for the farthest node of the instance leaves a third of
+// the whole builds of a growing colony.
+__device__ __forceinline__ void nb_mark(const Dev &d)
+{
+    const int W = n_work(d), T = *d.div_prev;
+    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < W; w += gridDim.x * blockDim.x) {
+        const int a = cell_of(d, w);
+        const int inst = inst_of(d, a);
+        InstState *st = &d.st[inst];
+        d.mark[a] = 0;
+        if (__ldcg(&st->rebuild) != 1) continue;
+        const InstParams &P = d.prm[inst];
+        const float4 lo = d.nbox[2 * a], hi = d.nbox[2 * a + 1];
+        const float da = d.cdisp[a];
+        int m = 0;
+        for (int q = 0; q < T; ++q) {
+            const DivEntry &e = d.divtab[q];
+            if (e.inst != inst) continue;
+            const int cs[2] = {e.parent, e.daughter};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int c = cs[k];
+                if (a == c) m |= 2;
+                else if (boxes_near(lo, hi, d.nbox[2 * c], d.nbox[2 * c + 1],
+                                    list_radius(P, false, da, d.cdisp[c]) * BOX_REACH))
+                    m |= 1;
+            }
+        }
+        if (!m) continue;
+        d.mark[a] = (uint8_t)m;
+        d.build[atomicAdd(d.n_build, 1)] = a;
+        if (m == 1 && da > 0.25f * P.skin && atomicExch(&st->rebuild, 2) != 2) {
+            st->rebuilds += 1;
+            st->rebuilds_div += 1;
+            d.flags[2] = 1;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(SLOTS) k_nb_mark(Dev d)
+{
+    if (d.flags[0]) nb_mark(d);
+}
+
+constexpr int NBW = SLOTS / 32;   // warps of a CTA, and cells whose nodes are staged together
+constexpr int MAXB = SLOTS;       // cells with boxes in reach that one pass takes
+constexpr int WL = 64;            // nodes of a warp's list
+
+// Nodes in reach of a warp's patch: minus their coordinates (the distance
+// tests are packed additions and multiplications of two nodes), the squared
+// list radius of their cell and slot << 8 | node.
+struct alignas(16) PatchList {
+    float x[WL], y[WL], z[WL], r2[WL];
+    uint16_t id[WL];
+};
+
+struct ListSmem {
+    float4 node[NBW][SLOTS];       // nodes in reach of the cell, by staged cell: x, y, z, node
+    PatchList list[NBW];
+    int count[NBW];
+    float rad[NBW];                // their list radii
+    int raw[MAXB], cell[MAXB];     // cells in reach: as found, ascending
+    unsigned touched[MAXC][6];     // partner nodes with an entry, by slot (CS3D_OPT_HALO_STATS)
+    uint8_t used[MAXB];
+    int n;
+    int todo[SLOTS], ntodo;        // cells of this CTA to build
+    // statistics of the instance st_inst, not yet in its state
+    int st_inst, built, max_cand, max_entries, max_halo;
+};
+
+// The nodes of cell c in reach (r) of the box lo, hi, in ascending order into
+// seg; returns their number.  One warp.
+__device__ __forceinline__ int stage_nodes(const Dev &d, int c, float4 lo, float4 hi, float r, float4 *seg)
+{
+    const int lane = threadIdx.x & 31;
+    const float4 *X = d.X + (size_t)c * SLOTS;
+    float4 x[(NODES + 31) / 32];
+#pragma unroll
+    for (int k = 0; k < (NODES + 31) / 32; ++k)
+        x[k] = lane + 32 * k < NODES ? X[lane + 32 * k] : make_float4(1e30f, 1e30f, 1e30f, 0.f);
+    int m = 0;
+#pragma unroll
+    for (int k = 0; k < (NODES + 31) / 32; ++k) {
+        const bool in = boxes_near(lo, hi, x[k], x[k], r);
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in)
+            seg[m + __popc(b & ((1u << lane) - 1u))] =
+                make_float4(x[k].x, x[k].y, x[k].z, __int_as_float(lane + 32 * k));
+        m += __popc(b);
+    }
+    return m;
+}
+
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long both(float v)
+{
+    return ((unsigned long long)__float_as_uint(v) << 32) | __float_as_uint(v);
+}
+
+// One thread's node in the list build: position (twice, for packed
+// arithmetic), its entry column and the entries so far.
+struct NodeEntries {
+    unsigned long long x, y, z;
+    uint16_t *ep;
+    int cnt;
+};
+
+// The n nodes of the warp's list against the node of every lane; with store,
+// entries for those within the radius.  Eight nodes at a time: the loads are
+// broadcasts and the distances independent.  Returns whether this lane's node
+// has any.
+__device__ __forceinline__ bool patch_flush(PatchList &L, int n, NodeEntries &e, bool store, ListSmem &sm, bool halo)
+{
+    const int lane = threadIdx.x & 31;
+    const int np = (n + 7) & ~7;
+    if (lane < np - n) L.r2[n + lane] = -1.0f;   // no distance is below
+    __syncwarp();
+    bool any = false;
+    for (int k = 0; k < np; k += 8) {
+        unsigned m = 0;
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+            const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&L.x[k + h]);
+            const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&L.y[k + h]);
+            const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&L.z[k + h]);
+            const float4 r2 = *reinterpret_cast<const float4 *>(&L.r2[k + h]);
+            const unsigned long long dx0 = add2(e.x, X.x), dx1 = add2(e.x, X.y), dy0 = add2(e.y, Y.x),
+                                     dy1 = add2(e.y, Y.y), dz0 = add2(e.z, Z.x), dz1 = add2(e.z, Z.y);
+            const unsigned long long d0 = fma2(dz0, dz0, fma2(dy0, dy0, fma2(dx0, dx0, 0ull)));
+            const unsigned long long d1 = fma2(dz1, dz1, fma2(dy1, dy1, fma2(dx1, dx1, 0ull)));
+            if (__uint_as_float((unsigned)d0) < r2.x) m |= 1u << h;
+            if (__uint_as_float((unsigned)(d0 >> 32)) < r2.y) m |= 2u << h;
+            if (__uint_as_float((unsigned)d1) < r2.z) m |= 4u << h;
+            if (__uint_as_float((unsigned)(d1 >> 32)) < r2.w) m |= 8u << h;
+        }
+        any |= m != 0u;
+        if (!store) continue;
+        while (m) {
+            const unsigned id = L.id[k + __ffs(m) - 1];
+            m &= m - 1u;
+            sm.used[id >> 8] = 1;
+            if (halo) atomicOr(&sm.touched[id >> 8][(id & 255u) >> 5], 1u << (id & 31u));
+            if (e.cnt < MAXE) e.ep[(size_t)e.cnt * SLOTS] = (uint16_t)id;
+            ++e.cnt;
+        }
+    }
+    __syncwarp();
+    return any;
+}
+
+// The m staged nodes of one cell (slot s, list radius rad) that are in reach
+// of the box of the warp's patch, onto the warp's list; a list with more than
+// 32 nodes is flushed.  n: its length.
+__device__ __forceinline__ bool patch_add(PatchList &L, int &n, const float4 *seg, int m, int s, float rad, float4 plo,
+                                          float4 phi, NodeEntries &e, bool store, ListSmem &sm, bool halo)
+{
+    const int lane = threadIdx.x & 31;
+    bool any = false;
+    for (int q0 = 0; q0 < m; q0 += 32) {
+        float4 y = make_float4(1e30f, 1e30f, 1e30f, 0.f);
+        if (q0 + lane < m) y = seg[q0 + lane];
+        const bool in = boxes_near(plo, phi, y, y, rad * BOX_REACH);
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            const int k = n + __popc(b & ((1u << lane) - 1u));
+            L.x[k] = -y.x; L.y[k] = -y.y; L.z[k] = -y.z;
+            L.r2[k] = rad * rad;
+            L.id[k] = (uint16_t)((s << 8) | __float_as_int(y.w));
+        }
+        n += __popc(b);
+        if (n > WL - 32) {
+            any |= patch_flush(L, n, e, store, sm, halo);
+            n = 0;
+        }
+    }
+    return any;
+}
+
+// Cells of the instance with a box in reach of the CTA's cell into sm.raw:
+// through the table, or (window >= 0) of the MAXB cells from `window` on.
+// sm.n may exceed MAXB.
+__device__ __forceinline__ void cells_in_reach(const Dev &d, const InstParams &P, const InstState *st, int a, int window,
+                                               float4 lo, float4 hi, bool full, float da, unsigned epoch, ListSmem &sm)
+{
+    const int t = threadIdx.x;
+    const auto near = [&](int c, float4 l, float4 h) {
+        return c != a && boxes_near(lo, hi, l, h, list_radius(P, full, da, full ? 0.0f : d.cdisp[c]) * BOX_REACH);
+    };
+    if (window >= 0) {
+        const int c = P.base + window + t;
+        if (window + t < st->n && near(c, d.nbox[2 * c], d.nbox[2 * c + 1]))
+            sm.raw[atomicAdd(&sm.n, 1)] = c;
+        return;
+    }
+    // the centre of a box in reach lies within r + its half extent of this box;
+    // a thousandth more covers the rounding of the bounds
+    const float inv = P.inv_bin, r = list_radius(P, full, da, st->ds) * BOX_REACH;
+    const float ex = (r + __uint_as_float(st->hmax[0])) * 1.001f, ey = (r + __uint_as_float(st->hmax[1])) * 1.001f,
+                ez = (r + __uint_as_float(st->hmax[2])) * 1.001f;
+    const int x0 = bin_coord(lo.x - ex, inv), y0 = bin_coord(lo.y - ey, inv), z0 = bin_coord(lo.z - ez, inv);
+    const long long nx = bin_coord(hi.x + ex, inv) - x0 + 1ll, ny = bin_coord(hi.y + ey, inv) - y0 + 1ll,
+                    nz = bin_coord(hi.z + ez, inv) - z0 + 1ll;
+    if (nx > 64 || ny > 64 || nz > 64 || nx * ny * nz > 4096) {   // some cell is far larger than the mesh at rest
+        if (t == 0) sm.n = MAXB + 1;
+        return;
+    }
+    const int nyz = (int)(ny * nz), nb = (int)nx * nyz;
+    for (int q = t; q < nb; q += SLOTS) {
+        const int ix = x0 + q / nyz, iy = y0 + (q % nyz) / (int)nz, iz = z0 + q % (int)nz;
+        const unsigned long long h = d.bins[bin_slot(*st, ix, iy, iz)];
+        int c = (unsigned)(h >> 32) == epoch ? (int)(unsigned)h : -1;
+        while (c >= 0) {
+            const int nxt = d.bnext[c];
+            const float4 l = d.nbox[2 * c], g = d.nbox[2 * c + 1];
+            // bins share table entries: only the cells of this very bin
+            if (near(c, l, g) && box_bin(l.x, g.x, inv) == ix && box_bin(l.y, g.y, inv) == iy &&
+                box_bin(l.z, g.z, inv) == iz) {
+                const int k = atomicAdd(&sm.n, 1);
+                if (k < MAXB) sm.raw[k] = c;
+            }
+            c = nxt;
+        }
+    }
+}
+
+// sm.raw[0 .. n) ascending into sm.cell (n <= MAXB).  Whole CTA; synchronises before and after.
+__device__ __forceinline__ void sort_reach(ListSmem &sm, int n)
+{
+    const int t = threadIdx.x;
+    if (t < n) {
+        const int key = sm.raw[t];
+        int k = 0;
+        for (int q = 0; q < n; ++q) k += sm.raw[q] < key;
+        sm.cell[k] = key;
+    }
+    __syncthreads();
+}
+
+// Statistics of the lists built so far into their instance's state (thread 0).
+__device__ __forceinline__ void list_stats(const Dev &d, ListSmem &sm)
+{
+    if (sm.st_inst < 0) return;
+    InstState *st = &d.st[sm.st_inst];
+    atomicAdd(&st->built, sm.built);
+    atomicMax(&st->max_cand, sm.max_cand);
+    atomicMax(&st->max_entries, sm.max_entries);
+    if (d.halo_stats) atomicMax(&st->max_halo, sm.max_halo);
+}
+
+// B3: the lists of cell a.  The whole CTA; its warps take a patch of 30
+// neighbouring nodes each.
+__device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned epoch, ListSmem &sm)
+{
+    const int t = threadIdx.x, wid = t >> 5, lane = t & 31;
+    const bool real = node < NODES;
+    const bool halo = d.halo_stats != 0;
+    const int inst = inst_of(d, a);
+    InstState *st = &d.st[inst];
+    const InstParams &P = d.prm[inst];
+    const bool full = st->rebuild == 2;
+    const float da = full ? 0.0f : d.cdisp[a];
+    const bool fresh = full || (d.mark[a] & 2);   // new anchors
+    const float4 lo = d.nbox[2 * a], hi = d.nbox[2 * a + 1];
+    const size_t g = (size_t)a * SLOTS + node;
+    const float4 x = real ? d.X[g] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
+    __syncthreads();
+    if (t == 0) {
+        sm.n = 0;
+        if (sm.st_inst != inst) {
+            list_stats(d, sm);
+            sm.st_inst = inst;
+            sm.built = sm.max_cand = sm.max_entries = sm.max_halo = 0;
+        }
+    }
+    sm.used[t] = 0;
+    if (halo && t < MAXC)
+        for (int q = 0; q < 6; ++q) sm.touched[t][q] = 0u;
+    __syncthreads();
+    cells_in_reach(d, P, st, a, -1, lo, hi, full, da, epoch, sm);
+    // box of the warp's patch
+    float4 plo, phi;
+    plo.x = warp_min(real ? x.x : 1e30f); phi.x = warp_max(real ? x.x : -1e30f);
+    plo.y = warp_min(real ? x.y : 1e30f); phi.y = warp_max(real ? x.y : -1e30f);
+    plo.z = warp_min(real ? x.z : 1e30f); phi.z = warp_max(real ? x.z : -1e30f);
+    NodeEntries e = {both(x.x), both(x.y), both(x.z), d.ent + (size_t)a * MAXE * SLOTS + node, 0};
+    PatchList &L = sm.list[wid];
+    int nslot = 0, nl = 0;
+    __syncthreads();
+    const int nr = sm.n;   // uniform
+    if (nr <= MAXC) {
+        // usual case: every cell in reach gets a slot, six at a time
+        sort_reach(sm, nr);
+        nslot = nr;
+        if (t < nr) d.cand[(size_t)a * MAXC + t] = sm.cell[t];
+        for (int c0 = 0; c0 < nr; c0 += NBW) {
+            if (c0 + wid < nr) {
+                const int c = sm.cell[c0 + wid];
+                const float rad = list_radius(P, full, da, full ? 0.0f : d.cdisp[c]);
+                const int m = stage_nodes(d, c, lo, hi, rad * BOX_REACH, sm.node[wid]);
+                if (lane == 0) { sm.count[wid] = m; sm.rad[wid] = rad; }
+            }
+            __syncthreads();
+            const int nc = min(NBW, nr - c0);
+            for (int c = 0; c < nc; ++c)
+                patch_add(L, nl, sm.node[c], sm.count[c], c0 + c, sm.rad[c], plo, phi, e, true, sm, halo);
+            __syncthreads();
+        }
+        patch_flush(L, nl, e, true, sm, halo);
+    } else {
+        // more cells in reach than slots: a slot only for a cell with an
+        // entry, one cell at a time, in ascending order
+        const int n = st->n;
+        for (int win = 0; win < n; win += MAXB) {
+            __syncthreads();
+            if (t == 0) sm.n = 0;
+            __syncthreads();
+            cells_in_reach(d, P, st, a, win, lo, hi, full, da, epoch, sm);
+            __syncthreads();
+            const int nw = sm.n;
+            sort_reach(sm, nw);
+            for (int c = 0; c < nw; ++c) {
+                const float rad = list_radius(P, full, da, full ? 0.0f : d.cdisp[sm.cell[c]]);
+                if (wid == 0) {
+                    const int m = stage_nodes(d, sm.cell[c], lo, hi, rad * BOX_REACH, sm.node[0]);
+                    if (lane == 0) sm.count[0] = m;
+                }
+                __syncthreads();
+                nl = 0;
+                bool any = patch_add(L, nl, sm.node[0], sm.count[0], 0, rad, plo, phi, e, false, sm, false);
+                any |= patch_flush(L, nl, e, false, sm, false);
+                if (__syncthreads_or(any)) {
+                    if (nslot < MAXC) {
+                        nl = 0;
+                        patch_add(L, nl, sm.node[0], sm.count[0], nslot, rad, plo, phi, e, true, sm, halo);
+                        patch_flush(L, nl, e, true, sm, halo);
+                        if (t == 0) d.cand[(size_t)a * MAXC + nslot] = sm.cell[c];
+                    }
+                    ++nslot;
+                }
+                __syncthreads();
+            }
+        }
+    }
+    if (real) {
+        d.nent[g] = (uint8_t)(e.cnt < MAXE ? e.cnt : MAXE);
+        // new anchors, except for the neighbours of divided cells: other
+        // cells' lists rely on their old anchors
+        if (fresh) d.Xb[g] = x;
+        if (e.cnt > MAXE) atomicOr(&st->err, CS3D_ERRBIT_ENTRY_OVERFLOW);
+    }
+    // the padding slots have no entries
+    if (t >= NODES) d.nent[(size_t)a * SLOTS + t] = 0;
+    const int wm = __reduce_max_sync(0xffffffffu, e.cnt);
+    if (lane == 0) atomicMax(&sm.max_entries, wm);
+    const int nused = __syncthreads_count(sm.used[t] != 0);
+    int nh = 0;
+    if (halo) {
+        __shared__ int hsum;
+        if (t == 0) hsum = 0;
+        __syncthreads();
+        if (t < MAXC) {
+            for (int q = 0; q < 6; ++q) nh += __popc(sm.touched[t][q]);
+            atomicAdd(&hsum, nh);
+        }
+        __syncthreads();
+        nh = hsum;
+    }
+    if (t == 0) {
+        if (nslot > MAXC) atomicOr(&st->err, CS3D_ERRBIT_CAND_OVERFLOW);
+        d.ncand[a] = nslot < MAXC ? nslot : MAXC;
+        sm.built += 1;
+        sm.max_cand = max(sm.max_cand, nslot > MAXC ? nslot : nused);
+        sm.max_halo = max(sm.max_halo, nh);
+    }
+}
+
+// The marked cells of partial builds, then the other cells of instances that
+// are rebuilt whole.  A CTA looks at its cells 192 at a time, one to a thread.
+__device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
+{
+    const int t = threadIdx.x;
+    const unsigned epoch = *d.epoch;
+    const int node = __ldg(&d.topo.patch[t]);
+    if (t == 0) sm.st_inst = -1;
+    const int N = *d.n_build;
+    for (int q = blockIdx.x; q < N; q += gridDim.x) nb_cell(d, d.build[q], node, epoch, sm);
+    const int W = d.flags[2] ? n_work(d) : 0;
+    for (int w0 = blockIdx.x; w0 < W; w0 += gridDim.x * SLOTS) {
+        __syncthreads();
+        if (t == 0) sm.ntodo = 0;
+        __syncthreads();
+        const int w = w0 + t * gridDim.x;
+        if (w < W) {
+            const int a = cell_of(d, w);
+            if (d.st[inst_of(d, a)].rebuild == 2 && !d.mark[a]) sm.todo[atomicAdd(&sm.ntodo, 1)] = a;
+        }
+        __syncthreads();
+        const int n = sm.ntodo;
+        for (int q = 0; q < n; ++q) nb_cell(d, sm.todo[q], node, epoch, sm);
+    }
+    __syncthreads();
+    if (t == 0) list_stats(d, sm);
+}
+
+__global__ void __launch_bounds__(SLOTS, 6) k_nb_lists(Dev d)
+{
+    __shared__ ListSmem sm;
+    if (d.flags[0]) nb_lists(d, sm);
 }
 
 }  // namespace cs3d

@@ -38,3 +38,56 @@ def test_com_correction_is_the_float_sum_in_cell_order(mesh, n):
         want = st[k].reshape(n, 192) - np.float32(s / np.float32(n))
         assert np.array_equal(got[k].reshape(n, 192)[:, :180], want[:, :180])
     sim.close()
+
+
+def _pairs_within(x, ra):
+    """(cell, node, cell, node) of the nodes of different cells within ra, sorted keys."""
+    from scipy.spatial import cKDTree
+    n = x.shape[0]
+    flat = x.reshape(n * 180, 3)
+    pairs = cKDTree(flat).query_pairs(ra * 1.01, output_type="ndarray")
+    pairs = pairs[pairs[:, 0] // 180 != pairs[:, 1] // 180]
+    r = np.linalg.norm(flat[pairs[:, 0]] - flat[pairs[:, 1]], axis=1)
+    assert len(r) == 0 or np.abs(r - ra).min() > 1e-7   # no pair that rounding decides
+    pairs = pairs[r < ra]
+    both = np.concatenate([pairs, pairs[:, ::-1]])
+    return np.sort(both[:, 0].astype(np.int64) * (n * 180) + both[:, 1])
+
+
+@pytest.mark.parametrize("small,scale", [(0, 1.0), (1, 1.0), (30, 8.0), (200, 8.0), (200, 14.0)])
+def test_list_build_around_a_large_cell(mesh, small, scale):
+    """Contact pairs against a search over all nodes where one cell's box
+    reaches `small` others: below and above the 128 candidate slots, and with
+    a cell so large that the table of the cells is left aside."""
+    rng = np.random.default_rng(3)
+    xyz = W.centred(W.scaled_xyz(mesh)).astype(np.float64)
+    turn = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+    k = int(np.ceil(max(small, 1) ** (1.0 / 3.0)))
+    c = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3)[:small] * 1.15 - 0.575 * (k - 1)
+    c = c + rng.uniform(-0.05, 0.05, c.shape)
+    big = xyz @ turn * scale
+    if small:   # one in contact with a node of the large cell
+        c[small // 2] = big[7] * (1.0 - 0.6 / scale) if scale > 1 else [2.15, 0.0, 0.0]
+    x = [big] + [xyz * (0.5 if scale > 1 else 1.0) + p for p in c]
+    x = (np.stack(x) + 20.0).astype(np.float32)
+    n = len(x)
+    st = {"n": n}
+    for q, key in enumerate("XYZ"):
+        st[key] = np.zeros((n, 192), np.float32)
+        st[key][:, :180] = x[..., q]
+        st[key] = st[key].reshape(-1)
+    p = W.base_params(box_len=(60.0, 60.0, 60.0), growth_rate=0.0, use_rigid_box=0)
+    rest = np.zeros((192, 3), np.float32)
+    rest[:180] = xyz
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), *[np.ascontiguousarray(rest[:, q]) for q in range(3)])
+    sim = cs.Simulation(p, topo, n)
+    sim.set_option(cs.OPT_RECORD_PAIRS, 1)
+    sim.set_option(cs.OPT_PAIR_CAPACITY, 1 << 20)
+    sim.load_state(st["X"], st["Y"], st["Z"], n_cells=n)
+    sim.forces()
+    got = sim.pairs(0).astype(np.int64)
+    got = np.sort((got[:, 0] * 180 + got[:, 1]) * (n * 180) + got[:, 2] * 180 + got[:, 3])
+    want = _pairs_within(x.astype(np.float64), float(np.float32(p["attraction_range"])))
+    assert np.array_equal(got, want)
+    assert small == 0 or len(want) > 0
+    sim.close()
