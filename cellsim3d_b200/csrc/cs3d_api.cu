@@ -44,6 +44,8 @@ struct cs3d_ctx {
     int grid_lists = 0;            // blocks of the neighbour lists
     int grid_boxes = 0;            // blocks of the cell boxes (a warp per cell)
     int grid_s2 = 0;               // blocks of S2 and the integrator
+    int grid_steps = 0;            // blocks of k_steps that are resident together (0: no cooperative launch)
+    int n_now = 0;                 // cells of all instances after the last call
     cudaGraphExec_t graph[2][2][2][3] = {};  // [parity][division][integrate first][S2 mode: 0, fused 1, fused last 2]
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // asynchronous read-back (cs3d_get_state_async): a copy stream, two
@@ -429,15 +431,37 @@ int launch_step(cs3d_ctx *c, int par, bool div, bool k1 = true, int fuse = 0, co
     if (div) {
         k_div_select<<<c->n_inst, 256, 0, s>>>(d, par); ++n; pf.mark(s, "div_select");
         k_div_apply<<<c->grid_cells, SLOTS, 0, s>>>(d, par); ++n; pf.mark(s, "div_apply");
-        k_grid_fix<<<c->grid_flat, 256, 0, s>>>(d, par); ++n; pf.mark(s, "grid_fix");
-        if (c->any_far) { k_far_count<<<c->n_inst, 32, 0, s>>>(d); ++n; pf.mark(s, "far_count"); }
         // S2 did the next half kick of every cell that does not divide
-        if (fuse) { k_integrate_divided<<<c->grid_cells, SLOTS, 0, s>>>(d); ++n; pf.mark(s, "integrate_divided"); }
+        k_div_finish<<<c->grid_cells, SLOTS, 0, s>>>(d, par, c->any_far, fuse != 0); ++n; pf.mark(s, "div_finish");
     }
     if (soften) { k_soften<<<c->n_inst, 32, 0, s>>>(d, (int)soften); ++n; pf.mark(s, "soften"); }
     if (c->any_com) { launch_com(d, s, c->grid_s2, pf); n += 2; }
     CK(cudaGetLastError());
     c->launches_per_step = n;
+    return CS3D_OK;
+}
+
+// Systems of up to one cell for each SM take their steps in k_steps (us a step,
+// this kernel against the launch sequence: 1 growing cell 17.5 / 26.1, 8 cells
+// 27.8 / 34.7, 64 39.0 / 43.2, 150 47.2 / 49.4, 300 56.7 / 56.4; beyond that
+// its fixed four CTAs an SM cost more than the launches).
+bool in_one_kernel(const cs3d_ctx *c) { return c->grid_steps > 0 && c->n_now <= c->nsm; }
+// After a launch the host looks at the cell counts again.
+constexpr int STEPS_PER_LAUNCH = 256;
+
+// n steps from step s on in one cooperative launch; the state is kicked.
+int launch_steps(cs3d_ctx *c, long long s, int n, bool last)
+{
+    Dev d = c->d;
+    int par = (int)((s - 1) & 1);
+    int n_div = c->any_growth ? (int)std::max<long long>(0, std::min<long long>(n, c->max_div_steps - s + 1)) : 0;
+    int is_last = last, com = c->any_com, far = c->any_far;
+    CK(cudaMemsetAsync(d.bar, 0, 2 * sizeof(unsigned), c->stream));
+    // as many CTAs as the cells may become: one without a cell only waits
+    const int grid = std::min(c->grid_steps, c->cap_total);
+    void *args[] = {&d, &par, &n, &n_div, &is_last, &com, &far};
+    CK(cudaLaunchCooperativeKernel((const void *)k_steps, dim3(grid), dim3(SLOTS), args, sizeof(StepsSmem), c->stream));
+    c->launches_per_step = 1;
     return CS3D_OK;
 }
 
@@ -490,7 +514,11 @@ int read_errors(cs3d_ctx *c, unsigned *any)
     CK(cudaMemcpyAsync(st.data(), c->d.st, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     unsigned bits = 0;
-    for (auto &q : st) bits |= q.err;
+    c->n_now = 0;
+    for (auto &q : st) {
+        bits |= q.err;
+        c->n_now += q.n;
+    }
     *any = bits;
     c->last_err_bits = bits;
     return CS3D_OK;
@@ -599,13 +627,13 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     for (int k = 0; k < n_inst; ++k) bins += (size_t)table_size(capacity[k]);
     AL(d.nbox, 2 * (size_t)c->cap_total); AL(d.bins, bins); AL(d.bnext, c->cap_total); AL(d.epoch, 1);
     AL(d.cdisp, c->cap_total); AL(d.build, c->cap_total); AL(d.n_build, 1); AL(d.mark, c->cap_total);
-    AL(d.divtab, c->cap_total); AL(d.div_total, 1); AL(d.div_prev, 1);
+    AL(d.divtab, c->cap_total); AL(d.div_total, 1); AL(d.div_prev, 1); AL(d.flagged, c->cap_total);
     d.ev_cap = std::max(1 << 16, 2 * c->cap_total);
     AL(d.events, d.ev_cap); AL(d.n_events, 1);
     d.far_cap = d.ev_cap;
     AL(d.farlog, d.far_cap); AL(d.n_far, 1);
     AL(d.pick, (size_t)c->cap_total + n_inst);
-    AL(d.flags, 4);
+    AL(d.flags, 4); AL(d.bar, 2); AL(d.deal, DEALS);
     d.pair_cap = 1;
     AL(d.pairs, 1); AL(d.n_pairs, 1);
 #undef AL
@@ -646,6 +674,10 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     int occ_s2 = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s2, k_s2<true, 0>, SLOTS, 0);
     c->grid_s2 = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ_s2, 1)));
+    int occ_steps = 0, coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_steps, k_steps, SLOTS, sizeof(StepsSmem));
+    c->grid_steps = coop ? c->nsm * occ_steps : 0;
     *out = c;
     return CS3D_OK;
 }
@@ -797,6 +829,7 @@ int cs3d_load_state(cs3d_ctx *c, int inst, int n, const float *X, const float *Y
     static const float one3[3] = {1.0f, 1.0f, 1.0f};   // the reference's initial system centre
     CK(cudaMemcpyAsync(d.st[inst].syscm, one3, sizeof one3, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    c->n_now += n - c->hn[inst];
     c->hn[inst] = n;
     c->need_init = true;
     return CS3D_OK;
@@ -845,6 +878,25 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
         int par = (int)((s - 1) & 1);
         bool div = c->any_growth && s <= c->max_div_steps;
         const bool soften = is_soften_step(c, s);
+        if (!soften && in_one_kernel(c)) {
+            int m = std::min(n_steps - k, STEPS_PER_LAUNCH);   // up to a softening step, which starts from the kicked state too
+            for (long long q : c->soften_steps)
+                if (q > s) m = (int)std::min<long long>(m, q - s);
+            const bool last = k + m == n_steps;
+            if (k1) {
+                k_integrate<<<c->grid_s2, SLOTS, 0, c->stream>>>(c->d);
+                CK(cudaGetLastError());
+            }
+            if ((rc = launch_steps(c, s, m, last))) return rc;
+            c->host_step = s + m - 1;
+            k1 = c->any_com;
+            c->prekicked = last && !c->any_com;
+            k += m - 1;
+            // the cells may have outgrown the kernel
+            unsigned bits = 0;
+            if (!last && (rc = read_errors(c, &bits))) return rc;
+            continue;
+        }
         // S2 integrates the next step unless the step shifts or softens
         // cells after S2 (CoM correction, growth-end softening); on the last
         // step of the call it also keeps the step-end positions
@@ -1286,10 +1338,10 @@ struct StaticScratch {
     uint16_t ent[SCAP * MAXE * SLOTS];
     uint8_t nent[SCAP * SLOTS];
     DivEntry divtab[SCAP];
-    int div_total, div_prev;
+    int div_total, div_prev, flagged[SCAP];
     int4 events[SEVENTS];
     int n_events;
-    int flags[4];
+    int flags[4], deal[DEALS];
     int4 pairs[1];
     unsigned long long n_pairs;
     uint32_t nnpack[SLOTS];
@@ -1342,9 +1394,9 @@ Dev static_dev(StaticScratch *s)
     d.ent = s->ent; d.nent = s->nent;
     d.nbox = s->nbox; d.bins = s->bins; d.bnext = s->bnext; d.epoch = &s->epoch;
     d.cdisp = s->cdisp; d.build = s->build; d.n_build = &s->n_build; d.mark = s->mark;
-    d.divtab = s->divtab; d.div_total = &s->div_total; d.div_prev = &s->div_prev;
+    d.divtab = s->divtab; d.div_total = &s->div_total; d.div_prev = &s->div_prev; d.flagged = s->flagged;
     d.events = s->events; d.n_events = &s->n_events; d.ev_cap = SEVENTS;
-    d.flags = s->flags;
+    d.flags = s->flags; d.deal = s->deal;
     d.pairs = s->pairs; d.n_pairs = &s->n_pairs; d.pair_cap = 1; d.record_pairs = 0;
     return d;
 }

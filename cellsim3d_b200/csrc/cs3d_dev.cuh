@@ -60,6 +60,7 @@ struct InstState {
     int mm[2][6];          // grid extents (ordered-int min/max) by step parity
     unsigned disp_step;    // max node displacement of the current step (float bits)
     int div_count;         // divisions in the current step
+    int flagged;           // cells S2 found due to divide (in d.flagged)
     int force_rebuild;
     int max_entries, max_cand, max_halo;
     unsigned hbase;        // first bin of this instance's slice of the cell table
@@ -140,6 +141,7 @@ struct Dev {
     unsigned *epoch;
     DivEntry *divtab;
     int *div_total;
+    int *flagged;       // [cell] by instance from its base on: cells due to divide
     int *div_prev;      // divisions of the previous step (divtab)
     int4 *events;       // (inst, step, parent, daughter)
     int4 *farlog;       // (inst, step, far cells, 0) of the internal-cells mitotic count
@@ -148,7 +150,9 @@ struct Dev {
     uint8_t *pick;      // [cap_total + n_inst] flags of the random soft-cell picks
     int *n_events;
     int ev_cap;
-    int *flags;         // [0] any rebuild, [1] any division, [2] any whole-instance rebuild
+    int *flags;         // [0] any rebuild, [1] any division, [2] any partial build turned whole
+    int *deal;          // counters of the cells dealt out, by phase (Dealer)
+    unsigned *bar;      // [0] arrivals, [1] barriers passed (k_steps; zero at its launch)
     int4 *pairs;        // (cell_a<<8 | node_i, cell_b<<8 | node_j, kind, 0)
     unsigned long long *n_pairs;
     long long pair_cap;

@@ -67,10 +67,44 @@ __device__ __forceinline__ int block_excl_scan(int v, int *wsum, int &total)
 }
 
 
+// Partner data: read-only for the length of a step's own kernel, but written
+// by other CTAs between the phases of k_steps (COOP), which must not read it
+// through the read-only path.
+template <bool COOP>
+__device__ __forceinline__ float4 ld_partner(const float4 *p)
+{
+    return COOP ? *p : __ldg(p);
+}
+
 // Active cells: the identity for a single instance, else the work table.
 __device__ __forceinline__ int n_work(const Dev &d) { return d.single ? d.st[0].n : *d.work_n; }
 __device__ __forceinline__ int cell_of(const Dev &d, int w) { return d.single ? w : d.work[w]; }
 __device__ __forceinline__ int inst_of(const Dev &d, int a) { return d.single ? 0 : d.cell_inst[a]; }
+
+// Cells of a phase dealt out to the CTAs one by one: a CTA begins with the
+// cell of its index and draws the next one while it works.  A cell next to a
+// division takes three times as long as another, so that with a fixed stride
+// the last CTA of S1 ended 60 % after the mean one (2500 growing cells).
+// next[]: two words of the CTA's shared memory; the counter is zero at the
+// start of the phase (step_begin).
+struct Dealer {
+    int *counter, *next;
+    int w, turn;
+
+    __device__ __forceinline__ Dealer(int *counter_, int *next_) : counter(counter_), next(next_), w(blockIdx.x), turn(0) {}
+    // at the start of a cell's work, before a barrier
+    __device__ __forceinline__ void draw()
+    {
+        if (threadIdx.x == 0) next[turn] = (int)gridDim.x + atomicAdd(counter, 1);
+    }
+    // after a barrier that follows draw()
+    __device__ __forceinline__ void advance()
+    {
+        w = next[turn];
+        turn ^= 1;
+    }
+};
+enum { DEAL_S1, DEAL_S2, DEAL_LISTS, DEAL_FULL, DEALS };
 
 // Kick of the split velocity Verlet with the reference's mixed precision:
 // the float sum is scaled by the double literal 0.5 and divided by the mass
@@ -305,6 +339,7 @@ static_assert(EPRE == 2 * SB && SB == 4, "the sweep's entry window is two batche
 // Partner positions and velocities are read from global memory (L1/L2
 // resident: the partners of a cell are a few hundred nodes).
 // ---------------------------------------------------------------------------
+template <bool COOP>
 __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const SlotData &sd, int a, int i, float3 x,
                                         float3 v, int ne, const uint32_t (&pre)[EPRE / 2], double &FX,
                                         double &FY, double &FZ, double3 &vsum)
@@ -342,7 +377,7 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
         }
         float4 xj[SB];
 #pragma unroll
-        for (int q = 0; q < SB; ++q) xj[q] = id[q] >= 0 ? __ldg(&d.X[id[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < SB; ++q) xj[q] = id[q] >= 0 ? ld_partner<COOP>(&d.X[id[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int q = 0; q < SB; ++q) {
             if (id[q] < 0) continue;
@@ -374,7 +409,7 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
         }
         float4 vj[SB];
 #pragma unroll
-        for (int q = 0; q < SB; ++q) vj[q] = id[q] >= 0 ? __ldg(&d.V[id[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < SB; ++q) vj[q] = id[q] >= 0 ? ld_partner<COOP>(&d.V[id[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int q = 0; q < SB; ++q) {
             if (id[q] < 0) continue;
@@ -390,6 +425,7 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
 // S2 sweep: sum of the velocity differences over the dissipative pairs found
 // by S1 (their list, in column layout), with the velocities after the half
 // kicks; tangential() takes its tangential part.
+template <bool COOP>
 __device__ __forceinline__ double3 sweep_s2(const Dev &d, const int *cell, int a, int i, float3 v, int nd)
 {
     const uint16_t *dl = d.dlist + (size_t)a * MAXD * SLOTS + i;
@@ -401,7 +437,7 @@ __device__ __forceinline__ double3 sweep_s2(const Dev &d, const int *cell, int a
         float4 vj[SB];
 #pragma unroll
         for (int q = 0; q < SB; ++q)
-            vj[q] = e[q] != 0xffffu ? __ldg(&d.Vb[cell[e[q] >> 8] * SLOTS + (int)(e[q] & 255u)])
+            vj[q] = e[q] != 0xffffu ? ld_partner<COOP>(&d.Vb[cell[e[q] >> 8] * SLOTS + (int)(e[q] & 255u)])
                                     : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int q = 0; q < SB; ++q) {
@@ -531,9 +567,8 @@ __global__ void __launch_bounds__(SLOTS) k_integrate(Dev d)
 
 // The next step's half kick and drift of the two cells of each division of
 // this step, after their placement (division steps whose S2 did the others).
-__global__ void __launch_bounds__(SLOTS) k_integrate_divided(Dev d)
+__device__ __forceinline__ void integrate_divided(const Dev &d, float *smax)
 {
-    __shared__ float smax[SLOTS / 32];
     const int T = *d.div_total;
     for (int q = blockIdx.x; q < T; q += gridDim.x) {
         const DivEntry e = d.divtab[q];
@@ -548,14 +583,15 @@ __global__ void __launch_bounds__(SLOTS) k_integrate_divided(Dev d)
 // ---------------------------------------------------------------------------
 // Slices of the cell table of the list build: every rebuilding instance gets
 // its own power-of-two range of bins (at least twice its cells), laid out
-// back to back.  Whole block (256 threads), after the rebuild decisions.
-__device__ void assign_hash_slices(const Dev &d)
+// back to back.  Whole block (NT threads), after the rebuild decisions.
+template <int NT>
+__device__ __forceinline__ void assign_hash_slices(const Dev &d)
 {
     __shared__ int wsum[32];
     __shared__ unsigned carry;
     if (threadIdx.x == 0) carry = 0u;
     __syncthreads();
-    for (int k0 = 0; k0 < d.n_inst; k0 += 256) {
+    for (int k0 = 0; k0 < d.n_inst; k0 += NT) {
         const int k = k0 + threadIdx.x;
         int size = 0;
         if (k < d.n_inst) {
@@ -570,7 +606,7 @@ __device__ void assign_hash_slices(const Dev &d)
             st->hbits = bits;
         }
         int tot;
-        const int off = block_excl_scan<256>(size, wsum, tot);
+        const int off = block_excl_scan<NT>(size, wsum, tot);
         if (k < d.n_inst) d.st[k].hbase = carry + (unsigned)off;
         if (threadIdx.x == 0) carry += (unsigned)tot;
         __syncthreads();
@@ -578,12 +614,14 @@ __device__ void assign_hash_slices(const Dev &d)
     if (threadIdx.x == 0) *d.epoch += 1u;   // empties the table
 }
 
-__global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
+template <int NT>
+__device__ __forceinline__ void step_begin(const Dev &d, int par_next)
 {
-    __shared__ int any, any_full;
+    __shared__ int any;
     if (threadIdx.x == 0) {
-        any = any_full = 0;
+        any = 0;
         *d.n_build = 0;
+        for (int q = 0; q < DEALS; ++q) d.deal[q] = 0;
         *d.div_prev = *d.div_total;   // the divisions the lists are rebuilt around
         *d.div_total = 0;
     }
@@ -628,7 +666,7 @@ __global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
         st->force_rebuild = 0;
         st->div_count = 0;
         if (full || part) {
-            if (full) { st->rebuilds += 1; any_full = 1; }
+            if (full) st->rebuilds += 1;
             any = 1;
         }
         for (int q = 0; q < 3; ++q) {
@@ -637,12 +675,18 @@ __global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
         }
     }
     __syncthreads();
-    assign_hash_slices(d);
+    if (any) assign_hash_slices<NT>(d);
     if (threadIdx.x == 0) {
         d.flags[0] = any;
-        d.flags[2] = any_full;
+        d.flags[1] = 0;
+        d.flags[2] = 0;
         *d.n_pairs = 0ull;
     }
+}
+
+__global__ void __launch_bounds__(256) k_step_begin(Dev d, int par_next)
+{
+    step_begin<256>(d, par_next);
 }
 
 // Whole-instance list rebuild of every instance at the next step.
@@ -667,11 +711,12 @@ __global__ void __launch_bounds__(256) k_init_begin(Dev d)
             }
     }
     __syncthreads();
-    assign_hash_slices(d);
+    assign_hash_slices<256>(d);
     if (threadIdx.x == 0) {
         d.flags[0] = 1;
-        d.flags[2] = 1;
+        d.flags[2] = 0;
         *d.n_build = 0;
+        for (int q = 0; q < DEALS; ++q) d.deal[q] = 0;
         *d.div_total = 0;
         *d.div_prev = 0;
         *d.n_pairs = 0ull;
@@ -733,13 +778,13 @@ __device__ __forceinline__ void cell_geom(const float4 *xs, GeomScratch &gs, flo
 // of |det| / 6 of the tetrahedra (centre of mass, triangle) and the area the
 // sum of the triangle areas.  The face centres first (one thread per face),
 // then the 552 triangles dealt out to all threads.
-__device__ __noinline__ void cell_volume(const Dev &d, const float4 *xs, float3 cm, GeomScratch &gs, bool sph,
+__device__ __noinline__ void cell_volume(const uint8_t *faces, const float4 *xs, float3 cm, GeomScratch &gs, bool sph,
                                          double &vol, double &area)
 {
     const int t = threadIdx.x, w = t >> 5, l = t & 31;
     const double cx = cm.x, cy = cm.y, cz = cm.z;
     if (t < CS3D_FACES) {
-        const uint8_t *F = d.topo.faces + 7 * t;
+        const uint8_t *F = faces + 7 * t;
         double ax = 0, ay = 0, az = 0;
         for (int q = 0; q < 5; ++q) {
             const float4 p = xs[F[q]];
@@ -757,7 +802,7 @@ __device__ __noinline__ void cell_volume(const Dev &d, const float4 *xs, float3 
     double tv = 0, fa = 0;
     for (int k = t; k < CS3D_FACES * 6; k += SLOTS) {
         const int f = k / 6, q = k - 6 * f;
-        const uint8_t *F = d.topo.faces + 7 * f;
+        const uint8_t *F = faces + 7 * f;
         const float4 p0 = xs[F[q]], p1 = xs[F[q + 1]];
         const double x0 = (double)p0.x - cx, y0 = (double)p0.y - cy, z0 = (double)p0.z - cz;
         const double x1 = (double)p1.x - cx, y1 = (double)p1.y - cy, z1 = (double)p1.z - cz;
@@ -800,20 +845,21 @@ struct S1Smem {
     SlotData sd;
     ArmForces arm;
     float press;         // the cell's pressure of this step
+    int next[2];
 };
 
-template <bool INIT>
-__global__ void __launch_bounds__(SLOTS, 4) k_s1(Dev d, int par)
+template <bool INIT, bool COOP>
+__device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
 {
-    extern __shared__ __align__(16) unsigned char s1_raw[];  // sizeof(S1Smem), > 48 KB
-    S1Smem &sm = *reinterpret_cast<S1Smem *>(s1_raw);
     const int W = n_work(d);
     const int i = threadIdx.x;
     const uint32_t nnp = (i < NODES) ? __ldg(&d.topo.nnpack[i]) : 0u;
     const int n0 = nnp & 255, n1 = (nnp >> 8) & 255, n2 = (nnp >> 16) & 255;
     const float sgn = (float)(int8_t)(nnp >> 24);
-    for (int w = blockIdx.x; w < W; w += gridDim.x) {
-        const int a = cell_of(d, w);
+    Dealer deal(&d.deal[DEAL_S1], sm.next);
+    while (deal.w < W) {
+        const int a = cell_of(d, deal.w);
+        deal.draw();
         const int inst = inst_of(d, a);
         const InstParams &P = d.prm[inst];
         const size_t g = (size_t)a * SLOTS + i;
@@ -899,7 +945,7 @@ __global__ void __launch_bounds__(SLOTS, 4) k_s1(Dev d, int par)
             }
             // contacts, src/propagate.cu:356-442 and the first dissipative sweep
             double3 vsum = make_double3(0.0, 0.0, 0.0);
-            const int nd = sweep_s1(d, P, sm.sd, a, i, x, v, ne, pre, FX, FY, FZ, vsum);
+            const int nd = sweep_s1<COOP>(d, P, sm.sd, a, i, x, v, ne, pre, FX, FY, FZ, vsum);
             const double3 vt = tangential(sm.xd, n0, n1, n2, sgn, vsum);
             if (nd > MAXD) atomic_or_err(&d.st[inst], CS3D_ERRBIT_ENTRY_OVERFLOW);
             // rigid box walls, src/propagate.cu:474-510 (float gap tests)
@@ -942,7 +988,15 @@ __global__ void __launch_bounds__(SLOTS, 4) k_s1(Dev d, int par)
             }
         }
         __syncthreads();
+        deal.advance();
     }
+}
+
+template <bool INIT>
+__global__ void __launch_bounds__(SLOTS, 4) k_s1(Dev d, int par)
+{
+    extern __shared__ __align__(16) unsigned char s1_raw[];  // sizeof(S1Smem)
+    s1_cells<INIT, false>(d, par, *reinterpret_cast<S1Smem *>(s1_raw));
 }
 
 // ---------------------------------------------------------------------------
@@ -958,6 +1012,8 @@ struct S2Smem {
 
     GeomScratch gs;
     int dflag;   // the cell divides (division steps)
+    float smax[SLOTS / 32];
+    int next[2];
 };
 
 // Integrate + ForwardTime of the next step (src/propagate.cu:681-763) on the
@@ -990,7 +1046,7 @@ __device__ __forceinline__ float next_kick(const Dev &d, const InstParams &P, si
     return sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
 }
 
-__device__ __forceinline__ void flush_mm(Dev &d, int inst, int pn, const float *acc)
+__device__ __forceinline__ void flush_mm(const Dev &d, int inst, int pn, const float *acc)
 {
     int *mm = d.st[inst].mm[pn];
     for (int q = 0; q < 3; ++q) {
@@ -1005,11 +1061,10 @@ __device__ __forceinline__ void flush_mm(Dev &d, int inst, int pn, const float *
 // cs3d_step call, which also keeps the step-end positions (Xe; the step-end
 // velocities are Vb) for the state read-back, so that the next call starts
 // without a k_integrate pass.
-template <bool DIV, int FUSE>
-__global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
+template <bool DIV, bool COOP>
+__device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, S2Smem &sm)
 {
-    __shared__ S2Smem sm;
-    __shared__ float smax[SLOTS / 32];
+    float *smax = sm.smax;
     const int W = n_work(d);
     const int i = threadIdx.x;
     const int pn = par ^ 1;
@@ -1018,8 +1073,10 @@ __global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
     const float sgn = (float)(int8_t)(nnp >> 24);
     int acc_inst = -1;
     float acc[6];
-    for (int w = blockIdx.x; w < W; w += gridDim.x) {
-        const int a = cell_of(d, w);
+    Dealer deal(&d.deal[DEAL_S2], sm.next);
+    while (deal.w < W) {
+        const int a = cell_of(d, deal.w);
+        deal.draw();
         const int inst = inst_of(d, a);
         const InstParams &P = d.prm[inst];
         InstState *st = &d.st[inst];
@@ -1036,7 +1093,7 @@ __global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
         float3 fdk = make_float3(0.f, 0.f, 0.f);
         if (i < NODES) {
             const float3 v = f3(v4);
-            const double3 vt = tangential(sm.xs, n0, n1, n2, sgn, sweep_s2(d, sm.cell, a, i, v, nd));
+            const double3 vt = tangential(sm.xs, n0, n1, n2, sgn, sweep_s2<COOP>(d, sm.cell, a, i, v, nd));
             const float3 fd = dis_force(P, sm.vs, i, n0, n1, n2, vt);
 
             d.FD[g] = make_float4(fd.x, fd.y, fd.z, 0.f);
@@ -1056,7 +1113,7 @@ __global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
         if (DIV) {
             if (st->step <= P.div_steps && P.growth > 0.0f) {
                 double vol, area;
-                cell_volume(d, sm.xs, cm, sm.gs, P.check_sph != 0, vol, area);
+                cell_volume(d.topo.faces, sm.xs, cm, sm.gs, P.check_sph != 0, vol, area);
                 if (i == 0) {
                     d.vol[a] = (float)vol;
                     if (!isfinite(vol)) { atomic_or_err(st, CS3D_ERRBIT_NONFINITE_VOL); vol = 1.0; }
@@ -1069,6 +1126,10 @@ __global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
                     }
                     d.divflag[a] = (uint8_t)flag;
                     sm.dflag = flag;
+                    if (flag) {
+                        d.flagged[P.base + atomicAdd(&st->flagged, 1)] = a;
+                        d.flags[1] = 1;
+                    }
                 }
             }
         }
@@ -1105,9 +1166,18 @@ __global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
             }
         }
         __syncthreads();
+        deal.advance();
     }
     if (threadIdx.x == 0 && acc_inst >= 0) flush_mm(d, acc_inst, pn, acc);
 }
+
+template <bool DIV, int FUSE>
+__global__ void __launch_bounds__(SLOTS, 5) k_s2(Dev d, int par)
+{
+    __shared__ S2Smem sm;
+    s2_cells<DIV, false>(d, par, FUSE, sm);
+}
+
 // Centre of mass, bounding boxes and grid extents only (initialisation,
 // src/GPUbounce.cu:739-763).
 __global__ void __launch_bounds__(SLOTS) k_geom(Dev d, int par)
@@ -1140,9 +1210,13 @@ __global__ void __launch_bounds__(SLOTS) k_geom(Dev d, int par)
 // ---------------------------------------------------------------------------
 // Division (src/GPUbounce.cu:1210-1286, src/postscriptinit.cu:148-256).
 // D1: one block per instance, dividers in ascending index order, one RANMAR
-// normal each (bit-exact float arithmetic of src/RandomVector.h:8-24).
+// normal each (bit-exact float arithmetic of src/RandomVector.h:8-24).  S2
+// left the flagged cells of each instance in a list, in no order.  The
+// generator's state is staged in shared memory: its draws are one dependent
+// chain, which took 4 us a division from global memory.
 // ---------------------------------------------------------------------------
-__device__ void ranmar_dev(InstState *st, float *out, int len)
+template <typename S>   // InstState or DivRng
+__device__ void ranmar_dev(S *st, float *out, int len)
 {
     for (int v = 0; v < len; ++v) {
         float uni = __fsub_rn(st->u[st->i97], st->u[st->j97]);
@@ -1158,7 +1232,8 @@ __device__ void ranmar_dev(InstState *st, float *out, int len)
     }
 }
 
-__device__ void random_vector_dev(InstState *st, float n[3])
+template <typename S>
+__device__ void random_vector_dev(S *st, float n[3])
 {
     float r[2], s;
     do {
@@ -1174,86 +1249,120 @@ __device__ void random_vector_dev(InstState *st, float n[3])
     n[2] = __fsub_rn(1.0f, __fmul_rn(2.0f, __fadd_rn(__fmul_rn(x1, x1), __fmul_rn(x2, x2))));
 }
 
-__global__ void __launch_bounds__(256) k_div_select(Dev d, int par)
+struct DivRng {
+    float u[98];
+    float rc, rcd, rcm;
+    int i97, j97;
+};
+
+struct DivSmem {
+    DivRng rng;
+    int warp_cnt[32];
+    int base;
+};
+
+// NT threads; k: the instance.
+template <int NT>
+__device__ __forceinline__ void div_select(const Dev &d, int par, int k, DivSmem &sm)
 {
-    const int k = blockIdx.x;
-    if (k >= d.n_inst) return;
     InstState *st = &d.st[k];
     const InstParams &P = d.prm[k];
     if (!(st->step <= P.div_steps && P.growth > 0.0f)) return;
-    __shared__ int cnt;
-    __shared__ int warp_cnt[8];
-    __shared__ int base_slot;
-    const int n0 = st->n;
-    if (threadIdx.x == 0) cnt = 0;
-    __syncthreads();
-    int mine = 0;
-    for (int c = threadIdx.x; c < n0; c += blockDim.x) mine += d.divflag[P.base + c] ? 1 : 0;
-    mine = warp_sum(mine);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&cnt, mine);
-    __syncthreads();
-    const int total = cnt;
+    const int total = st->flagged, t = threadIdx.x;
     if (total == 0) return;
+    const int n0 = st->n;
     const int room = P.cap - n0;
     const int ndiv = total < room ? total : room;
-    if (threadIdx.x == 0) {
+    __syncthreads();   // all have read the count
+    if (t == 0) {
         if (total > room) atomicOr(&st->err, CS3D_ERRBIT_CAPACITY);
-        base_slot = atomicAdd(d.div_total, ndiv);
+        sm.base = atomicAdd(d.div_total, ndiv);
         st->div_count = ndiv;
-        atomicOr(&d.flags[1], 1);
+        st->flagged = 0;
+    }
+    for (int q = t; q < 98; q += NT) sm.rng.u[q] = st->u[q];
+    if (t == 0) {
+        sm.rng.rc = st->rc; sm.rng.rcd = st->rcd; sm.rng.rcm = st->rcm;
+        sm.rng.i97 = st->i97; sm.rng.j97 = st->j97;
     }
     __syncthreads();
-    // ascending compaction in chunks of blockDim
-    int done = 0;
-    for (int c0 = 0; c0 < n0 && done < ndiv; c0 += blockDim.x) {
-        int c = c0 + threadIdx.x;
-        int f = (c < n0) ? (d.divflag[P.base + c] ? 1 : 0) : 0;
-        unsigned b = __ballot_sync(0xffffffffu, f);
-        int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        if (lane == 0) warp_cnt[wid] = __popc(b);
-        __syncthreads();
-        int off = done;
-        for (int q = 0; q < wid; ++q) off += warp_cnt[q];
-        off += __popc(b & ((1u << lane) - 1u));
-        if (f && off < ndiv) {
-            DivEntry &e = d.divtab[base_slot + off];
-            e.parent = P.base + c;
-            e.daughter = P.base + n0 + off;
-            e.inst = k;
+    const int base = sm.base;
+    if (total <= NT) {
+        // rank of each flagged cell among them
+        if (t < total) {
+            const int *f = d.flagged + P.base;
+            const int a = f[t];
+            int r = 0;
+            for (int q = 0; q < total; ++q) r += f[q] < a;
+            if (r < ndiv) {
+                DivEntry &e = d.divtab[base + r];
+                e.parent = a;
+                e.daughter = P.base + n0 + r;
+                e.inst = k;
+            }
         }
-        int tot = 0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) tot += warp_cnt[q];
-        done += tot;
         __syncthreads();
+    } else {
+        // many: ascending compaction of the flags in chunks of NT
+        int done = 0;
+        for (int c0 = 0; c0 < n0 && done < ndiv; c0 += NT) {
+            const int c = c0 + t;
+            const int f = (c < n0) ? (d.divflag[P.base + c] ? 1 : 0) : 0;
+            const unsigned b = __ballot_sync(0xffffffffu, f);
+            const int lane = t & 31, wid = t >> 5;
+            if (lane == 0) sm.warp_cnt[wid] = __popc(b);
+            __syncthreads();
+            int off = done;
+            for (int q = 0; q < wid; ++q) off += sm.warp_cnt[q];
+            off += __popc(b & ((1u << lane) - 1u));
+            if (f && off < ndiv) {
+                DivEntry &e = d.divtab[base + off];
+                e.parent = P.base + c;
+                e.daughter = P.base + n0 + off;
+                e.inst = k;
+            }
+            int tot = 0;
+            for (int q = 0; q < NT / 32; ++q) tot += sm.warp_cnt[q];
+            done += tot;
+            __syncthreads();
+        }
     }
     // normals in ascending order (one serial RNG stream per instance)
-    if (threadIdx.x == 0) {
-        int ev0 = atomicAdd(d.n_events, ndiv);
+    if (t == 0) {
+        const int ev0 = atomicAdd(d.n_events, ndiv);
+        const int w0 = d.single ? 0 : atomicAdd(d.work_n, ndiv);
         for (int q = 0; q < ndiv; ++q) {
-            DivEntry &e = d.divtab[base_slot + q];
+            DivEntry &e = d.divtab[base + q];
             float n[3];
-            random_vector_dev(st, n);
+            random_vector_dev(&sm.rng, n);
             e.n[0] = n[0]; e.n[1] = n[1]; e.n[2] = n[2];
             float nn = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
             if (fabsf(nn - 1.0f) > 1e-3f) atomicOr(&st->err, CS3D_ERRBIT_BAD_NORMAL);
             if (ev0 + q < d.ev_cap) d.events[ev0 + q] = make_int4(k, st->step, e.parent - P.base, e.daughter - P.base);
-            if (!d.single) d.work[atomicAdd(d.work_n, 1)] = e.daughter;
+            if (!d.single) d.work[w0 + q] = e.daughter;
         }
         st->n = n0 + ndiv;
+        st->rc = sm.rng.rc; st->i97 = sm.rng.i97; st->j97 = sm.rng.j97;
         for (int q = 0; q < 3; ++q) {
             st->mm[par ^ 1][2 * q] = f2o(1.0e30f);
             st->mm[par ^ 1][2 * q + 1] = f2o(-1.0e30f);
         }
     }
-    for (int c = threadIdx.x; c < n0; c += blockDim.x) d.divflag[P.base + c] = 0;
+    __syncthreads();
+    for (int q = t; q < 98; q += NT) st->u[q] = sm.rng.u[q];
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) k_div_select(Dev d, int par)
+{
+    __shared__ DivSmem sm;
+    if (d.flags[1] && (int)blockIdx.x < d.n_inst) div_select<256>(d, par, blockIdx.x, sm);
 }
 
 // D2: one block per division: the two daughters by half-space projection
 // through CM + n*gap/2 (FP64 geometry), velocities, pressures, stiffness.
-__global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par)
+__device__ __forceinline__ void div_apply(const Dev &d, int par, float4 *xs, GeomScratch &gs)
 {
-    __shared__ float4 xs[SLOTS];
-    __shared__ GeomScratch gs;
     const int T = *d.div_total;
     const int pn = par ^ 1;
     const int i = threadIdx.x;
@@ -1322,6 +1431,13 @@ __global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par)
     }
 }
 
+__global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par)
+{
+    __shared__ float4 xs[SLOTS];
+    __shared__ GeomScratch gs;
+    div_apply(d, par, xs, gs);
+}
+
 // CoM correction at the end of a step (correct_com, src/GPUbounce.cu:1430-1440
 // with calc_sys_CM :2504-2520 and CorrectCoMMotion, src/propagate.cu:766-776):
 // the mean of the cells' centres of mass (a float sum in cell order, as the
@@ -1368,7 +1484,7 @@ __global__ void __launch_bounds__(256) k_com_centre(Dev d)
 // over the active cells, bound by memory (64 B a node).  One block per
 // instance took 300 us a step at 1023 cells, with the centre's sum from
 // global memory.
-__global__ void __launch_bounds__(SLOTS) k_com_shift(Dev d)
+__device__ __forceinline__ void com_shift(const Dev &d)
 {
     const int W = n_work(d);
     for (int w = blockIdx.x; w < W; w += gridDim.x) {
@@ -1386,10 +1502,12 @@ __global__ void __launch_bounds__(SLOTS) k_com_shift(Dev d)
     }
 }
 
+__global__ void __launch_bounds__(SLOTS) k_com_shift(Dev d) { com_shift(d); }
+
 // calc_sys_CM, src/GPUbounce.cu:2504-2520: the float mean of the first n
 // centres of mass, summed in cell order; recorded as the instance's system
 // centre.
-__device__ float3 sys_centre(const Dev &d, const InstParams &P, InstState *st, int n)
+__device__ __forceinline__ float3 sys_centre(const Dev &d, const InstParams &P, InstState *st, int n)
 {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     for (int c = 0; c < n; ++c) {
@@ -1415,7 +1533,7 @@ __device__ __forceinline__ float dist2(float4 cm, float3 o)
 
 // getRmax2, src/GPUbounce.cu:2523-2536: the largest squared distance of the
 // first n centres of mass from the recorded system centre.
-__device__ float rmax2_from(const Dev &d, const InstParams &P, const InstState *st, int n)
+__device__ __forceinline__ float rmax2_from(const Dev &d, const InstParams &P, const InstState *st, int n)
 {
     const float3 o = make_float3(st->syscm[0], st->syscm[1], st->syscm[2]);
     float r2 = 0.0f;
@@ -1431,11 +1549,9 @@ __device__ float rmax2_from(const Dev &d, const InstParams &P, const InstState *
 // whose centre of mass lies farther than radius_cutoff x the largest distance
 // from the system's centre are not counted as dividing.  The daughters'
 // centres of mass are still 0 here (computed in their first step), as in the
-// reference.  One thread per instance.
-__global__ void k_far_count(Dev d)
+// reference.  One thread per instance (k).
+__device__ __forceinline__ void far_count(const Dev &d, int k)
 {
-    const int k = blockIdx.x;
-    if (k >= d.n_inst || threadIdx.x != 0) return;
     const InstParams &P = d.prm[k];
     InstState *st = &d.st[k];
     if (!(P.far_r > 0.0f) || !(st->step <= P.div_steps && P.growth > 0.0f)) return;
@@ -1515,7 +1631,7 @@ __global__ void __launch_bounds__(SLOTS) k_vol_hist(Dev d, int inst, float lo, f
         float4 blo, bhi;
         cell_geom(xs, gs, cm, blo, bhi);
         double vol, area;
-        cell_volume(d, xs, cm, gs, false, vol, area);
+        cell_volume(d.topo.faces, xs, cm, gs, false, vol, area);
         if (i == 0) {
             const float v = (float)vol;
             if (vols) vols[c] = v;
@@ -1533,7 +1649,7 @@ __global__ void __launch_bounds__(SLOTS) k_vol_hist(Dev d, int inst, float lo, f
 }
 
 // G: grid extents of instances that divided this step, from all boxes.
-__global__ void k_grid_fix(Dev d, int par)
+__device__ __forceinline__ void grid_fix(const Dev &d, int par)
 {
     const int pn = par ^ 1;
     const int W = n_work(d);
@@ -1547,6 +1663,22 @@ __global__ void k_grid_fix(Dev d, int par)
         atomicMin(&mm[2], f2o(lo.y)); atomicMax(&mm[3], f2o(hi.y));
         atomicMin(&mm[4], f2o(lo.z)); atomicMax(&mm[5], f2o(hi.z));
     }
+}
+
+// After the placement of the daughters: the grid extents, with far the
+// internal-cells count, and with fuse the next half kick of the divided cells.
+__device__ __forceinline__ void div_finish(const Dev &d, int par, bool far, bool fuse, float *smax)
+{
+    grid_fix(d, par);
+    if (far && threadIdx.x == 0)
+        for (int k = blockIdx.x; k < d.n_inst; k += gridDim.x) far_count(d, k);
+    if (fuse) integrate_divided(d, smax);
+}
+
+__global__ void __launch_bounds__(SLOTS) k_div_finish(Dev d, int par, int far, int fuse)
+{
+    __shared__ float smax[SLOTS / 32];
+    if (d.flags[1]) div_finish(d, par, far != 0, fuse != 0, smax);
 }
 
 // ---------------------------------------------------------------------------
@@ -1670,9 +1802,9 @@ __device__ __forceinline__ float list_radius(const InstParams &P, bool full, flo
 }
 constexpr float BOX_REACH = 1.0001f;
 
-// B2: the cells that partial builds concern (the divided ones and those whose
-// boxes come within the list radius of one) into d.build, one thread per
-// cell.  Where one of the latter has moved more than skin/4 from its anchors,
+// B2: the cells to build into d.build, one thread per cell: all cells of whole
+// builds, and those that partial builds concern (the divided ones and those
+// whose boxes come within the list radius of one).  Where one of the latter has moved more than skin/4 from its anchors,
 // its radius would lengthen its lists too much (64 entries a node is the
 // limit): the instance is rebuilt whole.  Deciding this for the cells at the
 // divisions and not for the farthest node of the instance leaves a third of
@@ -1684,8 +1816,15 @@ __device__ __forceinline__ void nb_mark(const Dev &d)
         const int a = cell_of(d, w);
         const int inst = inst_of(d, a);
         InstState *st = &d.st[inst];
+        const int rb = __ldcg(&st->rebuild);
+        if (rb != 1) {
+            // whole build (one that this phase decided on: left to the CTAs'
+            // second pass, unless it is seen here)
+            d.mark[a] = rb == 2 ? 4 : 0;
+            if (rb == 2) d.build[atomicAdd(d.n_build, 1)] = a;
+            continue;
+        }
         d.mark[a] = 0;
-        if (__ldcg(&st->rebuild) != 1) continue;
         const InstParams &P = d.prm[inst];
         const float4 lo = d.nbox[2 * a], hi = d.nbox[2 * a + 1];
         const float da = d.cdisp[a];
@@ -1739,8 +1878,7 @@ struct ListSmem {
     int raw[MAXB], cell[MAXB];     // cells in reach: as found, ascending
     unsigned touched[MAXC][6];     // partner nodes with an entry, by slot (CS3D_OPT_HALO_STATS)
     uint8_t used[MAXB];
-    int n;
-    int todo[SLOTS], ntodo;        // cells of this CTA to build
+    int n, hsum, next[2];
     // statistics of the instance st_inst, not yet in its state
     int st_inst, built, max_cand, max_entries, max_halo;
 };
@@ -2043,15 +2181,14 @@ __device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned 
     const int nused = __syncthreads_count(sm.used[t] != 0);
     int nh = 0;
     if (halo) {
-        __shared__ int hsum;
-        if (t == 0) hsum = 0;
+        if (t == 0) sm.hsum = 0;
         __syncthreads();
         if (t < MAXC) {
             for (int q = 0; q < 6; ++q) nh += __popc(sm.touched[t][q]);
-            atomicAdd(&hsum, nh);
+            atomicAdd(&sm.hsum, nh);
         }
         __syncthreads();
-        nh = hsum;
+        nh = sm.hsum;
     }
     if (t == 0) {
         if (nslot > MAXC) atomicOr(&st->err, CS3D_ERRBIT_CAND_OVERFLOW);
@@ -2062,8 +2199,8 @@ __device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned 
     }
 }
 
-// The marked cells of partial builds, then the other cells of instances that
-// are rebuilt whole.  A CTA looks at its cells 192 at a time, one to a thread.
+// The listed cells, then the other cells of the instances that nb_mark turned
+// to whole builds.
 __device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
 {
     const int t = threadIdx.x;
@@ -2071,20 +2208,22 @@ __device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
     const int node = __ldg(&d.topo.patch[t]);
     if (t == 0) sm.st_inst = -1;
     const int N = *d.n_build;
-    for (int q = blockIdx.x; q < N; q += gridDim.x) nb_cell(d, d.build[q], node, epoch, sm);
+    Dealer listed(&d.deal[DEAL_LISTS], sm.next);
+    while (listed.w < N) {
+        const int a = d.build[listed.w];
+        listed.draw();
+        nb_cell(d, a, node, epoch, sm);
+        listed.advance();
+    }
     const int W = d.flags[2] ? n_work(d) : 0;
-    for (int w0 = blockIdx.x; w0 < W; w0 += gridDim.x * SLOTS) {
-        __syncthreads();
-        if (t == 0) sm.ntodo = 0;
-        __syncthreads();
-        const int w = w0 + t * gridDim.x;
-        if (w < W) {
-            const int a = cell_of(d, w);
-            if (d.st[inst_of(d, a)].rebuild == 2 && !d.mark[a]) sm.todo[atomicAdd(&sm.ntodo, 1)] = a;
-        }
-        __syncthreads();
-        const int n = sm.ntodo;
-        for (int q = 0; q < n; ++q) nb_cell(d, sm.todo[q], node, epoch, sm);
+    __syncthreads();
+    Dealer other(&d.deal[DEAL_FULL], sm.next);
+    while (other.w < W) {
+        const int a = cell_of(d, other.w);
+        other.draw();
+        if (d.st[inst_of(d, a)].rebuild == 2 && !d.mark[a]) nb_cell(d, a, node, epoch, sm);   // uniform
+        else __syncthreads();
+        other.advance();
     }
     __syncthreads();
     if (t == 0) list_stats(d, sm);
@@ -2094,6 +2233,150 @@ __global__ void __launch_bounds__(SLOTS, 6) k_nb_lists(Dev d)
 {
     __shared__ ListSmem sm;
     if (d.flags[0]) nb_lists(d, sm);
+}
+
+// ---------------------------------------------------------------------------
+// Whole steps in one kernel (cooperative launch, all CTAs resident): the
+// phases of the launch sequence with grid barriers between them.  For small
+// systems, whose kernels are shorter than the gaps between launches: a step of
+// the sequence is 10 launches, most of which find nothing to do.
+// ---------------------------------------------------------------------------
+union StepsSmem {
+    S1Smem s1;
+    S2Smem s2;
+    ListSmem lists;
+    DivSmem div;
+    float com[3][SLOTS];
+};
+
+// Waits at most this many polls (about a microsecond each) for the other CTAs.
+constexpr unsigned SYNC_POLLS = 1u << 22;
+
+// Polls until *p >= v.  Relaxed loads: an acquiring one empties the SM's L1,
+// which the CTAs still at work beside this one need (S1 of 440 cells took 38 us
+// beside acquiring polls, 24 without).  False if the others did not come: the
+// CTA must return.  One thread.
+__device__ __forceinline__ bool poll_until(const Dev &d, const unsigned *p, unsigned v)
+{
+    for (unsigned polls = 0; polls < SYNC_POLLS; ++polls) {
+        unsigned u;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(u) : "l"(p) : "memory");
+        if (u >= v) {
+            __threadfence();
+            return true;
+        }
+        __nanosleep(20);
+    }
+    atomic_or_err(&d.st[0], CS3D_ERRBIT_SYNC);
+    return false;
+}
+
+// Barriers of the grid, every CTA in the same order.  b: barriers and serial
+// sections so far.
+struct GridBar {
+    unsigned arrived = 0, serials = 0;
+};
+
+__device__ __forceinline__ bool grid_sync(const Dev &d, GridBar &b)
+{
+    b.arrived += gridDim.x;
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&d.bar[0], 1u);
+        ok = poll_until(d, &d.bar[0], b.arrived);
+    }
+    return !__syncthreads_or(!ok);
+}
+
+// The same, with `serial` run by the last CTA to arrive (all its threads)
+// before the others go on.
+template <typename F>
+__device__ __forceinline__ bool grid_sync(const Dev &d, GridBar &b, F serial)
+{
+    __shared__ int last;
+    b.arrived += gridDim.x;
+    b.serials += 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&d.bar[0], 1u) == b.arrived - 1u;
+        if (last) __threadfence();
+    }
+    __syncthreads();
+    bool ok = true;
+    if (last) {
+        serial();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(&d.bar[1]), "r"(b.serials) : "memory");
+        }
+    } else if (threadIdx.x == 0) ok = poll_until(d, &d.bar[1], b.serials);
+    return !__syncthreads_or(!ok);
+}
+
+// n steps from the kicked state (X, V hold the first step's half kick and
+// drift); the first n_div of them test for division.  last: the call ends with
+// them (S2 mode 2 on the last one).  com: some instance corrects its
+// centre-of-mass motion, so that S2 leaves the kick to the phase that shifts
+// the nodes; far: some instance counts internal cells.
+__global__ void __launch_bounds__(SLOTS, 4) k_steps(Dev d, int par, int n, int n_div, int last, int com, int far)
+{
+    extern __shared__ __align__(16) unsigned char steps_raw[];
+    StepsSmem &sm = *reinterpret_cast<StepsSmem *>(steps_raw);
+    GridBar bar;
+    if (!grid_sync(d, bar, [&] { step_begin<SLOTS>(d, par ^ 1); })) return;
+    for (int k = 0; k < n; ++k, par ^= 1) {
+        const bool div = k < n_div, end = k + 1 == n;
+        const int fuse = com ? 0 : end && last ? 2 : 1;
+        const auto next = [&] { if (!end) step_begin<SLOTS>(d, par); };
+        if (d.flags[0]) {
+            nb_boxes(d);
+            if (!grid_sync(d, bar)) return;
+            nb_mark(d);
+            if (!grid_sync(d, bar)) return;
+            nb_lists(d, sm.lists);
+            if (!grid_sync(d, bar)) return;
+        }
+        s1_cells<false, true>(d, par, sm.s1);
+        if (!grid_sync(d, bar)) return;
+        if (div) s2_cells<true, true>(d, par, fuse, sm.s2);
+        else s2_cells<false, true>(d, par, fuse, sm.s2);
+        // the next step begins at the last barrier of this one
+        const auto centres = [&] {
+            for (int q = 0; q < d.n_inst; ++q) com_centre<SLOTS>(d, q, sm.com);
+        };
+        if (!grid_sync(d, bar, [&] {
+                if (d.flags[1]) return;
+                if (com) centres();
+                else next();
+            }))
+            return;
+        if (div && d.flags[1]) {
+            for (int q = blockIdx.x; q < d.n_inst; q += gridDim.x) div_select<SLOTS>(d, par, q, sm.div);
+            if (!grid_sync(d, bar)) return;
+            div_apply(d, par, sm.s2.xs, sm.s2.gs);
+            if (!grid_sync(d, bar)) return;
+            div_finish(d, par, far != 0, fuse != 0, sm.s2.smax);
+            if (!grid_sync(d, bar, [&] {
+                    if (com) centres();
+                    else next();
+                }))
+                return;
+        }
+        if (com) {
+            // a cell's shift and kick are its own CTA's
+            com_shift(d);
+            if (!end) {
+                __syncthreads();
+                const int W = n_work(d);
+                for (int w = blockIdx.x; w < W; w += gridDim.x) integrate_cell(d, cell_of(d, w), sm.s2.smax);
+            }
+            if (!grid_sync(d, bar, next)) return;
+        }
+    }
 }
 
 }  // namespace cs3d

@@ -53,6 +53,7 @@ extern "C" {
 #define CS3D_ERRBIT_HALO_OVERFLOW  0x100u  /* reserved, never raised */
 #define CS3D_ERRBIT_SOFT_CELLS     0x200u  /* more distinct softer cells requested than cell indices
                                               exist (the reference loops forever, src/GPUbounce.cu:1364-1384) */
+#define CS3D_ERRBIT_SYNC           0x400u  /* the blocks of a step kernel lost one another (never seen) */
 
 #define CS3D_MAX_CAND     128   /* contact-candidate cells per cell */
 #define CS3D_MAX_ENTRIES   64   /* contact-candidate nodes per node */

@@ -91,3 +91,42 @@ def test_list_build_around_a_large_cell(mesh, small, scale):
     assert np.array_equal(got, want)
     assert small == 0 or len(want) > 0
     sim.close()
+
+
+def _growing(n, **over):
+    """n cells close to each other; all of them divide in the first step (their volume is above the division volume)."""
+    st, box = _grid_state(n, spacing=2.25)
+    p = W.base_params(box_len=(box, box, box), div_time_steps=10 ** 9, rng_ij=11, rng_kl=1100)
+    p.update(over)
+    if p.get("correct_com"):
+        p["use_rigid_box"] = 0
+    return p, st
+
+
+@pytest.mark.parametrize("n,steps,over", [(1, 40, {}), (8, 300, {}), (20, 60, {"correct_com": 1}),
+                                          (20, 60, {"add_rands": 1, "rand_scale_factor": 0.1, "rand_seed": 5}),
+                                          (60, 40, {"count_internal_radius": 0.5}), (74, 12, {}), (75, 12, {}),
+                                          (148, 6, {"growth_rate": 0.0}), (149, 6, {"growth_rate": 0.0})])
+def test_steps_in_one_kernel_equal_the_launch_sequence(mesh, n, steps, over):
+    """A system small enough for the one-kernel path (alone) and the same
+    system beside another instance that makes the context too large for it:
+    states and events bit for bit, over sizes around the limit, divisions,
+    the options of a step and several launches."""
+    p, st = _growing(n, **over)
+    q, big = _growing(200, growth_rate=0.0)
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
+    got = []
+    for others in (0, 1):
+        ens = cs.Ensemble([p] + [q] * others, topo, [4 * n + 8] + [200] * others)
+        ens.load_state(0, st["X"], st["Y"], st["Z"], n_cells=n)
+        if others:
+            ens.load_state(1, big["X"], big["Y"], big["Z"], n_cells=200)
+        ens.step(steps - 1)
+        ens.step(1)
+        got.append((ens.state(0), ens.events(0), ens.forces(0), ens.cells(0), ens.far_counts(0)))
+        ens.close()
+    (a, ea, fa, ca, ra), (b, eb, fb, cb, rb) = got
+    assert a["n"] == b["n"] and np.array_equal(ea, eb) and np.array_equal(ra, rb)
+    for x, y in ((a, b), (fa, fb), (ca, cb)):
+        for k in x:
+            assert np.array_equal(x[k], y[k]), k
