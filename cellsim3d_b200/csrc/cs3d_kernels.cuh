@@ -192,11 +192,16 @@ __device__ __forceinline__ double sqrt_nr(double x)
 // difference of two angles near 2 rad whose float rounding alone (1.2e-7)
 // would exceed the 1e-5 relative force bar, so it is formed without
 // rounding theta.  u = cos(theta) (the reference's regularised ratio) is
-// formed in FP64; with c0, s0 = cos, sin of theta0 in FP64,
-//   sin(dth / 2) = (c0 - u) / (2 sin(theta0 + dth / 2)),   dth = theta - theta0.
-// A float estimate of dth from acosf is refined by one Newton step of this
-// equation in FP64 (sin/cos of dth/2 by their Taylor series, |dth/2| < 0.4
-// for |dth/2| up to ~1.2 rad), which leaves dth accurate to ~1e-12.
+// formed in FP64; with c0, s0 = cos, sin of theta0 in FP64 and
+// s = sin(theta) = sqrt(1 - u^2), dth = theta - theta0 has
+//   sin(dth) = s c0 - u s0,  cos(dth) = u c0 + s s0,  tan(dth / 2) = sin(dth) / (1 + cos(dth)),
+// and dth = 2 atan of that by a polynomial (Chebyshev interpolation of
+// atan(t) / t in t^2 up to 0.4, relative error 1.9e-12).  Beyond, at
+// |dth| > 1.13 rad, a float estimate of dth from acosf is refined by one
+// Newton step of sin(dth / 2) = (c0 - u) / (2 sin(theta0 + dth / 2)) in FP64
+// (sin/cos of dth/2 by their Taylor series); taken for all angles, that costs
+// S1 of 100,000 packed cells 1.68 ms against 1.53 (longer chains, and more
+// registers than the kernel has).
 __device__ __forceinline__ void sincos_small(double x, double &s, double &c)
 {
     const double x2 = x * x;
@@ -225,14 +230,9 @@ __device__ __forceinline__ Arm make_arm(const double3 &to, const double3 &from)
     return a;
 }
 
-// The angle between arms p and q: GetAngleForce(P, Q) (Fp) and
-// GetAngleForce(Q, P) (Fq).  |p||q| is the product of the two lengths, as the
-// reference forms it (sqrtf(ri_2) * sqrtf(rk_2)).
-__device__ __forceinline__ void angle_term(const Arm &p, const Arm &q, float th0f, double c0, double s0, double3 &Fp,
-                                           double3 &Fq)
+// theta - theta0 where it is large.
+__device__ __noinline__ double wide_angle(double u, float th0f, double c0, double s0)
 {
-    const double idk = p.x * q.x + p.y * q.y + p.z * q.z;
-    const double u = idk * rcp_nr(p.len * q.len + 1e-3);
     // float estimate, then one Newton step on g(h) = sin(h) sin(theta0 + h) - (c0 - u)/2, h = dth/2
     double h = 0.5 * (double)(acosf((float)u) - th0f);
     double sh, ch;
@@ -241,7 +241,34 @@ __device__ __forceinline__ void angle_term(const Arm &p, const Arm &q, float th0
     const double g = sh * s1 - 0.5 * (c0 - u);
     const double dg = ch * s1 + sh * c1t;                            // d/dh of sin(h) sin(theta0 + h)
     h -= g * rcp_nr(dg);
-    const double dth = 2.0 * h;
+    return 2.0 * h;
+}
+
+// The angle between arms p and q: GetAngleForce(P, Q) (Fp) and
+// GetAngleForce(Q, P) (Fq).  |p||q| is the product of the two lengths, as the
+// reference forms it (sqrtf(ri_2) * sqrtf(rk_2)).
+__device__ __forceinline__ void angle_term(const Arm &p, const Arm &q, float th0f, double c0, double s0, double3 &Fp,
+                                           double3 &Fq)
+{
+    const double idk = p.x * q.x + p.y * q.y + p.z * q.z;
+    const double u = idk * rcp_nr(p.len * q.len + 1e-3);
+    double dth;
+    const double v = 1.0 - u * u, s = v * rsqrt_nr(v);
+    const double t = (s * c0 - u * s0) * rcp_nr(1.0 + (u * c0 + s * s0));
+    const double z = t * t;
+    if (z <= 0.4) {
+        double q = -0.010709327812319008;
+        q = fma(q, z, 0.03360965597502365);
+        q = fma(q, z, -0.05672578427922923);
+        q = fma(q, z, 0.07437129908232694);
+        q = fma(q, z, -0.09048784092942751);
+        q = fma(q, z, 0.1110678238876255);
+        q = fma(q, z, -0.14285455109241751);
+        q = fma(q, z, 0.19999992038868686);
+        q = fma(q, z, -0.3333333323770785);
+        q = fma(q, z, 0.999999999998091);
+        dth = 2.0 * t * q;
+    } else dth = wide_angle(u, th0f, c0, s0);
     const double c1 = -rsqrt_nr(p.r2 * q.r2 - idk * idk + 1e-3);
     const double f = -1000.0 * c1 * dth;
     const double cp = idk * p.ir2, cq = idk * q.ir2;
@@ -254,7 +281,7 @@ __device__ __forceinline__ void angle_term(const Arm &p, const Arm &q, float th0
 struct SlotData {
     int cell[MAXC];
     float4 lo[MAXC], hi[MAXC];
-    short rlo[MAXC][3], rhi[MAXC][3];
+    int4 range[MAXC];   // lowest and highest bin as 16-bit numbers, low | high << 16, by axis
     float mn[3];
     int div[3];
 };
@@ -267,14 +294,14 @@ __device__ __forceinline__ void slots_load(const Dev &d, int a, const InstState 
     // read in full whatever the count, so that no load waits for another
     // (entries past the count are never used)
     if (t < MAXC) sd.cell[t] = d.cand[(size_t)a * MAXC + t];
-    if (t == 0) {
+    // thread 0 has the drawing of the next cell to do
+    if (t >= 160 && t < 163) {
+        const int q = t - 160;
         const int *mm = st->mm[par];
-        for (int q = 0; q < 3; ++q) {
-            float mn = fminf(o2f(mm[2 * q]), 1.0e8f);
-            float mx = fmaxf(o2f(mm[2 * q + 1]), -1.0e8f);
-            sd.mn[q] = mn;
-            sd.div[q] = grid_div(mn, mx);
-        }
+        float mn = fminf(o2f(mm[2 * q]), 1.0e8f);
+        float mx = fmaxf(o2f(mm[2 * q + 1]), -1.0e8f);
+        sd.mn[q] = mn;
+        sd.div[q] = grid_div(mn, mx);
     }
 }
 
@@ -288,9 +315,12 @@ __device__ __forceinline__ void slots_boxes(const Dev &d, const InstParams &P, i
         sd.lo[t] = lo;
         sd.hi[t] = hi;
         int st, en;
-        bin_range_axis(lo.x, hi.x, P.ra, sd.mn[0], sd.div[0], st, en); sd.rlo[t][0] = (short)st; sd.rhi[t][0] = (short)en;
-        bin_range_axis(lo.y, hi.y, P.ra, sd.mn[1], sd.div[1], st, en); sd.rlo[t][1] = (short)st; sd.rhi[t][1] = (short)en;
-        bin_range_axis(lo.z, hi.z, P.ra, sd.mn[2], sd.div[2], st, en); sd.rlo[t][2] = (short)st; sd.rhi[t][2] = (short)en;
+        int4 rg;
+        bin_range_axis(lo.x, hi.x, P.ra, sd.mn[0], sd.div[0], st, en); rg.x = (st & 0xffff) | en << 16;
+        bin_range_axis(lo.y, hi.y, P.ra, sd.mn[1], sd.div[1], st, en); rg.y = (st & 0xffff) | en << 16;
+        bin_range_axis(lo.z, hi.z, P.ra, sd.mn[2], sd.div[2], st, en); rg.z = (st & 0xffff) | en << 16;
+        rg.w = 0;
+        sd.range[t] = rg;
     }
 }
 
@@ -299,128 +329,148 @@ __device__ __forceinline__ void slots_boxes(const Dev &d, const InstParams &P, i
 // lies in the slot cell's stale insertion range (the cell is in the node's
 // bin list, src/propagatebound.cu:209-256) and the node is within the
 // cut-off of the slot cell's stale box (src/propagate.cu:382-392).
-struct SlotPred {
-    int cur;
-    bool ok;
-    int nb0, nb1, nb2;
+struct NodeBins {
+    int b0, b1, b2;   // the node's stale grid bin
 };
 
-__device__ __forceinline__ void pred_init(SlotPred &sp, const SlotData &sd, float3 x)
+__device__ __forceinline__ NodeBins node_bins(const SlotData &sd, float3 x)
 {
-    sp.cur = -1;
-    sp.ok = false;
-    sp.nb0 = node_bin_axis(x.x, sd.mn[0], sd.div[0]);
-    sp.nb1 = node_bin_axis(x.y, sd.mn[1], sd.div[1]);
-    sp.nb2 = node_bin_axis(x.z, sd.mn[2], sd.div[2]);
+    return {node_bin_axis(x.x, sd.mn[0], sd.div[0]), node_bin_axis(x.y, sd.mn[1], sd.div[1]),
+            node_bin_axis(x.z, sd.mn[2], sd.div[2])};
 }
 
-__device__ __forceinline__ bool pred_ok(SlotPred &sp, const SlotData &sd, const InstParams &P, float3 x, int s)
+__device__ __forceinline__ bool slot_ok(const SlotData &sd, const InstParams &P, float3 x, NodeBins nb, int s)
 {
-    if (s != sp.cur) {
-        sp.cur = s;
-        sp.ok = sp.nb0 >= sd.rlo[s][0] && sp.nb0 <= sd.rhi[s][0] && sp.nb1 >= sd.rlo[s][1] &&
-                sp.nb1 <= sd.rhi[s][1] && sp.nb2 >= sd.rlo[s][2] && sp.nb2 <= sd.rhi[s][2] &&
-                aabb_keep(sd.lo[s], sd.hi[s], x.x, x.y, x.z, P.ra2);
-    }
-    return sp.ok;
+    const int4 g = sd.range[s];
+    return nb.b0 >= (short)g.x && nb.b0 <= g.x >> 16 && nb.b1 >= (short)g.y && nb.b1 <= g.y >> 16 &&
+           nb.b2 >= (short)g.z && nb.b2 <= g.z >> 16 && aabb_keep(sd.lo[s], sd.hi[s], x.x, x.y, x.z, P.ra2);
 }
-
-constexpr int EPRE = 8;  // entries prefetched per node at the start of a cell
-constexpr int SB = 4;    // entries whose partner loads are in flight together
-static_assert(EPRE == 2 * SB && SB == 4, "the sweep's entry window is two batches of four entries");
 
 // ---------------------------------------------------------------------------
-// S1 contact sweep of node i over its entries: conservative contact force
-// (strict cut-off, src/propagate.cu:406-442) added to F, sum of the velocity
-// differences v_i - v_j of the dissipative pairs (non-strict cut-off,
+// The contact sweep of S1 shares a warp's entries among its lanes.  A node has
+// one or two entries on average and the nodes next to another cell five to
+// forty: with a lane walking its own node's entries, a warp took as many
+// rounds as its busiest node has entries and most lanes waited.  Here the
+// entries of the warp's 32 nodes (eight of each node at a time, the first of
+// every node, then the second, ...) are laid out back to back, a round takes
+// 32 of them, one to a lane, and the owners then add up the results of their
+// entries in entry order, so that a node's sums do not depend on the sharing.
+// An owner seldom has more than two entries in a round.  S1 of 100,000 packed
+// cells 2.01 -> 1.86 ms, of 3000 growing ones 97 -> 85 us (with an owner's
+// entries side by side, up to 32 to a round, 1.89 ms and 95 us); S2's sweep,
+// two loads and three additions a pair, is slower this way (0.62 -> 0.65 ms).
+// ---------------------------------------------------------------------------
+constexpr int EPRE = 8;    // entries of a node laid out at a time
+
+struct alignas(16) SweepSmem {
+    double res[6][32];           // results of a round: force, velocity difference
+    uint32_t item[EPRE * 32];    // owner lane << 16 | slot << 8 | node
+    unsigned own[32];            // results of the round that are the node's
+};
+
+// S1 contact sweep of the warp's nodes (i: this lane's): conservative contact
+// force (strict cut-off, src/propagate.cu:406-442) added to F, sum of the
+// velocity differences v_i - v_j of the dissipative pairs (non-strict cut-off,
 // src/propagate.cu:600-656) in vsum (its tangential part is taken once, by
 // tangential()).  Lists the dissipative pairs for S2 (positions do not change
 // before S2) and returns their number.
 // Partner positions and velocities are read from global memory (L1/L2
 // resident: the partners of a cell are a few hundred nodes).
-// ---------------------------------------------------------------------------
 template <bool COOP>
-__device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const SlotData &sd, int a, int i, float3 x,
-                                        float3 v, int ne, const uint32_t (&pre)[EPRE / 2], double &FX,
+__device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const SlotData &sd, SweepSmem &ss, int a,
+                                        int i, float3 x, float3 v, int ne, const uint32_t (&pre)[EPRE / 2], double &FX,
                                         double &FY, double &FZ, double3 &vsum)
 {
+    const int lane = i & 31;
+    const int most = __reduce_max_sync(0xffffffffu, ne);
+    if (most == 0) return 0;   // uniform in the warp
     const uint16_t *ep = d.ent + (size_t)a * MAXE * SLOTS + i;
     uint16_t *dl = d.dlist + (size_t)a * MAXD * SLOTS + i;
-    SlotPred sp;
-    pred_init(sp, sd, x);
+    const NodeBins nb = node_bins(sd, x);
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t w[EPRE / 2] = {pre[0], pre[1], pre[2], pre[3]};
     int nd = 0;
-    // a window of two batches of entries in registers (two per word): the
-    // current batch, and the next one, loaded a batch ahead
-    uint32_t w0 = pre[0], w1 = pre[1], w2 = pre[2], w3 = pre[3];
-    for (int k0 = 0; k0 < ne; k0 += SB) {
-        unsigned e[SB];
-        e[0] = w0 & 0xffffu;
-        e[1] = k0 + 1 < ne ? (w0 >> 16) : 0xffffu;
-        e[2] = k0 + 2 < ne ? (w1 & 0xffffu) : 0xffffu;
-        e[3] = k0 + 3 < ne ? (w1 >> 16) : 0xffffu;
-        w0 = w2;
-        w1 = w3;
-        {
-            const int kn = k0 + 2 * SB;
-            unsigned f[SB];
+    ss.own[lane] = 0u;
+    for (int k0 = 0; k0 < most; k0 += EPRE) {
+        int m = 0;
 #pragma unroll
-            for (int q = 0; q < SB; ++q) f[q] = kn + q < ne ? ep[(size_t)(kn + q) * SLOTS] : 0xffffu;
-            w2 = f[0] | (f[1] << 16);
-            w3 = f[2] | (f[3] << 16);
+        for (int k = 0; k < EPRE; ++k) {
+            const bool has = k0 + k < ne;
+            const unsigned b = __ballot_sync(0xffffffffu, has);
+            if (has)
+                ss.item[m + __popc(b & below)] = (unsigned)lane << 16 | (k & 1 ? w[k / 2] >> 16 : w[k / 2] & 0xffffu);
+            m += __popc(b);
         }
-        int id[SB];
+        __syncwarp();
+        // the next eight, in flight during the rounds
 #pragma unroll
-        for (int q = 0; q < SB; ++q) {
-            id[q] = -1;
-            if (e[q] != 0xffffu && pred_ok(sp, sd, P, x, (int)(e[q] >> 8)))
-                id[q] = sd.cell[e[q] >> 8] * SLOTS + (int)(e[q] & 255u);
+        for (int k = 0; k < EPRE; ++k) {
+            const int q = k0 + EPRE + k;
+            const unsigned e = q < ne ? ep[(size_t)q * SLOTS] : 0u;
+            w[k / 2] = k & 1 ? w[k / 2] | e << 16 : e;
         }
-        float4 xj[SB];
-#pragma unroll
-        for (int q = 0; q < SB; ++q) xj[q] = id[q] >= 0 ? ld_partner<COOP>(&d.X[id[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int q = 0; q < SB; ++q) {
-            if (id[q] < 0) continue;
-            const float dx = __fsub_rn(x.x, xj[q].x), dy = __fsub_rn(x.y, xj[q].y), dz = __fsub_rn(x.z, xj[q].z);
-            const float r2 = r2_ref(dx, dy, dz);
-            if (r2 > P.ra2) { id[q] = -1; continue; }
-            if (nd < MAXD) dl[(size_t)nd * SLOTS] = (uint16_t)e[q];
-            ++nd;
-            if (d.record_pairs) {
-                const unsigned long long slot = atomicAdd(d.n_pairs, 1ull);
-                if ((long long)slot < d.pair_cap)
-                    d.pairs[slot] = make_int4((a << 8) | i, ((id[q] / SLOTS) << 8) | (id[q] % SLOTS),
-                                              r2 < P.ra2 ? 3 : 2, 0);
+        for (int b = 0; b < m; b += 32) {
+            const bool act = b + lane < m;
+            const unsigned it = act ? ss.item[b + lane] : (unsigned)lane << 16;
+            const int o = it >> 16, s = (it >> 8) & 255u, j = it & 255u;
+            const float3 xo = make_float3(__shfl_sync(0xffffffffu, x.x, o), __shfl_sync(0xffffffffu, x.y, o),
+                                          __shfl_sync(0xffffffffu, x.z, o));
+            const float3 vo = make_float3(__shfl_sync(0xffffffffu, v.x, o), __shfl_sync(0xffffffffu, v.y, o),
+                                          __shfl_sync(0xffffffffu, v.z, o));
+            const NodeBins no = {__shfl_sync(0xffffffffu, nb.b0, o), __shfl_sync(0xffffffffu, nb.b1, o),
+                                 __shfl_sync(0xffffffffu, nb.b2, o)};
+            bool pass = act && slot_ok(sd, P, xo, no, s);
+            const int id = pass ? sd.cell[s] * SLOTS + j : 0;
+            float4 xj = make_float4(0.f, 0.f, 0.f, 0.f), vj = xj;
+            if (pass) {
+                xj = ld_partner<COOP>(&d.X[id]);
+                vj = ld_partner<COOP>(&d.V[id]);
             }
-            if (r2 < P.ra2) {
+            const float r2 = r2_ref(__fsub_rn(xo.x, xj.x), __fsub_rn(xo.y, xj.y), __fsub_rn(xo.z, xj.z));
+            pass = pass && !(r2 > P.ra2);
+            if (pass) {
+                atomicOr(&ss.own[o], 1u << lane);
+                if (d.record_pairs) {
+                    const unsigned long long slot = atomicAdd(d.n_pairs, 1ull);
+                    if ((long long)slot < d.pair_cap)
+                        d.pairs[slot] = make_int4((a << 8) | (i - lane + o), ((id / SLOTS) << 8) | (id % SLOTS),
+                                                  r2 < P.ra2 ? 3 : 2, 0);
+                }
                 // distance in FP64 from the exact difference of the float
                 // positions: (rr - R) cancels for stiff repulsion
-                const double ex = (double)x.x - xj[q].x, ey = (double)x.y - xj[q].y, ez = (double)x.z - xj[q].z;
+                const double ex = (double)xo.x - xj.x, ey = (double)xo.y - xj.y, ez = (double)xo.z - xj.z;
                 const double R2 = ex * ex + ey * ey + ez * ez;
                 const double iR = rsqrt_nr(R2);
                 const double R = R2 * iR;
                 double k = 0.0;
-                if (R < (double)P.ra) k += -(double)P.asE * ((double)P.ra - R) * iR;
-                if (R <= (double)P.rr) k += (double)P.rsE * ((double)P.rr - R) * iR;
-                FX += k * ex;
-                FY += k * ey;
-                FZ += k * ez;
+                if (r2 < P.ra2) {
+                    if (R < (double)P.ra) k += -(double)P.asE * ((double)P.ra - R) * iR;
+                    if (R <= (double)P.rr) k += (double)P.rsE * ((double)P.rr - R) * iR;
+                }
+                ss.res[0][lane] = k * ex; ss.res[1][lane] = k * ey; ss.res[2][lane] = k * ez;
+                // velocity differences of floats are exact in FP64
+                ss.res[3][lane] = (double)vo.x - vj.x;
+                ss.res[4][lane] = (double)vo.y - vj.y;
+                ss.res[5][lane] = (double)vo.z - vj.z;
             }
-        }
-        float4 vj[SB];
-#pragma unroll
-        for (int q = 0; q < SB; ++q) vj[q] = id[q] >= 0 ? ld_partner<COOP>(&d.V[id[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int q = 0; q < SB; ++q) {
-            if (id[q] < 0) continue;
-            // velocity differences of floats are exact in FP64
-            vsum.x += (double)v.x - vj[q].x;
-            vsum.y += (double)v.y - vj[q].y;
-            vsum.z += (double)v.z - vj[q].z;
+            __syncwarp();
+            unsigned mine = ss.own[lane];
+            ss.own[lane] = 0u;
+            while (mine) {
+                const int q = __ffs(mine) - 1;
+                mine &= mine - 1u;
+                if (nd < MAXD) dl[(size_t)nd * SLOTS] = (uint16_t)ss.item[b + q];
+                ++nd;
+                FX += ss.res[0][q]; FY += ss.res[1][q]; FZ += ss.res[2][q];
+                vsum.x += ss.res[3][q]; vsum.y += ss.res[4][q]; vsum.z += ss.res[5][q];
+            }
+            __syncwarp();
         }
     }
     return nd;
 }
+
+constexpr int SB = 4;      // pairs whose partner loads are in flight together
 
 // S2 sweep: sum of the velocity differences over the dissipative pairs found
 // by S1 (their list, in column layout), with the velocities after the half
@@ -839,10 +889,26 @@ struct ArmForces {
     double x[SLOTS * 3], y[SLOTS * 3], z[SLOTS * 3];
 };
 
+// The next cell's nodes and first entries towards L2: a system of more than
+// some 20,000 cells does not stay there between steps.  With the bins of a
+// node by multiplication (div_dl), a candidate's bin range in one word an
+// axis and the cell's set-up spread over the warps: S1 of 100,000 packed
+// cells 1.86 -> 1.68 ms, of 3000 growing ones 85 -> 80 us.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_cell(const Dev &d, int a)
+{
+    const int t = threadIdx.x;
+    constexpr int LINES = SLOTS * 16 / 128;   // a cell's positions, and as much of its entries (8 a node)
+    if (t < LINES) prefetch_l2((const char *)(d.X + (size_t)a * SLOTS) + 128 * t);
+    else if (t < 2 * LINES) prefetch_l2((const char *)(d.V + (size_t)a * SLOTS) + 128 * (t - LINES));
+    else if (t < 3 * LINES) prefetch_l2((const char *)(d.ent + (size_t)a * MAXE * SLOTS) + 128 * (t - 2 * LINES));
+}
+
 struct S1Smem {
     double3 xd[SLOTS];   // FP64 copies of the positions and velocities: the
     double3 vd[SLOTS];   // FP64 terms read them without conversions
     SlotData sd;
+    SweepSmem sweep[SLOTS / 32];
     ArmForces arm;
     float press;         // the cell's pressure of this step
     int next[2];
@@ -875,7 +941,7 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         sm.xd[i] = make_double3(x4.x, x4.y, x4.z);
         sm.vd[i] = make_double3(v4.x, v4.y, v4.z);
         slots_load(d, a, &d.st[inst], par, sm.sd);
-        if (i == 0) {
+        if (i == 128) {
             // this step's PressureUpdate (none before the initial forces)
             const float pr = INIT ? d.press[a] : pressure_update(d, P, a, d.st[inst].step);
             if (!INIT) d.press[a] = pr;
@@ -883,6 +949,8 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         }
         __syncthreads();
         slots_boxes(d, P, par, sm.sd, nc);
+        const int wn = sm.next[deal.turn];
+        if (wn < W) prefetch_cell(d, cell_of(d, wn));
         const float3 x = f3(x4);
         const float3 v = f3(v4);
         // bond angles: thread = vertex, three angles each
@@ -905,6 +973,10 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
             sm.arm.x[o + 2] = F12q.x + F02q.x; sm.arm.y[o + 2] = F12q.y + F02q.y; sm.arm.z[o + 2] = F12q.z + F02q.z;
         }
         __syncthreads();
+        double CX = 0.0, CY = 0.0, CZ = 0.0;
+        double3 vsum = make_double3(0.0, 0.0, 0.0);
+        // contacts, src/propagate.cu:356-442 and the first dissipative sweep
+        const int nd = sweep_s1<COOP>(d, P, sm.sd, sm.sweep[i >> 5], a, i, x, v, ne, pre, CX, CY, CZ, vsum);
         if (i < NODES) {
             // The node force is accumulated in FP64: its terms (pressure up
             // to ~1e3, stiff contact repulsion up to ~1e4) can cancel to a
@@ -943,9 +1015,9 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
                 FY += sm.arm.y[am.x] + sm.arm.y[am.y] + sm.arm.y[am.z] - (sm.arm.y[o] + sm.arm.y[o + 1] + sm.arm.y[o + 2]);
                 FZ += sm.arm.z[am.x] + sm.arm.z[am.y] + sm.arm.z[am.z] - (sm.arm.z[o] + sm.arm.z[o + 1] + sm.arm.z[o + 2]);
             }
-            // contacts, src/propagate.cu:356-442 and the first dissipative sweep
-            double3 vsum = make_double3(0.0, 0.0, 0.0);
-            const int nd = sweep_s1<COOP>(d, P, sm.sd, a, i, x, v, ne, pre, FX, FY, FZ, vsum);
+            FX += CX;
+            FY += CY;
+            FZ += CZ;
             const double3 vt = tangential(sm.xd, n0, n1, n2, sgn, vsum);
             if (nd > MAXD) atomic_or_err(&d.st[inst], CS3D_ERRBIT_ENTRY_OVERFLOW);
             // rigid box walls, src/propagate.cu:474-510 (float gap tests)
@@ -1009,7 +1081,6 @@ struct S2Smem {
     float4 xs[SLOTS];
     float4 vs[SLOTS];
     int cell[MAXC];
-
     GeomScratch gs;
     int dflag;   // the cell divides (division steps)
     float smax[SLOTS / 32];
@@ -1092,8 +1163,7 @@ __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, 
 
         float3 fdk = make_float3(0.f, 0.f, 0.f);
         if (i < NODES) {
-            const float3 v = f3(v4);
-            const double3 vt = tangential(sm.xs, n0, n1, n2, sgn, sweep_s2<COOP>(d, sm.cell, a, i, v, nd));
+            const double3 vt = tangential(sm.xs, n0, n1, n2, sgn, sweep_s2<COOP>(d, sm.cell, a, i, f3(v4), nd));
             const float3 fd = dis_force(P, sm.vs, i, n0, n1, n2, vt);
 
             d.FD[g] = make_float4(fd.x, fd.y, fd.z, 0.f);

@@ -130,3 +130,47 @@ def test_steps_in_one_kernel_equal_the_launch_sequence(mesh, n, steps, over):
     for x, y in ((a, b), (fa, fb), (ca, cb)):
         for k in x:
             assert np.array_equal(x[k], y[k]), k
+
+
+def _pack(x):
+    st = {"n": len(x)}
+    for q, key in enumerate("XYZ"):
+        a = np.zeros((len(x), 192), np.float32)
+        a[:, :180] = x[..., q]
+        st[key] = a.reshape(-1)
+    return st
+
+
+def _distorted(mesh, noise):
+    """The mesh at rest and three copies with random displacements of their nodes."""
+    rng = np.random.default_rng(17)
+    xyz = W.centred(W.scaled_xyz(mesh)).astype(np.float64)
+    x = np.stack([xyz] + [xyz + rng.normal(0, noise, xyz.shape) + [4.0 * (k + 1), 0, 0] for k in range(3)]) + 5.0
+    return _pack(x.astype(np.float32))
+
+
+def _crowded(mesh, flat):
+    """The mesh at rest and a pair of flattened copies face to face."""
+    rng = np.random.default_rng(19)
+    xyz = W.centred(W.scaled_xyz(mesh)).astype(np.float64)
+    a = xyz * [1.0, 1.0, flat] + rng.normal(0, 1e-3, xyz.shape)
+    b = a[:, [1, 0, 2]] + [0.03, 0.02, a[:, 2].max() - a[:, 2].min() + 0.15]
+    return _pack((np.stack([xyz + [6.0, 0, 0], a, b]) + 3.0).astype(np.float32))
+
+
+@pytest.mark.parametrize("make,arg", [(_distorted, 0.01), (_distorted, 0.06), (_distorted, 0.12),
+                                      (_crowded, 1.0), (_crowded, 0.3), (_crowded, 0.1)])
+def test_forces_of_bent_and_crowded_cells(mesh, make, arg):
+    """Initial forces and contact pairs against the FP64 oracle, where bond
+    angles lie on both sides of the polynomial's range (distorted cells) and
+    where nodes have from none to several groups of eight entries (flattened
+    cells face to face)."""
+    from parity import TOL, force_errors, make_pair, sorted_pairs
+    st = make(mesh, arg)
+    p = W.base_params(box_len=(60.0, 60.0, 60.0), growth_rate=0.0, use_rigid_box=0)
+    sim, orc = make_pair(p, st, mesh, capacity=st["n"])
+    ec, ed = force_errors(sim, orc)
+    assert ec[0] < TOL and ed[0] < TOL, (ec, ed)
+    for kind in (0, 1):
+        assert np.array_equal(sorted_pairs(sim.pairs(kind)), sorted_pairs(orc.recorded_pairs(kind)))
+    sim.close()
