@@ -115,6 +115,7 @@ struct TopoTables {
     uint4 arm[SLOTS];
     uint8_t faces[CS3D_FACES * 7];
     uint8_t patch[SLOTS];
+    uint32_t tri[CS3D_FACES * 6];
     double2 cs0[3 * SLOTS];
     double r0i[3 * SLOTS];
 };
@@ -194,6 +195,10 @@ int topo_tables(const cs3d_topology *t, TopoTables &o)
         if (t->faces[f] < 0 || t->faces[f] >= NODES) return CS3D_E_ARG;
         o.faces[f] = (uint8_t)t->faces[f];
     }
+    for (int k = 0; k < CS3D_FACES * 6; ++k) {
+        const uint8_t *F = o.faces + 7 * (k / 6) + k % 6;
+        o.tri[k] = F[0] | F[1] << 8 | (k / 6) << 16;
+    }
     node_patches(t, o.patch);
     return CS3D_OK;
 }
@@ -212,6 +217,7 @@ int upload_topology(cs3d_ctx *c, const cs3d_topology *t)
     if ((rc = dalloc(c, &T.arm, SLOTS))) return rc;
     if ((rc = dalloc(c, &T.faces, CS3D_FACES * 7))) return rc;
     if ((rc = dalloc(c, &T.patch, SLOTS))) return rc;
+    if ((rc = dalloc(c, &T.tri, CS3D_FACES * 6))) return rc;
     CK(cudaMemcpyAsync(T.cs0, tt.cs0, sizeof tt.cs0, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.r0i, tt.r0i, sizeof tt.r0i, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.nnpack, tt.nnp, sizeof tt.nnp, cudaMemcpyHostToDevice, c->stream));
@@ -220,6 +226,7 @@ int upload_topology(cs3d_ctx *c, const cs3d_topology *t)
     CK(cudaMemcpyAsync(T.arm, tt.arm, sizeof tt.arm, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.faces, tt.faces, sizeof tt.faces, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(T.patch, tt.patch, sizeof tt.patch, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(T.tri, tt.tri, sizeof tt.tri, cudaMemcpyHostToDevice, c->stream));
     // the host tables go out of scope: the copies must have completed
     CK(cudaStreamSynchronize(c->stream));
     return CS3D_OK;

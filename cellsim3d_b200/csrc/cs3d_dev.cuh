@@ -91,6 +91,7 @@ struct Topo {
     double *r0i;        // [192*3] 1/R0 in FP64
     uint4 *arm;         // [192] x, y, z: arm-force index n*3 + k for the three neighbours n
     uint8_t *faces;     // [92*7]
+    uint32_t *tri;      // [92*6] triangles of the faces: v0 | v1 << 8 | face << 16
     uint8_t *patch;     // [192] node of each thread: 30 neighbouring nodes to a warp (0xff: none)
 };
 

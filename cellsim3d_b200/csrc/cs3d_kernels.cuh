@@ -35,6 +35,19 @@ __device__ __forceinline__ T warp_sum(T v)
     return v;
 }
 
+__device__ __forceinline__ float warp_min(float v)
+{
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 __device__ __forceinline__ void atomic_or_err(InstState *st, unsigned bits) { atomicOr(&st->err, bits); }
 
 // Block-wide exclusive scan (NT threads, NT a multiple of 32); wsum[32].
@@ -595,7 +608,7 @@ __device__ __forceinline__ void integrate_cell(const Dev &d, int a, float *smax)
             d.X[g] = xn;
             d.V[g] = v;
         }
-        for (int o = 16; o > 0; o >>= 1) disp = fmaxf(disp, __shfl_xor_sync(0xffffffffu, disp, o));
+        disp = warp_max(disp);
         if ((i & 31) == 0) smax[i >> 5] = disp;
         __syncthreads();
         if (i == 0) {
@@ -783,56 +796,73 @@ struct GeomScratch {
     double fc[CS3D_FACES][3];   // face centres relative to the cell's centre of mass
 };
 
-// Centre of mass (FP64 sum, src/centermass.cu:8-50) and bounding box
-// (src/propagatebound.cu:10-141) of the cell staged in xs.
-__device__ __forceinline__ void cell_geom(const float4 *xs, GeomScratch &gs, float3 &cm, float4 &lo, float4 &hi)
+// t / 180, correctly rounded as div_m.
+__device__ __forceinline__ double div_nodes(double t)
 {
-    int i = threadIdx.x, w = i >> 5, l = i & 31;
-    double sx = 0, sy = 0, sz = 0;
-    float mnx = 1e30f, mny = 1e30f, mnz = 1e30f, mxx = -1e30f, mxy = -1e30f, mxz = -1e30f;
-    if (i < NODES) {
-        float4 p = xs[i];
-        sx = p.x; sy = p.y; sz = p.z;
-        mnx = mxx = p.x; mny = mxy = p.y; mnz = mxz = p.z;
-    }
-    sx = warp_sum(sx); sy = warp_sum(sy); sz = warp_sum(sz);
-    for (int o = 16; o > 0; o >>= 1) {
-        mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-        mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-        mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
-        mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-        mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-        mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
-    }
+    constexpr double r = 1.0 / NODES;
+    const double q = t * r;
+    return fma(fma(-q, (double)NODES, t), r, q);
+}
+
+// Centre of mass (FP64 sum, src/centermass.cu:8-50) and bounding box
+// (src/propagatebound.cu:10-141) of the cell staged in xs: first the warps'
+// sums and extents, then, after the barrier, whoever needs them adds them up.
+__device__ __forceinline__ void cell_geom(const float4 *xs, GeomScratch &gs)
+{
+    const int i = threadIdx.x, w = i >> 5, l = i & 31;
+    const bool real = i < NODES;
+    const float4 p = xs[real ? i : 0];
+    const double sx = warp_sum(real ? (double)p.x : 0.0), sy = warp_sum(real ? (double)p.y : 0.0),
+                 sz = warp_sum(real ? (double)p.z : 0.0);
+    const float mnx = warp_min(p.x), mny = warp_min(p.y), mnz = warp_min(p.z);
+    const float mxx = warp_max(p.x), mxy = warp_max(p.y), mxz = warp_max(p.z);
     if (l == 0) {
         gs.sum[w][0] = sx; gs.sum[w][1] = sy; gs.sum[w][2] = sz;
         gs.mn[w][0] = mnx; gs.mn[w][1] = mny; gs.mn[w][2] = mnz;
         gs.mx[w][0] = mxx; gs.mx[w][1] = mxy; gs.mx[w][2] = mxz;
     }
     __syncthreads();
+}
+
+__device__ __forceinline__ float3 geom_centre(const GeomScratch &gs)
+{
     double tx = 0, ty = 0, tz = 0;
-    float a0 = 1e30f, a1 = 1e30f, a2 = 1e30f, b0 = -1e30f, b1 = -1e30f, b2 = -1e30f;
+    for (int q = 0; q < SLOTS / 32; ++q) { tx += gs.sum[q][0]; ty += gs.sum[q][1]; tz += gs.sum[q][2]; }
+    return make_float3((float)div_nodes(tx), (float)div_nodes(ty), (float)div_nodes(tz));
+}
+
+__device__ __forceinline__ void geom_box(const GeomScratch &gs, float4 &lo, float4 &hi)
+{
+    lo = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
+    hi = make_float4(-1e30f, -1e30f, -1e30f, 0.0f);
     for (int q = 0; q < SLOTS / 32; ++q) {
-        tx += gs.sum[q][0]; ty += gs.sum[q][1]; tz += gs.sum[q][2];
-        a0 = fminf(a0, gs.mn[q][0]); a1 = fminf(a1, gs.mn[q][1]); a2 = fminf(a2, gs.mn[q][2]);
-        b0 = fmaxf(b0, gs.mx[q][0]); b1 = fmaxf(b1, gs.mx[q][1]); b2 = fmaxf(b2, gs.mx[q][2]);
+        lo.x = fminf(lo.x, gs.mn[q][0]); lo.y = fminf(lo.y, gs.mn[q][1]); lo.z = fminf(lo.z, gs.mn[q][2]);
+        hi.x = fmaxf(hi.x, gs.mx[q][0]); hi.y = fmaxf(hi.y, gs.mx[q][1]); hi.z = fmaxf(hi.z, gs.mx[q][2]);
     }
-    cm = make_float3((float)(tx / 180.0), (float)(ty / 180.0), (float)(tz / 180.0));
-    lo = make_float4(a0, a1, a2, 0.0f);
-    hi = make_float4(b0, b1, b2, 0.0f);
+}
+
+// sqrt(x) to within an ulp or so (0 for x below 1e-280, where no triangle of a
+// cell is): the approximate inverse root refined once, then Heron's step.
+__device__ __forceinline__ double sqrt_full(double x)
+{
+    const double r = rsqrt_nr(x), s = x * r;
+    return x > 1e-280 ? fma(0.5 * r, fma(-s, s, x), s) : 0.0;
 }
 
 // Volume, area and the division test, src/volume.cu:5-163, in FP64.  Each
 // face (12 pentagons, 80 hexagons, vertices relative to the cell's centre of
 // mass) is cut into triangles at its vertex average; the volume is the sum
 // of |det| / 6 of the tetrahedra (centre of mass, triangle) and the area the
-// sum of the triangle areas.  The face centres first (one thread per face),
-// then the 552 triangles dealt out to all threads.
-__device__ __noinline__ void cell_volume(const uint8_t *faces, const float4 *xs, float3 cm, GeomScratch &gs, bool sph,
+// sum of the triangle areas.  The face centres first (one thread per face)
+// , then the 552 triangles dealt out to all threads.
+__device__ __noinline__ void cell_volume(const uint8_t *faces, const uint32_t *tris, const float4 *xs, float3 cm, GeomScratch &gs, bool sph,
                                          double &vol, double &area)
 {
     const int t = threadIdx.x, w = t >> 5, l = t & 31;
     const double cx = cm.x, cy = cm.y, cz = cm.z;
+    uint32_t tri[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) tri[k] = t + k * SLOTS < CS3D_FACES * 6 ? __ldg(&tris[t + k * SLOTS]) : 0u;
     if (t < CS3D_FACES) {
         const uint8_t *F = faces + 7 * t;
         double ax = 0, ay = 0, az = 0;
@@ -850,10 +880,11 @@ __device__ __noinline__ void cell_volume(const uint8_t *faces, const float4 *xs,
     }
     __syncthreads();
     double tv = 0, fa = 0;
-    for (int k = t; k < CS3D_FACES * 6; k += SLOTS) {
-        const int f = k / 6, q = k - 6 * f;
-        const uint8_t *F = faces + 7 * f;
-        const float4 p0 = xs[F[q]], p1 = xs[F[q + 1]];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (t + k * SLOTS >= CS3D_FACES * 6) break;
+        const float4 p0 = xs[tri[k] & 255u], p1 = xs[(tri[k] >> 8) & 255u];
+        const int f = tri[k] >> 16;
         const double x0 = (double)p0.x - cx, y0 = (double)p0.y - cy, z0 = (double)p0.z - cz;
         const double x1 = (double)p1.x - cx, y1 = (double)p1.y - cy, z1 = (double)p1.z - cz;
         const double ax = gs.fc[f][0], ay = gs.fc[f][1], az = gs.fc[f][2];
@@ -865,7 +896,7 @@ __device__ __noinline__ void cell_volume(const uint8_t *faces, const float4 *xs,
             const double u1 = x0 - ax, v1 = y0 - ay, w1 = z0 - az;
             const double u2 = x1 - ax, v2 = y1 - ay, w2 = z1 - az;
             const double xx = v1 * w2 - w1 * v2, yy = w1 * u2 - u1 * w2, zz = u1 * v2 - v1 * u2;
-            fa += 0.5 * sqrt(xx * xx + yy * yy + zz * zz);
+            fa += 0.5 * sqrt_full(xx * xx + yy * yy + zz * zz);
         }
     }
     tv = warp_sum(tv);
@@ -1126,6 +1157,16 @@ __device__ __forceinline__ void flush_mm(const Dev &d, int inst, int pn, const f
     }
 }
 
+__device__ __forceinline__ void prefetch_cell_s2(const Dev &d, int a)
+{
+    const int t = threadIdx.x;
+    constexpr int LINES = SLOTS * 16 / 128;
+    const size_t o = (size_t)a * SLOTS;
+    const float4 *p = t < LINES ? d.X + o : t < 2 * LINES ? d.Vb + o : t < 3 * LINES ? d.FC + o : d.Xb + o;
+    if (t < 4 * LINES) prefetch_l2((const char *)p + 128 * (t % LINES));
+    else if (t < 4 * LINES + 12) prefetch_l2((const char *)(d.dlist + o * MAXD) + 128 * (t - 4 * LINES));
+}
+
 // FUSE: the first half kick and drift of the next step (k_integrate) are
 // done here, on the force and velocity in registers: FUSE 1 when the next
 // step follows in the same launch sequence, FUSE 2 on the last step of a
@@ -1166,33 +1207,39 @@ __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, 
             const double3 vt = tangential(sm.xs, n0, n1, n2, sgn, sweep_s2<COOP>(d, sm.cell, a, i, f3(v4), nd));
             const float3 fd = dis_force(P, sm.vs, i, n0, n1, n2, vt);
 
-            d.FD[g] = make_float4(fd.x, fd.y, fd.z, 0.f);
+            // between fused steps only the two cells of a division still need
+            // the force: it went into the next kick
+            if (FUSE != 1) d.FD[g] = make_float4(fd.x, fd.y, fd.z, 0.f);
             fdk = fd;
             if (FUSE == 2 && !DIV) d.Xe[g] = x4;
             if (FUSE && !DIV) disp = next_kick(d, P, g, x4, v4, fd);
             else d.V[g] = v4;
         }
         if (FUSE && !DIV) {
-            for (int o = 16; o > 0; o >>= 1) disp = fmaxf(disp, __shfl_xor_sync(0xffffffffu, disp, o));
+            disp = warp_max(disp);
             if ((i & 31) == 0) smax[i >> 5] = disp;
         }
         if (i == 0) sm.dflag = 0;
+        cell_geom(sm.xs, sm.gs);
+        const int wn = sm.next[deal.turn];
+        if (wn < W) prefetch_cell_s2(d, cell_of(d, wn));
         float3 cm;
-        float4 lo, hi;
-        cell_geom(sm.xs, sm.gs, cm, lo, hi);
+        if (DIV || i == 0) cm = geom_centre(sm.gs);
         if (DIV) {
             if (st->step <= P.div_steps && P.growth > 0.0f) {
                 double vol, area;
-                cell_volume(d.topo.faces, sm.xs, cm, sm.gs, P.check_sph != 0, vol, area);
+                cell_volume(d.topo.faces, d.topo.tri, sm.xs, cm, sm.gs, P.check_sph != 0, vol, area);
                 if (i == 0) {
                     d.vol[a] = (float)vol;
                     if (!isfinite(vol)) { atomic_or_err(st, CS3D_ERRBIT_NONFINITE_VOL); vol = 1.0; }
                     int flag = vol > (double)P.divvol;
                     if (P.check_sph) {
                         d.area[a] = (float)area;
-                        double cb = cbrt(vol);
-                        double psi = 4.835975862049408 * cb * cb / area;
-                        if (fabs(1.0 - psi) > 0.05) flag = 0;
+                        if (flag) {
+                            double cb = cbrt(vol);
+                            double psi = 4.835975862049408 * cb * cb / area;
+                            if (fabs(1.0 - psi) > 0.05) flag = 0;
+                        }
                     }
                     d.divflag[a] = (uint8_t)flag;
                     sm.dflag = flag;
@@ -1211,7 +1258,8 @@ __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, 
             const bool divides = sm.dflag != 0;   // uniform
             if (FUSE == 2 && !divides && i < NODES) d.Xe[g] = x4;
             if (!divides && i < NODES) disp = next_kick(d, P, g, x4, v4, fdk);
-            for (int o = 16; o > 0; o >>= 1) disp = fmaxf(disp, __shfl_xor_sync(0xffffffffu, disp, o));
+            if (FUSE == 1 && divides && i < NODES) d.FD[g] = make_float4(fdk.x, fdk.y, fdk.z, 0.f);
+            disp = warp_max(disp);
             if ((i & 31) == 0) smax[i >> 5] = disp;
             __syncthreads();
         }
@@ -1222,6 +1270,8 @@ __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, 
                 d.cdisp[a] = mx;
                 atomicMax(&st->disp_step, __float_as_uint(mx));
             }
+            float4 lo, hi;
+            geom_box(sm.gs, lo, hi);
             d.CM[a] = make_float4(cm.x, cm.y, cm.z, 0.f);
             d.aabb[pn][2 * a] = lo;
             d.aabb[pn][2 * a + 1] = hi;
@@ -1261,10 +1311,11 @@ __global__ void __launch_bounds__(SLOTS) k_geom(Dev d, int par)
         const int inst = inst_of(d, a);
         xs[i] = (i < NODES) ? d.X[(size_t)a * SLOTS + i] : make_float4(0, 0, 0, 0);
         __syncthreads();
-        float3 cm;
-        float4 lo, hi;
-        cell_geom(xs, gs, cm, lo, hi);
+        cell_geom(xs, gs);
         if (i == 0) {
+            const float3 cm = geom_centre(gs);
+            float4 lo, hi;
+            geom_box(gs, lo, hi);
             d.CM[a] = make_float4(cm.x, cm.y, cm.z, 0.f);
             d.aabb[par][2 * a] = lo;
             d.aabb[par][2 * a + 1] = hi;
@@ -1468,15 +1519,19 @@ __device__ __forceinline__ void div_apply(const Dev &d, int par, float4 *xs, Geo
         __syncthreads();
         xs[i] = xa;
         __syncthreads();
-        float3 c1;
         float4 lo, hi;
-        cell_geom(xs, gs, c1, lo, hi);
-        if (i == 0) { d.aabb[pn][2 * a] = lo; d.aabb[pn][2 * a + 1] = hi; }
+        cell_geom(xs, gs);
+        if (i == 0) {
+            geom_box(gs, lo, hi);
+            d.aabb[pn][2 * a] = lo;
+            d.aabb[pn][2 * a + 1] = hi;
+        }
         __syncthreads();
         xs[i] = xb;
         __syncthreads();
-        cell_geom(xs, gs, c1, lo, hi);
+        cell_geom(xs, gs);
         if (i == 0) {
+            geom_box(gs, lo, hi);
             d.aabb[pn][2 * b] = lo;
             d.aabb[pn][2 * b + 1] = hi;
             d.press[a] = P.minp;
@@ -1697,11 +1752,9 @@ __global__ void __launch_bounds__(SLOTS) k_vol_hist(Dev d, int inst, float lo, f
         const int i = threadIdx.x;
         xs[i] = i < NODES ? d.X[(size_t)a * SLOTS + i] : make_float4(0.f, 0.f, 0.f, 0.f);
         __syncthreads();
-        float3 cm;
-        float4 blo, bhi;
-        cell_geom(xs, gs, cm, blo, bhi);
+        cell_geom(xs, gs);
         double vol, area;
-        cell_volume(d.topo.faces, xs, cm, gs, false, vol, area);
+        cell_volume(d.topo.faces, d.topo.tri, xs, geom_centre(gs), gs, false, vol, area);
         if (i == 0) {
             const float v = (float)vol;
             if (vols) vols[c] = v;
@@ -1788,19 +1841,6 @@ __device__ __forceinline__ unsigned bin_slot(const InstState &st, int ix, int iy
     h ^= h >> 15;
     h *= 0x9e3779b1u;
     return st.hbase + (h >> (32 - st.hbits));
-}
-
-__device__ __forceinline__ float warp_min(float v)
-{
-    float r;
-    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float warp_max(float v)
-{
-    float r;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
 }
 
 // B1: boxes at the current positions and the cell table, one warp per cell.
