@@ -205,16 +205,11 @@ __device__ __forceinline__ double sqrt_nr(double x)
 // difference of two angles near 2 rad whose float rounding alone (1.2e-7)
 // would exceed the 1e-5 relative force bar, so it is formed without
 // rounding theta.  u = cos(theta) (the reference's regularised ratio) is
-// formed in FP64; with c0, s0 = cos, sin of theta0 in FP64 and
-// s = sin(theta) = sqrt(1 - u^2), dth = theta - theta0 has
-//   sin(dth) = s c0 - u s0,  cos(dth) = u c0 + s s0,  tan(dth / 2) = sin(dth) / (1 + cos(dth)),
-// and dth = 2 atan of that by a polynomial (Chebyshev interpolation of
-// atan(t) / t in t^2 up to 0.4, relative error 1.9e-12).  Beyond, at
-// |dth| > 1.13 rad, a float estimate of dth from acosf is refined by one
-// Newton step of sin(dth / 2) = (c0 - u) / (2 sin(theta0 + dth / 2)) in FP64
-// (sin/cos of dth/2 by their Taylor series); taken for all angles, that costs
-// S1 of 100,000 packed cells 1.68 ms against 1.53 (longer chains, and more
-// registers than the kernel has).
+// formed in FP64; with c0, s0 = cos, sin of theta0 in FP64,
+//   sin(dth / 2) = (c0 - u) / (2 sin(theta0 + dth / 2)),   dth = theta - theta0.
+// A float estimate of dth from acosf is refined by one Newton step of this
+// equation in FP64 (sin/cos of dth/2 by their Taylor series, |dth/2| < 0.4
+// for |dth/2| up to ~1.2 rad), which leaves dth accurate to ~1e-12.
 __device__ __forceinline__ void sincos_small(double x, double &s, double &c)
 {
     const double x2 = x * x;
@@ -243,20 +238,6 @@ __device__ __forceinline__ Arm make_arm(const double3 &to, const double3 &from)
     return a;
 }
 
-// theta - theta0 where it is large.
-__device__ __noinline__ double wide_angle(double u, float th0f, double c0, double s0)
-{
-    // float estimate, then one Newton step on g(h) = sin(h) sin(theta0 + h) - (c0 - u)/2, h = dth/2
-    double h = 0.5 * (double)(acosf((float)u) - th0f);
-    double sh, ch;
-    sincos_small(h, sh, ch);
-    const double s1 = s0 * ch + c0 * sh, c1t = c0 * ch - s0 * sh;  // sin, cos of theta0 + h
-    const double g = sh * s1 - 0.5 * (c0 - u);
-    const double dg = ch * s1 + sh * c1t;                            // d/dh of sin(h) sin(theta0 + h)
-    h -= g * rcp_nr(dg);
-    return 2.0 * h;
-}
-
 // The angle between arms p and q: GetAngleForce(P, Q) (Fp) and
 // GetAngleForce(Q, P) (Fq).  |p||q| is the product of the two lengths, as the
 // reference forms it (sqrtf(ri_2) * sqrtf(rk_2)).
@@ -265,23 +246,15 @@ __device__ __forceinline__ void angle_term(const Arm &p, const Arm &q, float th0
 {
     const double idk = p.x * q.x + p.y * q.y + p.z * q.z;
     const double u = idk * rcp_nr(p.len * q.len + 1e-3);
-    double dth;
-    const double v = 1.0 - u * u, s = v * rsqrt_nr(v);
-    const double t = (s * c0 - u * s0) * rcp_nr(1.0 + (u * c0 + s * s0));
-    const double z = t * t;
-    if (z <= 0.4) {
-        double q = -0.010709327812319008;
-        q = fma(q, z, 0.03360965597502365);
-        q = fma(q, z, -0.05672578427922923);
-        q = fma(q, z, 0.07437129908232694);
-        q = fma(q, z, -0.09048784092942751);
-        q = fma(q, z, 0.1110678238876255);
-        q = fma(q, z, -0.14285455109241751);
-        q = fma(q, z, 0.19999992038868686);
-        q = fma(q, z, -0.3333333323770785);
-        q = fma(q, z, 0.999999999998091);
-        dth = 2.0 * t * q;
-    } else dth = wide_angle(u, th0f, c0, s0);
+    // float estimate, then one Newton step on g(h) = sin(h) sin(theta0 + h) - (c0 - u)/2, h = dth/2
+    double h = 0.5 * (double)(acosf((float)u) - th0f);
+    double sh, ch;
+    sincos_small(h, sh, ch);
+    const double s1 = s0 * ch + c0 * sh, c1t = c0 * ch - s0 * sh;  // sin, cos of theta0 + h
+    const double g = sh * s1 - 0.5 * (c0 - u);
+    const double dg = ch * s1 + sh * c1t;                            // d/dh of sin(h) sin(theta0 + h)
+    h -= g * rcp_nr(dg);
+    const double dth = 2.0 * h;
     const double c1 = -rsqrt_nr(p.r2 * q.r2 - idk * idk + 1e-3);
     const double f = -1000.0 * c1 * dth;
     const double cp = idk * p.ir2, cq = idk * q.ir2;
@@ -368,15 +341,17 @@ __device__ __forceinline__ bool slot_ok(const SlotData &sd, const InstParams &P,
 // every node, then the second, ...) are laid out back to back, a round takes
 // 32 of them, one to a lane, and the owners then add up the results of their
 // entries in entry order, so that a node's sums do not depend on the sharing.
-// An owner seldom has more than two entries in a round.  S1 of 100,000 packed
-// cells 2.01 -> 1.86 ms, of 3000 growing ones 97 -> 85 us (with an owner's
-// entries side by side, up to 32 to a round, 1.89 ms and 95 us); S2's sweep,
-// two loads and three additions a pair, is slower this way (0.62 -> 0.65 ms).
+// An owner seldom has more than two entries in a round, and adds them to its
+// running force exactly as a lane walking its own entries would.  S1 of 100,000
+// packed cells 2.01 -> 1.86 ms, of 3000 growing ones 97 -> 85 us (with an
+// owner's entries side by side, up to 32 to a round, 1.89 ms and 95 us); S2's
+// sweep, two loads and three additions a pair, is slower this way (0.62 ->
+// 0.65 ms).
 // ---------------------------------------------------------------------------
 constexpr int EPRE = 8;    // entries of a node laid out at a time
 
 struct alignas(16) SweepSmem {
-    double res[6][32];           // results of a round: force, velocity difference
+    double res[7][32];           // results of a round: force over distance, distance, velocity difference
     uint32_t item[EPRE * 32];    // owner lane << 16 | slot << 8 | node
     unsigned own[32];            // results of the round that are the node's
 };
@@ -460,11 +435,12 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
                     if (R < (double)P.ra) k += -(double)P.asE * ((double)P.ra - R) * iR;
                     if (R <= (double)P.rr) k += (double)P.rsE * ((double)P.rr - R) * iR;
                 }
-                ss.res[0][lane] = k * ex; ss.res[1][lane] = k * ey; ss.res[2][lane] = k * ez;
+                ss.res[0][lane] = k;
+                ss.res[1][lane] = ex; ss.res[2][lane] = ey; ss.res[3][lane] = ez;
                 // velocity differences of floats are exact in FP64
-                ss.res[3][lane] = (double)vo.x - vj.x;
-                ss.res[4][lane] = (double)vo.y - vj.y;
-                ss.res[5][lane] = (double)vo.z - vj.z;
+                ss.res[4][lane] = (double)vo.x - vj.x;
+                ss.res[5][lane] = (double)vo.y - vj.y;
+                ss.res[6][lane] = (double)vo.z - vj.z;
             }
             __syncwarp();
             unsigned mine = ss.own[lane];
@@ -474,8 +450,11 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
                 mine &= mine - 1u;
                 if (nd < MAXD) dl[(size_t)nd * SLOTS] = (uint16_t)ss.item[b + q];
                 ++nd;
-                FX += ss.res[0][q]; FY += ss.res[1][q]; FZ += ss.res[2][q];
-                vsum.x += ss.res[3][q]; vsum.y += ss.res[4][q]; vsum.z += ss.res[5][q];
+                const double k = ss.res[0][q];
+                FX = fma(k, ss.res[1][q], FX);
+                FY = fma(k, ss.res[2][q], FY);
+                FZ = fma(k, ss.res[3][q], FZ);
+                vsum.x += ss.res[4][q]; vsum.y += ss.res[5][q]; vsum.z += ss.res[6][q];
             }
             __syncwarp();
         }
@@ -1004,16 +983,12 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
             sm.arm.x[o + 2] = F12q.x + F02q.x; sm.arm.y[o + 2] = F12q.y + F02q.y; sm.arm.z[o + 2] = F12q.z + F02q.z;
         }
         __syncthreads();
-        double CX = 0.0, CY = 0.0, CZ = 0.0;
-        double3 vsum = make_double3(0.0, 0.0, 0.0);
-        // contacts, src/propagate.cu:356-442 and the first dissipative sweep
-        const int nd = sweep_s1<COOP>(d, P, sm.sd, sm.sweep[i >> 5], a, i, x, v, ne, pre, CX, CY, CZ, vsum);
+        // The node force is accumulated in FP64: its terms (pressure up
+        // to ~1e3, stiff contact repulsion up to ~1e4) can cancel to a
+        // net force orders of magnitude smaller, and the sum is rounded to
+        // float once, as the reference stores it.
+        double FX = 0.0, FY = 0.0, FZ = 0.0;
         if (i < NODES) {
-            // The node force is accumulated in FP64: its terms (pressure up
-            // to ~1e3, stiff contact repulsion up to ~1e4) can cancel to a
-            // net force orders of magnitude smaller, and the sum is rounded to
-            // float once, as the reference stores it.
-            double FX = 0.0, FY = 0.0, FZ = 0.0;
             if (isnan(x.x) || isnan(x.y) || isnan(x.z)) atomic_or_err(&d.st[inst], CS3D_ERRBIT_NAN);
             // springs, src/propagate.cu:298-314:
             // k (R - R0) / R0 * d / R = k (1/R0 - 1/R) d
@@ -1046,9 +1021,11 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
                 FY += sm.arm.y[am.x] + sm.arm.y[am.y] + sm.arm.y[am.z] - (sm.arm.y[o] + sm.arm.y[o + 1] + sm.arm.y[o + 2]);
                 FZ += sm.arm.z[am.x] + sm.arm.z[am.y] + sm.arm.z[am.z] - (sm.arm.z[o] + sm.arm.z[o + 1] + sm.arm.z[o + 2]);
             }
-            FX += CX;
-            FY += CY;
-            FZ += CZ;
+        }
+        // contacts, src/propagate.cu:356-442 and the first dissipative sweep
+        double3 vsum = make_double3(0.0, 0.0, 0.0);
+        const int nd = sweep_s1<COOP>(d, P, sm.sd, sm.sweep[i >> 5], a, i, x, v, ne, pre, FX, FY, FZ, vsum);
+        if (i < NODES) {
             const double3 vt = tangential(sm.xd, n0, n1, n2, sgn, vsum);
             if (nd > MAXD) atomic_or_err(&d.st[inst], CS3D_ERRBIT_ENTRY_OVERFLOW);
             // rigid box walls, src/propagate.cu:474-510 (float gap tests)
@@ -1172,7 +1149,10 @@ __device__ __forceinline__ void prefetch_cell_s2(const Dev &d, int a)
 // step follows in the same launch sequence, FUSE 2 on the last step of a
 // cs3d_step call, which also keeps the step-end positions (Xe; the step-end
 // velocities are Vb) for the state read-back, so that the next call starts
-// without a k_integrate pass.
+// without a k_integrate pass.  A stream over X, Vb, FC and Xb with the
+// partners' velocities gathered: S2 of 100,000 packed cells 0.62 -> 0.52 ms with
+// the next cell prefetched, extents by redux, one thread's box and centre, the
+// centre's division by 180 as a product, and no store of forces nobody reads.
 template <bool DIV, bool COOP>
 __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, S2Smem &sm)
 {
