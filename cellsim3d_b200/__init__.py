@@ -45,6 +45,13 @@ def _f32(a, n=None):
     return a
 
 
+def _rows(keys, k):
+    """Arrays of k floats, for the library to fill: rows of one allocation,
+    which the system backs with large pages where six small ones would take a
+    fault for every 4 KB."""
+    return dict(zip(keys, np.empty((len(keys), k), dtype=np.float32)))
+
+
 def version():
     return _lib.lib().cs3d_version()
 
@@ -269,7 +276,7 @@ class Ensemble:
                 if key not in a or a[key].size < n:
                     a[key] = np.zeros(n, dtype=np.float32)
         else:
-            a = {key: np.zeros(k, dtype=np.float32) for key in ("X", "Y", "Z", "VX", "VY", "VZ")}
+            a = _rows(("X", "Y", "Z", "VX", "VY", "VZ"), k)
             a["pressure"] = np.zeros(n, dtype=np.float32)
             a["youngs"] = np.zeros(n, dtype=np.float32)
         nn = C.c_int32()
@@ -300,7 +307,7 @@ class Ensemble:
     def forces(self, inst=0):
         n = self.n_cells(inst)
         k = n * 192
-        a = {key: np.zeros(k, dtype=np.float32) for key in ("FCX", "FCY", "FCZ", "FDX", "FDY", "FDZ")}
+        a = _rows(("FCX", "FCY", "FCZ", "FDX", "FDY", "FDZ"), k)
         st = _lib.lib().cs3d_get_forces(self.h, inst, *[_fp(a[q]) for q in ("FCX", "FCY", "FCZ", "FDX", "FDY", "FDZ")])
         _lib.check(st, "cs3d_get_forces")
         return a

@@ -4,6 +4,7 @@
 // extern "C" and return CS3D_* status codes.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -23,7 +24,7 @@ struct cs3d_ctx {
     int cap_total = 0;
     int nsm = 148;
     std::vector<InstParams> hprm;
-    std::vector<int> hn;           // host copy of the loaded cell counts
+    std::vector<int> hn;           // cell counts: loaded, or as of the last step
     Dev d{};
     // device allocations to free
     std::vector<void *> allocs;
@@ -46,6 +47,8 @@ struct cs3d_ctx {
     int grid_s2 = 0;               // blocks of S2 and the integrator
     int grid_steps = 0;            // blocks of k_steps that are resident together (0: no cooperative launch)
     int n_now = 0;                 // cells of all instances after the last call
+    std::vector<InstState> hst;    // the instances' states as last read
+    std::vector<char> buf;         // small transfers
     cudaGraphExec_t graph[2][2][2][3] = {};  // [parity][division][integrate first][S2 mode: 0, fused 1, fused last 2]
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // asynchronous read-back (cs3d_get_state_async): a copy stream, two
@@ -70,18 +73,19 @@ namespace {
         }                                                \
     } while (0)
 
-template <typename T>
-int dalloc(cs3d_ctx *c, T **p, size_t count)
-{
-    void *q = nullptr;
-    size_t bytes = count * sizeof(T);
-    if (bytes == 0) bytes = 16;
-    if (cudaMalloc(&q, bytes) != cudaSuccess) return CS3D_E_NOMEM;
-    if (cudaMemsetAsync(q, 0, bytes, c->stream) != cudaSuccess) { cudaFree(q); return CS3D_E_CUDA; }
-    c->allocs.push_back(q);
-    *p = (T *)q;
-    return CS3D_OK;
-}
+// Device memory of a context: one allocation, its arrays back to back (an
+// allocation each took half of cs3d_create's time).  A first pass with base
+// null adds up the sizes, a second one hands out the addresses.
+struct Arena {
+    char *base = nullptr;
+    size_t at = 0;
+    template <typename T>
+    void take(T *&p, size_t count)
+    {
+        p = base ? (T *)(base + at) : nullptr;
+        at += (std::max<size_t>(count * sizeof(T), 16) + 255) / 256 * 256;
+    }
+};
 
 void free_all(cs3d_ctx *c)
 {
@@ -110,15 +114,31 @@ void free_all(cs3d_ctx *c)
 // angles at n that have i as an arm end, the NeighNeighs cases of
 // src/propagate.cu:63-78).
 struct TopoTables {
-    uint32_t nnp[SLOTS];
+    double2 cs0[3 * SLOTS];
     float4 r0[SLOTS], th[SLOTS];
     uint4 arm[SLOTS];
+    double r0i[3 * SLOTS];
+    uint32_t nnp[SLOTS];
+    uint32_t tri[CS3D_FACES * 6];
     uint8_t faces[CS3D_FACES * 7];
     uint8_t patch[SLOTS];
-    uint32_t tri[CS3D_FACES * 6];
-    double2 cs0[3 * SLOTS];
-    double r0i[3 * SLOTS];
 };
+
+// The kernels' pointers into the device copy of the tables.
+Topo topo_pointers(TopoTables *t)
+{
+    Topo T;
+    T.nnpack = t->nnp;
+    T.r0 = t->r0;
+    T.th0 = t->th;
+    T.cs0 = t->cs0;
+    T.r0i = t->r0i;
+    T.arm = t->arm;
+    T.faces = t->faces;
+    T.tri = t->tri;
+    T.patch = t->patch;
+    return T;
+}
 
 // Nodes m[0 .. n) in the order of their distance along the bonds (within the
 // set) from its most outlying node.
@@ -203,35 +223,6 @@ int topo_tables(const cs3d_topology *t, TopoTables &o)
     return CS3D_OK;
 }
 
-int upload_topology(cs3d_ctx *c, const cs3d_topology *t)
-{
-    TopoTables tt;
-    int rc = topo_tables(t, tt);
-    if (rc) return rc;
-    Topo &T = c->d.topo;
-    if ((rc = dalloc(c, &T.cs0, 3 * SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.r0i, 3 * SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.nnpack, SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.r0, SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.th0, SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.arm, SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.faces, CS3D_FACES * 7))) return rc;
-    if ((rc = dalloc(c, &T.patch, SLOTS))) return rc;
-    if ((rc = dalloc(c, &T.tri, CS3D_FACES * 6))) return rc;
-    CK(cudaMemcpyAsync(T.cs0, tt.cs0, sizeof tt.cs0, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.r0i, tt.r0i, sizeof tt.r0i, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.nnpack, tt.nnp, sizeof tt.nnp, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.r0, tt.r0, sizeof tt.r0, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.th0, tt.th, sizeof tt.th, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.arm, tt.arm, sizeof tt.arm, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.faces, tt.faces, sizeof tt.faces, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.patch, tt.patch, sizeof tt.patch, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(T.tri, tt.tri, sizeof tt.tri, cudaMemcpyHostToDevice, c->stream));
-    // the host tables go out of scope: the copies must have completed
-    CK(cudaStreamSynchronize(c->stream));
-    return CS3D_OK;
-}
-
 InstParams make_inst(const cs3d_params &p, int base, int cap, float skin, float inv_bin)
 {
     InstParams q{};
@@ -296,41 +287,79 @@ int check_params(const cs3d_params &p)
     return CS3D_OK;
 }
 
-// Staged SoA (6 arrays of k floats) -> float4 positions (and velocities);
-// padding nodes (180..191 of each cell) are left zero.
-__global__ void k_pack(const float *stage, float4 *X, float4 *V, size_t k)
+// A loaded instance: staged SoA (3 or 6 arrays of k = n*192 floats, then with
+// has_p / has_e the cells' pressures / stiffnesses) into its arrays, and zeros in
+// the rest of them up to its capacity; padding nodes (180..191 of each cell)
+// are zero.
+__global__ void k_load(Dev d, int inst, int n, int with_v, int has_p, int has_e, const float *stage)
 {
-    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < k; g += (size_t)gridDim.x * blockDim.x) {
-        if (g % SLOTS >= NODES) continue;
-        X[g] = make_float4(stage[g], stage[k + g], stage[2 * k + g], 0.f);
-        if (V) V[g] = make_float4(stage[3 * k + g], stage[4 * k + g], stage[5 * k + g], 0.f);
+    const InstParams &P = d.prm[inst];
+    const size_t k = (size_t)n * SLOTS, off = (size_t)P.base * SLOTS, slots = (size_t)P.cap * SLOTS;
+    const float *cells = stage + (with_v ? 6 : 3) * k;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < slots; g += (size_t)gridDim.x * blockDim.x) {
+        const bool real = g < k && g % SLOTS < NODES;
+        d.X[off + g] = real ? make_float4(stage[g], stage[k + g], stage[2 * k + g], 0.f) : zero;
+        d.V[off + g] = real && with_v ? make_float4(stage[3 * k + g], stage[4 * k + g], stage[5 * k + g], 0.f) : zero;
+        d.Vb[off + g] = zero;
+        d.FC[off + g] = zero;
+        d.FD[off + g] = zero;
+        if (g < (size_t)P.cap) {
+            const int c = (int)g, a = P.base + c;
+            d.press[a] = c >= n ? 0.f : has_p ? cells[c] : P.minp;
+            d.E[a] = c >= n ? 0.f : has_e ? cells[(has_p ? n : 0) + c] : P.stiff1;
+            d.CM[a] = zero;
+            d.vol[a] = 0.f;
+            d.area[a] = 0.f;
+            d.divflag[a] = 0;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        InstState &st = d.st[inst];
+        st.n = n;
+        st.step = 0;
+        st.err = 0u;
+        st.syscm[0] = st.syscm[1] = st.syscm[2] = 1.0f;   // the reference's initial system centre
     }
 }
 
-// float4 arrays a, b -> staged SoA components (a.xyz, b.xyz).
-__global__ void k_unpack(float *stage, const float4 *a, const float4 *b, size_t k)
+// float4 arrays a, b -> staged SoA components (a.xyz, b.xyz), and n per-cell
+// values each of p, e behind them.
+__global__ void k_unpack(float *stage, const float4 *a, const float4 *b, size_t k, const float *p, const float *e, int n)
 {
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < k; g += (size_t)gridDim.x * blockDim.x) {
         if (a) { const float4 v = a[g]; stage[g] = v.x; stage[k + g] = v.y; stage[2 * k + g] = v.z; }
         if (b) { const float4 v = b[g]; stage[3 * k + g] = v.x; stage[4 * k + g] = v.y; stage[5 * k + g] = v.z; }
+        if (p && g < (size_t)n) stage[6 * k + g] = p[g];
+        if (e && g < (size_t)n) stage[6 * k + n + g] = e[g];
     }
 }
 
-// Rebuild the active-cell work table from the device cell counts.
-__global__ void k_build_work(Dev d)
+// The active-cell work table from the device cell counts, one warp for an
+// instance; with one instance the table is the identity and not used.
+__global__ void __launch_bounds__(1024) k_build_work(Dev d)
 {
-    __shared__ int off;
-    if (threadIdx.x == 0) off = 0;
-    __syncthreads();
-    for (int k = 0; k < d.n_inst; ++k) {
-        int n = d.st[k].n, base = d.prm[k].base;
-        for (int c = threadIdx.x; c < n; c += blockDim.x) d.work[off + c] = base + c;
+    __shared__ int wsum[32];
+    __shared__ int first[1024];
+    int done = 0;   // cells of the instances before k0
+    for (int k0 = 0; k0 < d.n_inst; k0 += 1024) {
+        const int k = k0 + threadIdx.x;
+        int tot;
+        const int at = block_excl_scan<1024>(k < d.n_inst ? d.st[k].n : 0, wsum, tot);
+        first[threadIdx.x] = done + at;
         __syncthreads();
-        if (threadIdx.x == 0) off += n;
+        const int m = d.n_inst - k0 < 1024 ? d.n_inst - k0 : 1024;
+        for (int q = threadIdx.x >> 5; q < m; q += 32) {
+            const int n = d.st[k0 + q].n, base = d.prm[k0 + q].base;
+            for (int c = threadIdx.x & 31; c < n; c += 32) d.work[first[q] + c] = base + c;
+        }
+        done += tot;
         __syncthreads();
     }
-    if (threadIdx.x == 0) *d.work_n = off;
+    if (threadIdx.x == 0) *d.work_n = done;
 }
+
+constexpr size_t SMALL_BYTES = 256 << 10;
 
 // Optional per-launch event recording (profiling pass of cs3d_profile_step).
 struct Prof {
@@ -393,7 +422,7 @@ int run_init(cs3d_ctx *c)
 {
     const Dev &d = c->d;
     cudaStream_t s = c->stream;
-    k_build_work<<<1, 256, 0, s>>>(d);
+    if (!d.single) k_build_work<<<1, 1024, 0, s>>>(d);
     k_init_begin<<<1, 256, 0, s>>>(d);
     k_geom<<<c->grid_cells, SLOTS, 0, s>>>(d, 0);
     // correct_com at set-up (src/GPUbounce.cu:785-805): after the first grid,
@@ -515,52 +544,82 @@ int settle(cs3d_ctx *c)
     return CS3D_OK;
 }
 
-int read_errors(cs3d_ctx *c, unsigned *any)
+int wait_stream(cs3d_ctx *c)
 {
-    std::vector<InstState> st(c->n_inst);
-    CK(cudaMemcpyAsync(st.data(), c->d.st, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    unsigned bits = 0;
-    c->n_now = 0;
-    for (auto &q : st) {
-        bits |= q.err;
-        c->n_now += q.n;
-    }
-    *any = bits;
-    c->last_err_bits = bits;
     return CS3D_OK;
 }
 
-int inst_count(cs3d_ctx *c, int inst, int *n)
+// The instances' states to the host, without waiting.
+int fetch_states(cs3d_ctx *c)
 {
-    int v = 0;
-    CK(cudaMemcpyAsync(&v, &c->d.st[inst].n, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    *n = v;
+    CK(cudaMemcpyAsync(c->hst.data(), c->d.st, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
+    return CS3D_OK;
+}
+
+// Error bits and cell counts from the fetched states.
+unsigned take_states(cs3d_ctx *c)
+{
+    unsigned bits = 0;
+    c->n_now = 0;
+    for (int k = 0; k < c->n_inst; ++k) {
+        bits |= c->hst[k].err;
+        c->hn[k] = c->hst[k].n;
+        c->n_now += c->hst[k].n;
+    }
+    c->last_err_bits = bits;
+    return bits;
+}
+
+int read_errors(cs3d_ctx *c, unsigned *any)
+{
+    if (int rc = fetch_states(c)) return rc;
+    if (int rc = wait_stream(c)) return rc;
+    *any = take_states(c);
     return CS3D_OK;
 }
 
 // Host <-> device transfers of 192-stride SoA node arrays go through a
-// device staging area (c->d.stage, 6 arrays of cap*192 floats): the host
-// copies move the caller's arrays as they are (at full PCIe speed when the
-// caller's memory is pinned) and kernels convert to and from the float4
-// layout.
+// device staging area (c->d.stage, 6 arrays of cap*192 floats and 2 per-cell
+// ones) and kernels that convert to and from the float4 layout.  Up to
+// SMALL_BYTES they take one copy through the context's buffer: a copy costs
+// some 3 us to issue, more than the CPU's memcpy.  The buffer is pageable, so
+// that a copy from it has left it when the call returns (page-locking it would
+// add 1 to 3 ms to cs3d_create).  Larger ones move the caller's arrays as they
+// are, at full PCIe speed when the caller's memory is pinned.
 
 // Gather up to two float4 arrays of instance inst (n cells) into staged
-// SoA components (k = 0..5 -> a.x, a.y, a.z, b.x, b.y, b.z), then copy the
-// requested ones to the host.
-int fetch_soa(cs3d_ctx *c, int inst, int n, const float4 *a, const float4 *b, float *const out[6])
+// SoA components (k = 0..5 -> a.x, a.y, a.z, b.x, b.y, b.z) and two per-cell
+// arrays, then copy the requested ones to the host.
+int fetch_soa(cs3d_ctx *c, int inst, int n, const float4 *a, const float4 *b, float *const out[6], float *p = nullptr,
+              float *e = nullptr)
 {
-    if (n == 0) return CS3D_OK;
+    if (n == 0 || (!a && !b && !p && !e)) return wait_stream(c);
     const size_t k = (size_t)n * SLOTS;
-    const size_t off = (size_t)c->hprm[inst].base * SLOTS;
-    k_unpack<<<c->grid_flat, 256, 0, c->stream>>>(c->d.stage, a ? a + off : nullptr, b ? b + off : nullptr, k);
+    const int base = c->hprm[inst].base;
+    const size_t off = (size_t)base * SLOTS;
+    const float *dp = p ? c->d.press + base : nullptr, *de = e ? c->d.E + base : nullptr;
+    float *stage = c->d.stage;
+    const int grid = (int)std::min<size_t>((k + 255) / 256, (size_t)c->nsm * 8);
+    k_unpack<<<grid, 256, 0, c->stream>>>(stage, a ? a + off : nullptr, b ? b + off : nullptr, k, dp, de, n);
     CK(cudaGetLastError());
+    const size_t from = a ? 0 : b ? 3 * k : 6 * k, to = p || e ? 6 * k + 2 * (size_t)n : b ? 6 * k : 3 * k;
+    if (sizeof(float) * (to - from) <= SMALL_BYTES) {
+        char *h = c->buf.data();
+        CK(cudaMemcpyAsync(h, stage + from, sizeof(float) * (to - from), cudaMemcpyDeviceToHost, c->stream));
+        if (int rc = wait_stream(c)) return rc;
+        const float *f = (const float *)h;
+        for (int q = 0; q < 6; ++q)
+            if (out[q]) memcpy(out[q], f + (size_t)q * k - from, sizeof(float) * k);
+        if (p) memcpy(p, f + 6 * k - from, sizeof(float) * n);
+        if (e) memcpy(e, f + 6 * k + n - from, sizeof(float) * n);
+        return CS3D_OK;
+    }
     for (int q = 0; q < 6; ++q)
-        if (out[q]) CK(cudaMemcpyAsync(out[q], c->d.stage + (size_t)q * k, sizeof(float) * k, cudaMemcpyDeviceToHost,
-                                       c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    return CS3D_OK;
+        if (out[q]) CK(cudaMemcpyAsync(out[q], stage + (size_t)q * k, sizeof(float) * k, cudaMemcpyDeviceToHost, c->stream));
+    if (p) CK(cudaMemcpyAsync(p, stage + 6 * k, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
+    if (e) CK(cudaMemcpyAsync(e, stage + 6 * k + n, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
+    return wait_stream(c);
 }
 
 }  // namespace
@@ -593,6 +652,8 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     c->n_inst = n_inst;
     c->cap_total = (int)total;
     c->hn.assign(n_inst, 0);
+    c->hst.resize(n_inst);
+    c->buf.resize(SMALL_BYTES);
     int base = 0;
     const float inv_bin = inv_bin_edge(topo);
     for (int k = 0; k < n_inst; ++k) {
@@ -613,13 +674,21 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     d.single = n_inst == 1 ? 1 : 0;
     d.cap_total = c->cap_total;
     const size_t nodes = (size_t)c->cap_total * SLOTS;
-    int rc = CS3D_OK;
-#define AL(ptr, cnt) if (!rc) rc = dalloc(c, &(ptr), (cnt))
-    AL(d.prm, n_inst);
+    size_t bins = 0;
+    for (int k = 0; k < n_inst; ++k) bins += (size_t)table_size(capacity[k]);
+    TopoTables *dtopo = nullptr;
+    d.ev_cap = std::max(1 << 16, 2 * c->cap_total);
+    d.far_cap = d.ev_cap;
+    d.pair_cap = 1;
+    Arena ar;
+    const auto lay_out = [&] {
+        ar.at = 0;
+#define AL(ptr, cnt) ar.take(ptr, (cnt))
+    AL(dtopo, 1); AL(d.prm, n_inst);
     AL(d.st, n_inst);
     AL(d.X, nodes); AL(d.V, nodes); AL(d.Vb, nodes); AL(d.FC, nodes); AL(d.FD, nodes); AL(d.FR, nodes);
     AL(d.Xe, nodes);
-    AL(d.stage, 6 * nodes);
+    AL(d.stage, 6 * nodes + 2 * (size_t)c->cap_total);
     AL(d.CM, c->cap_total);
     AL(d.press, c->cap_total); AL(d.E, c->cap_total); AL(d.vol, c->cap_total); AL(d.area, c->cap_total);
     AL(d.divflag, c->cap_total);
@@ -630,21 +699,30 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     AL(d.dlist, (size_t)c->cap_total * MAXD * SLOTS); AL(d.ndis, nodes);
     AL(d.Xb, nodes);
     AL(d.ent, (size_t)c->cap_total * MAXE * SLOTS); AL(d.nent, nodes);
-    size_t bins = 0;
-    for (int k = 0; k < n_inst; ++k) bins += (size_t)table_size(capacity[k]);
     AL(d.nbox, 2 * (size_t)c->cap_total); AL(d.bins, bins); AL(d.bnext, c->cap_total); AL(d.epoch, 1);
     AL(d.cdisp, c->cap_total); AL(d.build, c->cap_total); AL(d.n_build, 1); AL(d.mark, c->cap_total);
     AL(d.divtab, c->cap_total); AL(d.div_total, 1); AL(d.div_prev, 1); AL(d.flagged, c->cap_total);
-    d.ev_cap = std::max(1 << 16, 2 * c->cap_total);
     AL(d.events, d.ev_cap); AL(d.n_events, 1);
-    d.far_cap = d.ev_cap;
     AL(d.farlog, d.far_cap); AL(d.n_far, 1);
     AL(d.pick, (size_t)c->cap_total + n_inst);
     AL(d.flags, 4); AL(d.bar, 2); AL(d.deal, DEALS);
-    d.pair_cap = 1;
     AL(d.pairs, 1); AL(d.n_pairs, 1);
 #undef AL
-    if (!rc) rc = upload_topology(c, topo);
+    };
+    lay_out();
+    int rc = CS3D_OK;
+    void *mem = nullptr;
+    if (cudaMalloc(&mem, ar.at) != cudaSuccess) rc = CS3D_E_NOMEM;
+    else {
+        c->allocs.push_back(mem);
+        if (cudaMemsetAsync(mem, 0, ar.at, c->stream) != cudaSuccess) rc = CS3D_E_CUDA;
+        ar.base = (char *)mem;
+        lay_out();
+        d.topo = topo_pointers(dtopo);
+    }
+    TopoTables tt;
+    if (!rc) rc = topo_tables(topo, tt);
+    if (!rc && cudaMemcpyAsync(dtopo, &tt, sizeof tt, cudaMemcpyHostToDevice, c->stream) != cudaSuccess) rc = CS3D_E_CUDA;
     if (rc) { free_all(c); delete c; return rc; }
     // instance parameters, RANMAR streams and slot ownership
     std::vector<InstState> st(n_inst);
@@ -799,60 +877,54 @@ int cs3d_load_state(cs3d_ctx *c, int inst, int n, const float *X, const float *Y
     cudaSetDevice(c->device);
     // the other instances back to their step-end state: the re-initialisation
     // that follows a load starts from it
+    if (c->n_inst == 1) c->prekicked = false;   // all of it is replaced
     if (int rc = settle(c)) return rc;
-    const size_t slots = (size_t)P.cap * SLOTS;
     const size_t k = (size_t)n * SLOTS;
-    const size_t off0 = (size_t)P.base * SLOTS;
-    const Dev &d0 = c->d;
     // the caller's SoA arrays into the staging area, packed on the device
     const float *in[6] = {X, Y, Z, VX, VY, VZ};
     const bool with_v = VX && VY && VZ;
-    for (int q = 0; q < (with_v ? 6 : 3); ++q)
-        if (k) CK(cudaMemcpyAsync(d0.stage + (size_t)q * k, in[q], sizeof(float) * k, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemsetAsync(d0.X + off0, 0, sizeof(float4) * slots, c->stream));
-    CK(cudaMemsetAsync(d0.V + off0, 0, sizeof(float4) * slots, c->stream));
-    if (k) k_pack<<<c->grid_flat, 256, 0, c->stream>>>(d0.stage, d0.X + off0, with_v ? d0.V + off0 : nullptr, k);
-    CK(cudaGetLastError());
-    std::vector<float> p(P.cap, 0.f), e(P.cap, 0.f);
-    for (int k = 0; k < n; ++k) {
-        p[k] = pressure ? pressure[k] : P.minp;
-        e[k] = youngs ? youngs[k] : P.stiff1;
+    const int m = with_v ? 6 : 3;
+    const size_t words = m * k + (pressure ? n : 0) + (youngs ? n : 0);
+    float *stage = c->d.stage;
+    const bool small = sizeof(float) * words <= SMALL_BYTES;
+    if (small && words) {
+        char *h = c->buf.data();
+        float *f = (float *)h;
+        for (int q = 0; q < m; ++q, f += k) memcpy(f, in[q], sizeof(float) * k);
+        if (pressure) { memcpy(f, pressure, sizeof(float) * n); f += n; }
+        if (youngs) memcpy(f, youngs, sizeof(float) * n);
+        CK(cudaMemcpyAsync(stage, h, sizeof(float) * words, cudaMemcpyHostToDevice, c->stream));
+    } else if (words) {
+        float *f = stage;
+        for (int q = 0; q < m; ++q, f += k) CK(cudaMemcpyAsync(f, in[q], sizeof(float) * k, cudaMemcpyHostToDevice, c->stream));
+        if (pressure) { CK(cudaMemcpyAsync(f, pressure, sizeof(float) * n, cudaMemcpyHostToDevice, c->stream)); f += n; }
+        if (youngs) CK(cudaMemcpyAsync(f, youngs, sizeof(float) * n, cudaMemcpyHostToDevice, c->stream));
     }
-    const size_t off = off0;
-    const Dev &d = c->d;
-    CK(cudaMemsetAsync(d.Vb + off, 0, sizeof(float4) * slots, c->stream));
-    CK(cudaMemsetAsync(d.FC + off, 0, sizeof(float4) * slots, c->stream));
-    CK(cudaMemsetAsync(d.FD + off, 0, sizeof(float4) * slots, c->stream));
-    CK(cudaMemsetAsync(d.CM + P.base, 0, sizeof(float4) * P.cap, c->stream));
-    CK(cudaMemsetAsync(d.vol + P.base, 0, sizeof(float) * P.cap, c->stream));
-    CK(cudaMemsetAsync(d.area + P.base, 0, sizeof(float) * P.cap, c->stream));
-    CK(cudaMemsetAsync(d.divflag + P.base, 0, P.cap, c->stream));
-    CK(cudaMemcpyAsync(d.press + P.base, p.data(), sizeof(float) * P.cap, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d.E + P.base, e.data(), sizeof(float) * P.cap, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(&d.st[inst].n, &n, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    int zero = 0;
-    CK(cudaMemcpyAsync(&d.st[inst].step, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(&d.st[inst].err, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    static const float one3[3] = {1.0f, 1.0f, 1.0f};   // the reference's initial system centre
-    CK(cudaMemcpyAsync(d.st[inst].syscm, one3, sizeof one3, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    const int grid = (int)std::min<size_t>(((size_t)P.cap * SLOTS + 255) / 256, (size_t)c->nsm * 8);
+    k_load<<<grid, 256, 0, c->stream>>>(c->d, inst, n, with_v, pressure != nullptr, youngs != nullptr, stage);
+    CK(cudaGetLastError());
+    // the caller's arrays are free to change from here on
+    if (!small)
+        if (int rc = wait_stream(c)) return rc;
     c->n_now += n - c->hn[inst];
     c->hn[inst] = n;
     c->need_init = true;
     return CS3D_OK;
 }
 
+// The generator's words of an instance's state, in the order of cs3d_rng.
+constexpr size_t RNG_BYTES = sizeof(InstState) - offsetof(InstState, u);
+static_assert(offsetof(InstState, rc) - offsetof(InstState, u) == offsetof(cs3d_rng, c) &&
+                  offsetof(InstState, j97) - offsetof(InstState, u) == offsetof(cs3d_rng, j97) &&
+                  RNG_BYTES == offsetof(cs3d_rng, ok),
+              "InstState ends with cs3d_rng's fields");
+
 int cs3d_set_rng(cs3d_ctx *c, int inst, const cs3d_rng *r)
 {
     if (!c || !r || inst < 0 || inst >= c->n_inst || !r->ok) return CS3D_E_ARG;
     cudaSetDevice(c->device);
-    InstState st;
-    CK(cudaMemcpyAsync(&st, &c->d.st[inst], sizeof st, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    memcpy(st.u, r->u, sizeof st.u);
-    st.rc = r->c; st.rcd = r->cd; st.rcm = r->cm; st.i97 = r->i97; st.j97 = r->j97;
-    CK(cudaMemcpyAsync(&c->d.st[inst], &st, sizeof st, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    memcpy(c->buf.data(), r, RNG_BYTES);
+    CK(cudaMemcpyAsync(c->d.st[inst].u, c->buf.data(), RNG_BYTES, cudaMemcpyHostToDevice, c->stream));
     return CS3D_OK;
 }
 
@@ -860,12 +932,11 @@ int cs3d_get_rng(cs3d_ctx *c, int inst, cs3d_rng *r)
 {
     if (!c || !r || inst < 0 || inst >= c->n_inst) return CS3D_E_ARG;
     cudaSetDevice(c->device);
-    InstState st;
-    CK(cudaMemcpyAsync(&st, &c->d.st[inst], sizeof st, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    char *h = c->buf.data();
+    CK(cudaMemcpyAsync(h, c->d.st[inst].u, RNG_BYTES, cudaMemcpyDeviceToHost, c->stream));
+    if (int rc = wait_stream(c)) return rc;
     memset(r, 0, sizeof *r);
-    memcpy(r->u, st.u, sizeof r->u);
-    r->c = st.rc; r->cd = st.rcd; r->cm = st.rcm; r->i97 = st.i97; r->j97 = st.j97;
+    memcpy(r, h, RNG_BYTES);
     r->ok = 1;
     return CS3D_OK;
 }
@@ -921,10 +992,9 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
         c->prekicked = fuse == 2;
     }
     CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaEventSynchronize(c->ev1));
-    CK(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
     unsigned bits = 0;
     if ((rc = read_errors(c, &bits))) return rc;
+    CK(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
     if (bits & CS3D_ERRBIT_CAPACITY) return CS3D_E_CAPACITY;
     if (bits) return CS3D_E_DEVICE_FLAGS;
     return CS3D_OK;
@@ -995,20 +1065,13 @@ int cs3d_get_state(cs3d_ctx *c, int inst, int *n_cells, float *X, float *Y, floa
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;
-    int n = 0;
-    if ((rc = inst_count(c, inst, &n))) return rc;
+    const int n = c->hn[inst];
     if (n_cells) *n_cells = n;
-    if (X || Y || Z || VX || VY || VZ) {
-        float *const out[6] = {X, Y, Z, VX, VY, VZ};
-        const float4 *xs = c->prekicked ? c->d.Xe : c->d.X, *vs = c->prekicked ? c->d.Vb : c->d.V;
-        if ((rc = fetch_soa(c, inst, n, (X || Y || Z) ? xs : nullptr, (VX || VY || VZ) ? vs : nullptr, out)))
-            return rc;
-    }
-    const int base = c->hprm[inst].base;
-    if (pressure && n) CK(cudaMemcpyAsync(pressure, c->d.press + base, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
-    if (youngs && n) CK(cudaMemcpyAsync(youngs, c->d.E + base, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    return CS3D_OK;
+    const bool wx = X || Y || Z, wv = VX || VY || VZ;
+    if (!wx && !wv && !pressure && !youngs) return CS3D_OK;
+    float *const out[6] = {X, Y, Z, VX, VY, VZ};
+    const float4 *xs = c->prekicked ? c->d.Xe : c->d.X, *vs = c->prekicked ? c->d.Vb : c->d.V;
+    return fetch_soa(c, inst, n, wx ? xs : nullptr, wv ? vs : nullptr, out, pressure, youngs);
 }
 
 int cs3d_get_state_async(cs3d_ctx *c, int inst, int slot, int *n_cells, float *X, float *Y, float *Z, float *VX,
@@ -1018,8 +1081,7 @@ int cs3d_get_state_async(cs3d_ctx *c, int inst, int slot, int *n_cells, float *X
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;
-    int n = 0;
-    if ((rc = inst_count(c, inst, &n))) return rc;
+    const int n = c->hn[inst];
     if (n_cells) *n_cells = n;
     if (!c->copy_stream) CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     if (!c->astage[slot]) {
@@ -1040,13 +1102,13 @@ int cs3d_get_state_async(cs3d_ctx *c, int inst, int slot, int *n_cells, float *X
     const size_t off = (size_t)c->hprm[inst].base * SLOTS;
     const int base = c->hprm[inst].base;
     const bool wx = X || Y || Z, wv = VX || VY || VZ;
-    if (wx || wv)
-        k_unpack<<<c->grid_flat, 256, 0, c->stream>>>(stage, wx ? (c->prekicked ? c->d.Xe : c->d.X) + off : nullptr,
-                                                      wv ? (c->prekicked ? c->d.Vb : c->d.V) + off : nullptr, k);
+    if (wx || wv || pressure || youngs)
+        k_unpack<<<std::min(n, c->nsm * 8), 256, 0, c->stream>>>(stage, wx ? (c->prekicked ? c->d.Xe : c->d.X) + off : nullptr,
+                                                      wv ? (c->prekicked ? c->d.Vb : c->d.V) + off : nullptr, k,
+                                                      pressure ? c->d.press + base : nullptr,
+                                                      youngs ? c->d.E + base : nullptr, n);
     CK(cudaGetLastError());
     float *cellv = stage + 6 * k;
-    if (pressure) CK(cudaMemcpyAsync(cellv, c->d.press + base, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
-    if (youngs) CK(cudaMemcpyAsync(cellv + n, c->d.E + base, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaEventRecord(c->aready[slot], c->stream));
     CK(cudaStreamWaitEvent(c->copy_stream, c->aready[slot], 0));
     float *const out[6] = {X, Y, Z, VX, VY, VZ};
@@ -1091,8 +1153,7 @@ int cs3d_get_forces(cs3d_ctx *c, int inst, float *FCX, float *FCY, float *FCZ, f
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;
-    int n = 0;
-    if ((rc = inst_count(c, inst, &n))) return rc;
+    const int n = c->hn[inst];
     float *const out[6] = {FCX, FCY, FCZ, FDX, FDY, FDZ};
     return fetch_soa(c, inst, n, (FCX || FCY || FCZ) ? c->d.FC : nullptr, (FDX || FDY || FDZ) ? c->d.FD : nullptr,
                      out);
@@ -1104,8 +1165,7 @@ int cs3d_get_random_force(cs3d_ctx *c, int inst, float *FRX, float *FRY, float *
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;
-    int n = 0;
-    if ((rc = inst_count(c, inst, &n))) return rc;
+    const int n = c->hn[inst];
     float *const out[6] = {FRX, FRY, FRZ, nullptr, nullptr, nullptr};
     return fetch_soa(c, inst, n, c->d.FR, nullptr, out);
 }
@@ -1116,8 +1176,7 @@ int cs3d_get_cells(cs3d_ctx *c, int inst, float *cm, float *volume, float *area,
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;
-    int n = 0;
-    if ((rc = inst_count(c, inst, &n))) return rc;
+    const int n = c->hn[inst];
     const int base = c->hprm[inst].base;
     if (cm && n) {
         std::vector<float4> b(n);
@@ -1227,8 +1286,7 @@ int cs3d_volume_histogram(cs3d_ctx *c, int inst, float lo, float hi, int nbins, 
     int rc = ensure_init(c);
     if (rc) return rc;
     if ((rc = settle(c))) return rc;   // the volumes of the step-end positions
-    int n = 0;
-    if ((rc = inst_count(c, inst, &n))) return rc;
+    const int n = c->hn[inst];
     // scratch for the counts and the volumes, freed before returning
     unsigned long long *dc = nullptr;
     float *dv = nullptr;
@@ -1322,9 +1380,16 @@ constexpr int SCAP = CS3D_STATIC_MAX_CELLS;
 constexpr int SBINS = table_size(SCAP);
 constexpr int SEVENTS = 16;
 
-struct StaticScratch {
+// What a call brings along, in one copy.
+struct StaticHead {
     InstParams prm;
     InstState st;
+    alignas(16) TopoTables topo;
+};
+
+struct StaticScratch {
+    StaticHead head;
+    alignas(16)
     float4 X[SCAP * SLOTS], V[SCAP * SLOTS], Vb[SCAP * SLOTS], FC[SCAP * SLOTS], FD[SCAP * SLOTS], Xb[SCAP * SLOTS];
     float4 FR[SCAP * SLOTS];
     float4 CM[SCAP];
@@ -1351,12 +1416,6 @@ struct StaticScratch {
     int flags[4], deal[DEALS];
     int4 pairs[1];
     unsigned long long n_pairs;
-    uint32_t nnpack[SLOTS];
-    float4 r0[SLOTS], th0[SLOTS];
-    uint4 arm[SLOTS];
-    uint8_t faces[CS3D_FACES * 7], patch[SLOTS];
-    double2 cs0[3 * SLOTS];
-    double r0i[3 * SLOTS];
 };
 
 // The scratch of cs3d_forces_static.  In host code this name is only a
@@ -1380,16 +1439,9 @@ Dev static_dev(StaticScratch *s)
     d.n_inst = 1;
     d.cap_total = SCAP;
     d.single = 1;
-    d.prm = &s->prm;
-    d.st = &s->st;
-    d.topo.nnpack = s->nnpack;
-    d.topo.r0 = s->r0;
-    d.topo.th0 = s->th0;
-    d.topo.arm = s->arm;
-    d.topo.faces = s->faces;
-    d.topo.patch = s->patch;
-    d.topo.cs0 = s->cs0;
-    d.topo.r0i = s->r0i;
+    d.prm = &s->head.prm;
+    d.st = &s->head.st;
+    d.topo = topo_pointers(&s->head.topo);
     d.X = s->X; d.V = s->V; d.Vb = s->Vb; d.FC = s->FC; d.FD = s->FD; d.Xb = s->Xb; d.FR = s->FR;
     d.CM = s->CM;
     d.press = s->press; d.E = s->E; d.vol = s->vol; d.area = s->area;
@@ -1488,8 +1540,8 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
         return CS3D_E_ARG;
     }
     if (check_params(*params)) return CS3D_E_CONFIG;
-    TopoTables tt;
-    int rc = topo_tables(topo, tt);
+    StaticHead head;
+    int rc = topo_tables(topo, head.topo);
     if (rc) return rc;
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -1498,30 +1550,15 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     cudaStream_t s = (cudaStream_t)stream;
     StaticScratch *S = sd->base;
     const Dev d = static_dev(S);
-    // parameters, mesh tables and a cleared instance state
-    const InstParams ip = make_inst(*params, 0, SCAP, 0.1f, inv_bin_edge(topo));
-    InstState st0;
-    memset(&st0, 0, sizeof st0);
-    st0.n = n_cells;
-    CK(cudaMemcpyAsync(&S->prm, &ip, sizeof ip, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(&S->st, &st0, sizeof st0, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->nnpack, tt.nnp, sizeof tt.nnp, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->r0, tt.r0, sizeof tt.r0, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->th0, tt.th, sizeof tt.th, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->arm, tt.arm, sizeof tt.arm, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->faces, tt.faces, sizeof tt.faces, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->patch, tt.patch, sizeof tt.patch, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->cs0, tt.cs0, sizeof tt.cs0, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(S->r0i, tt.r0i, sizeof tt.r0i, cudaMemcpyHostToDevice, s));
-    // the previous call's neighbour lists, boxes and flags must not leak in
-    CK(cudaMemsetAsync(S->ncand, 0, sizeof S->ncand, s));
-    CK(cudaMemsetAsync(S->nent, 0, sizeof S->nent, s));
-    CK(cudaMemsetAsync(S->flags, 0, sizeof S->flags, s));
-    CK(cudaMemsetAsync(&S->n_events, 0, sizeof S->n_events, s));
+    // parameters, mesh tables and a cleared instance state (the whole build of
+    // the lists replaces everything else that an earlier call left)
+    head.prm = make_inst(*params, 0, SCAP, 0.1f, inv_bin_edge(topo));
+    memset(&head.st, 0, sizeof head.st);
+    head.st.n = n_cells;
+    CK(cudaMemcpyAsync(&S->head, &head, sizeof head, cudaMemcpyHostToDevice, s));
     k_static_load<<<sd->grid_flat, 256, 0, s>>>(d, n_cells, X, Y, Z, VX, VY, VZ, pressure, youngs, params->min_pressure,
                                                   params->stiffness1);
     // the initialisation sequence of run_init on the static buffers
-    k_build_work<<<1, 256, 0, s>>>(d);
     k_init_begin<<<1, 256, 0, s>>>(d);
     k_geom<<<sd->grid_cells, SLOTS, 0, s>>>(d, 0);
     // correct_com at set-up, as run_init (src/GPUbounce.cu:785-805): the shift
@@ -1532,7 +1569,7 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     k_static_store<<<sd->grid_flat, 256, 0, s>>>(d, n_cells, FCX, FCY, FCZ, FDX, FDY, FDZ);
     CK(cudaGetLastError());
     unsigned err = 0;
-    CK(cudaMemcpyAsync(&err, &S->st.err, sizeof err, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&err, &S->head.st.err, sizeof err, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return err ? CS3D_E_DEVICE_FLAGS : CS3D_OK;
 }
