@@ -138,7 +138,7 @@ struct Dev {
     float *cdisp;       // [cell] largest distance of its nodes from their anchors
     int *build;         // cells of this step's partial builds
     int *n_build;
-    uint8_t *mark;      // [cell] of them: 1 near a divided cell, 2 divided
+    uint8_t *mark;      // [cell] in partial builds: 1 near a divided cell, 2 divided
     unsigned *epoch;
     DivEntry *divtab;
     int *div_total;
@@ -151,7 +151,7 @@ struct Dev {
     uint8_t *pick;      // [cap_total + n_inst] flags of the random soft-cell picks
     int *n_events;
     int ev_cap;
-    int *flags;         // [0] any rebuild, [1] any division, [2] any partial build turned whole
+    int *flags;         // [0] any rebuild, [1] any division
     int *deal;          // counters of the cells dealt out, by phase (Dealer)
     unsigned *bar;      // [0] arrivals, [1] barriers passed (k_steps; zero at its launch)
     int4 *pairs;        // (cell_a<<8 | node_i, cell_b<<8 | node_j, kind, 0)

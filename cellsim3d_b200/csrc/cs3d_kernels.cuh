@@ -117,7 +117,7 @@ struct Dealer {
         turn ^= 1;
     }
 };
-enum { DEAL_S1, DEAL_S2, DEAL_LISTS, DEAL_FULL, DEALS };
+enum { DEAL_S1, DEAL_S2, DEAL_LISTS, DEALS };
 
 // Kick of the split velocity Verlet with the reference's mixed precision:
 // the float sum is scaled by the double literal 0.5 and divided by the mass
@@ -391,11 +391,13 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
         }
         __syncwarp();
         // the next eight, in flight during the rounds
+        if (k0 + EPRE < most) {
 #pragma unroll
-        for (int k = 0; k < EPRE; ++k) {
-            const int q = k0 + EPRE + k;
-            const unsigned e = q < ne ? ep[(size_t)q * SLOTS] : 0u;
-            w[k / 2] = k & 1 ? w[k / 2] | e << 16 : e;
+            for (int k = 0; k < EPRE; ++k) {
+                const int q = k0 + EPRE + k;
+                const unsigned e = q < ne ? ep[(size_t)q * SLOTS] : 0u;
+                w[k / 2] = k & 1 ? w[k / 2] | e << 16 : e;
+            }
         }
         for (int b = 0; b < m; b += 32) {
             const bool act = b + lane < m;
@@ -721,7 +723,6 @@ __device__ __forceinline__ void step_begin(const Dev &d, int par_next)
     if (threadIdx.x == 0) {
         d.flags[0] = any;
         d.flags[1] = 0;
-        d.flags[2] = 0;
         *d.n_pairs = 0ull;
     }
 }
@@ -756,7 +757,6 @@ __global__ void __launch_bounds__(256) k_init_begin(Dev d)
     assign_hash_slices<256>(d);
     if (threadIdx.x == 0) {
         d.flags[0] = 1;
-        d.flags[2] = 0;
         *d.n_build = 0;
         for (int q = 0; q < DEALS; ++q) d.deal[q] = 0;
         *d.div_total = 0;
@@ -918,8 +918,10 @@ struct S1Smem {
     double3 xd[SLOTS];   // FP64 copies of the positions and velocities: the
     double3 vd[SLOTS];   // FP64 terms read them without conversions
     SlotData sd;
-    SweepSmem sweep[SLOTS / 32];
-    ArmForces arm;
+    union {                         // the angles' arms are read before the sweep begins: the
+        SweepSmem sweep[SLOTS / 32];  // room is worth more as L1 (S1 of 100,000 packed
+        ArmForces arm;                // cells 1.76 -> 1.73 ms, a barrier included)
+    };
     float press;         // the cell's pressure of this step
     int next[2];
 };
@@ -1022,6 +1024,7 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
                 FZ += sm.arm.z[am.x] + sm.arm.z[am.y] + sm.arm.z[am.z] - (sm.arm.z[o] + sm.arm.z[o + 1] + sm.arm.z[o + 2]);
             }
         }
+        __syncthreads();
         // contacts, src/propagate.cu:356-442 and the first dissipative sweep
         double3 vsum = make_double3(0.0, 0.0, 0.0);
         const int nd = sweep_s1<COOP>(d, P, sm.sd, sm.sweep[i >> 5], a, i, x, v, ne, pre, FX, FY, FZ, vsum);
@@ -1894,11 +1897,7 @@ constexpr float BOX_REACH = 1.0001f;
 
 // B2: the cells to build into d.build, one thread per cell: all cells of whole
 // builds, and those that partial builds concern (the divided ones and those
-// whose boxes come within the list radius of one).  Where one of the latter has moved more than skin/4 from its anchors,
-// its radius would lengthen its lists too much (64 entries a node is the
-// limit): the instance is rebuilt whole.  Deciding this for the cells at the
-// divisions and not for the farthest node of the instance leaves a third of
-// the whole builds of a growing colony.
+// whose boxes come within the list radius of one).
 __device__ __forceinline__ void nb_mark(const Dev &d)
 {
     const int W = n_work(d), T = *d.div_prev;
@@ -1906,15 +1905,12 @@ __device__ __forceinline__ void nb_mark(const Dev &d)
         const int a = cell_of(d, w);
         const int inst = inst_of(d, a);
         InstState *st = &d.st[inst];
-        const int rb = __ldcg(&st->rebuild);
+        const int rb = st->rebuild;
         if (rb != 1) {
-            // whole build (one that this phase decided on: left to the CTAs'
-            // second pass, unless it is seen here)
-            d.mark[a] = rb == 2 ? 4 : 0;
             if (rb == 2) d.build[atomicAdd(d.n_build, 1)] = a;
+            d.mark[a] = 0;
             continue;
         }
-        d.mark[a] = 0;
         const InstParams &P = d.prm[inst];
         const float4 lo = d.nbox[2 * a], hi = d.nbox[2 * a + 1];
         const float da = d.cdisp[a];
@@ -1932,14 +1928,8 @@ __device__ __forceinline__ void nb_mark(const Dev &d)
                     m |= 1;
             }
         }
-        if (!m) continue;
         d.mark[a] = (uint8_t)m;
-        d.build[atomicAdd(d.n_build, 1)] = a;
-        if (m == 1 && da > 0.25f * P.skin && atomicExch(&st->rebuild, 2) != 2) {
-            st->rebuilds += 1;
-            st->rebuilds_div += 1;
-            d.flags[2] = 1;
-        }
+        if (m) d.build[atomicAdd(d.n_build, 1)] = a;
     }
 }
 
@@ -2163,9 +2153,11 @@ __device__ __forceinline__ void list_stats(const Dev &d, ListSmem &sm)
     if (d.halo_stats) atomicMax(&st->max_halo, sm.max_halo);
 }
 
-// B3: the lists of cell a.  The whole CTA; its warps take a patch of 30
-// neighbouring nodes each.
-__device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned epoch, ListSmem &sm)
+// B3: the lists of cell a, with the radius of whole builds (full) or with the
+// cells' displacements.  The whole CTA; its warps take a patch of 30
+// neighbouring nodes each.  False, without full only, if some node has more
+// entries than it has room for.
+__device__ __forceinline__ bool nb_cell(const Dev &d, int a, int node, unsigned epoch, bool full, ListSmem &sm)
 {
     const int t = threadIdx.x, wid = t >> 5, lane = t & 31;
     const bool real = node < NODES;
@@ -2173,9 +2165,8 @@ __device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned 
     const int inst = inst_of(d, a);
     InstState *st = &d.st[inst];
     const InstParams &P = d.prm[inst];
-    const bool full = st->rebuild == 2;
     const float da = full ? 0.0f : d.cdisp[a];
-    const bool fresh = full || (d.mark[a] & 2);   // new anchors
+    const bool fresh = st->rebuild == 2 || (d.mark[a] & 2);   // new anchors
     const float4 lo = d.nbox[2 * a], hi = d.nbox[2 * a + 1];
     const size_t g = (size_t)a * SLOTS + node;
     const float4 x = real ? d.X[g] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
@@ -2257,6 +2248,7 @@ __device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned 
             }
         }
     }
+    if (!full && __syncthreads_or(e.cnt > MAXE)) return false;
     if (real) {
         d.nent[g] = (uint8_t)(e.cnt < MAXE ? e.cnt : MAXE);
         // new anchors, except for the neighbours of divided cells: other
@@ -2287,10 +2279,13 @@ __device__ __forceinline__ void nb_cell(const Dev &d, int a, int node, unsigned 
         sm.max_cand = max(sm.max_cand, nslot > MAXC ? nslot : nused);
         sm.max_halo = max(sm.max_halo, nh);
     }
+    return true;
 }
 
-// The listed cells, then the other cells of the instances that nb_mark turned
-// to whole builds.
+// The listed cells.  Where a partial build's radius gives a node more entries
+// than it has room for (cells far from their anchors in a crowd), the cell's
+// lists are built with the radius of a whole build, which covers this step, and
+// the instance is rebuilt whole in the next one.
 __device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
 {
     const int t = threadIdx.x;
@@ -2298,22 +2293,17 @@ __device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
     const int node = __ldg(&d.topo.patch[t]);
     if (t == 0) sm.st_inst = -1;
     const int N = *d.n_build;
-    Dealer listed(&d.deal[DEAL_LISTS], sm.next);
-    while (listed.w < N) {
-        const int a = d.build[listed.w];
-        listed.draw();
-        nb_cell(d, a, node, epoch, sm);
-        listed.advance();
-    }
-    const int W = d.flags[2] ? n_work(d) : 0;
-    __syncthreads();
-    Dealer other(&d.deal[DEAL_FULL], sm.next);
-    while (other.w < W) {
-        const int a = cell_of(d, other.w);
-        other.draw();
-        if (d.st[inst_of(d, a)].rebuild == 2 && !d.mark[a]) nb_cell(d, a, node, epoch, sm);   // uniform
-        else __syncthreads();
-        other.advance();
+    Dealer deal(&d.deal[DEAL_LISTS], sm.next);
+    while (deal.w < N) {
+        const int a = d.build[deal.w];
+        deal.draw();
+        InstState *st = &d.st[inst_of(d, a)];
+        bool full = st->rebuild == 2;
+        while (!nb_cell(d, a, node, epoch, full, sm)) {
+            full = true;
+            if (t == 0) st->force_rebuild = 1;
+        }
+        deal.advance();
     }
     __syncthreads();
     if (t == 0) list_stats(d, sm);

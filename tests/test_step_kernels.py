@@ -174,3 +174,25 @@ def test_forces_of_bent_and_crowded_cells(mesh, make, arg):
     for kind in (0, 1):
         assert np.array_equal(sorted_pairs(sim.pairs(kind)), sorted_pairs(orc.recorded_pairs(kind)))
     sim.close()
+
+
+@pytest.mark.parametrize("skin", [0.25, 0.35])
+def test_crowded_partial_builds_fall_back(mesh, skin):
+    """A growing colony with a wide list skin against the default one, bit for
+    bit.  At 0.35 the radius of a partial build around a division gives some
+    node more entries than it has room for (a whole build stays below): the
+    cell takes the smaller radius and the instance is rebuilt in the next step."""
+    p, st = _growing(64)
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
+    got = []
+    for s in (0.1, skin):
+        sim = cs.Simulation(p, topo, 512)
+        sim.set_option(cs.OPT_SKIN, int(round(s * 1e6)))
+        sim.load_state(st["X"], st["Y"], st["Z"], n_cells=64)
+        sim.step(1200)
+        got.append((sim.state(), sim.events()))
+        sim.close()
+    (a, ea), (b, eb) = got
+    assert np.array_equal(ea, eb)
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
