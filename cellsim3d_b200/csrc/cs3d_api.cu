@@ -377,15 +377,14 @@ struct Prof {
 
 // Neighbour-list build: the cells' boxes and table, then the per-cell lists.
 // Both kernels return at once when no instance rebuilds this step.
-int launch_nl_kernels(const Dev &d, cudaStream_t s, int grid_lists, int grid_boxes, const Prof &pf = Prof())
+int launch_nl_kernels(const Dev &d, int par, cudaStream_t s, int grid_lists, int grid_boxes, const Prof &pf = Prof())
 {
-    k_nb_boxes<<<grid_boxes, SLOTS, 0, s>>>(d); pf.mark(s, "nb_boxes");
-    k_nb_mark<<<grid_boxes, SLOTS, 0, s>>>(d); pf.mark(s, "nb_mark");
+    k_nb_boxes<<<grid_boxes, SLOTS, 0, s>>>(d, par); pf.mark(s, "nb_boxes");
     k_nb_lists<<<grid_lists, SLOTS, 0, s>>>(d); pf.mark(s, "nb_lists");
     CK(cudaGetLastError());
     return CS3D_OK;
 }
-constexpr int NL_LAUNCHES = 3;
+constexpr int NL_LAUNCHES = 2;
 
 // Centre-of-mass correction: every instance's centre, then the shift.
 void launch_com(const Dev &d, cudaStream_t s, int grid, const Prof &pf = Prof())
@@ -394,9 +393,9 @@ void launch_com(const Dev &d, cudaStream_t s, int grid, const Prof &pf = Prof())
     k_com_shift<<<grid, SLOTS, 0, s>>>(d); pf.mark(s, "com_shift");
 }
 
-int launch_nl_build(cs3d_ctx *c, const Prof &pf = Prof())
+int launch_nl_build(cs3d_ctx *c, int par, const Prof &pf = Prof())
 {
-    return launch_nl_kernels(c->d, c->stream, c->grid_lists, c->grid_boxes, pf);
+    return launch_nl_kernels(c->d, par, c->stream, c->grid_lists, c->grid_boxes, pf);
 }
 
 // Bins of the list build's cell table for a capacity of `cells` cells.
@@ -429,7 +428,7 @@ int run_init(cs3d_ctx *c)
     // before the first force evaluation
     if (c->any_com) launch_com(d, s, c->grid_s2);
     CK(cudaGetLastError());
-    int rc = launch_nl_build(c);
+    int rc = launch_nl_build(c, 0);
     if (rc) return rc;
     k_s1<true><<<c->grid_cells, SLOTS, sizeof(S1Smem), s>>>(d, 0);
     CK(cudaGetLastError());
@@ -453,7 +452,7 @@ int launch_step(cs3d_ctx *c, int par, bool div, bool k1 = true, int fuse = 0, co
     int n = 0;
     if (k1) { k_integrate<<<c->grid_s2, SLOTS, 0, s>>>(d); ++n; pf.mark(s, "integrate"); }
     k_step_begin<<<1, 256, 0, s>>>(d, par ^ 1); ++n; pf.mark(s, "step_begin");
-    int rc = launch_nl_build(c, pf);
+    int rc = launch_nl_build(c, par, pf);
     if (rc) return rc;
     n += NL_LAUNCHES;
     k_s1<false><<<c->grid_cells, SLOTS, sizeof(S1Smem), s>>>(d, par); ++n; pf.mark(s, "s1_con_dis");
@@ -465,10 +464,9 @@ int launch_step(cs3d_ctx *c, int par, bool div, bool k1 = true, int fuse = 0, co
     else k_s2<false, 0><<<c->grid_s2, SLOTS, 0, s>>>(d, par);
     ++n; pf.mark(s, fuse ? "s2_dis_geom_integrate" : "s2_dis_geom");
     if (div) {
-        k_div_select<<<c->n_inst, 256, 0, s>>>(d, par); ++n; pf.mark(s, "div_select");
-        k_div_apply<<<c->grid_cells, SLOTS, 0, s>>>(d, par); ++n; pf.mark(s, "div_apply");
+        k_div_select<<<c->n_inst, 256, 0, s>>>(d, par, c->any_far); ++n; pf.mark(s, "div_select");
         // S2 did the next half kick of every cell that does not divide
-        k_div_finish<<<c->grid_cells, SLOTS, 0, s>>>(d, par, c->any_far, fuse != 0); ++n; pf.mark(s, "div_finish");
+        k_div_apply<<<c->grid_cells, SLOTS, 0, s>>>(d, par, fuse != 0); ++n; pf.mark(s, "div_apply");
     }
     if (soften) { k_soften<<<c->n_inst, 32, 0, s>>>(d, (int)soften); ++n; pf.mark(s, "soften"); }
     if (c->any_com) { launch_com(d, s, c->grid_s2, pf); n += 2; }
@@ -1564,7 +1562,7 @@ extern "C" int cs3d_forces_static(const cs3d_params *params, const cs3d_topology
     // correct_com at set-up, as run_init (src/GPUbounce.cu:785-805): the shift
     // moves the positions the wall and contact forces see
     if (params->correct_com) launch_com(d, s, sd->grid_cells);
-    if ((rc = launch_nl_kernels(d, s, sd->grid_lists, sd->grid_boxes))) return rc;
+    if ((rc = launch_nl_kernels(d, 0, s, sd->grid_lists, sd->grid_boxes))) return rc;
     k_s1<true><<<sd->grid_cells, SLOTS, sizeof(S1Smem), s>>>(d, 0);
     k_static_store<<<sd->grid_flat, 256, 0, s>>>(d, n_cells, FCX, FCY, FCZ, FDX, FDY, FDZ);
     CK(cudaGetLastError());

@@ -609,18 +609,6 @@ __global__ void __launch_bounds__(SLOTS) k_integrate(Dev d)
     for (int w = blockIdx.x; w < W; w += gridDim.x) integrate_cell(d, cell_of(d, w), smax);
 }
 
-// The next step's half kick and drift of the two cells of each division of
-// this step, after their placement (division steps whose S2 did the others).
-__device__ __forceinline__ void integrate_divided(const Dev &d, float *smax)
-{
-    const int T = *d.div_total;
-    for (int q = blockIdx.x; q < T; q += gridDim.x) {
-        const DivEntry e = d.divtab[q];
-        integrate_cell(d, e.parent, smax);
-        integrate_cell(d, e.daughter, smax);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Per-step bookkeeping (one block): step counter, rebuild decision, reset of
 // the accumulators that this step fills.
@@ -834,8 +822,8 @@ __device__ __forceinline__ double sqrt_full(double x)
 // of |det| / 6 of the tetrahedra (centre of mass, triangle) and the area the
 // sum of the triangle areas.  The face centres first (one thread per face)
 // , then the 552 triangles dealt out to all threads.
-__device__ __noinline__ void cell_volume(const uint8_t *faces, const uint32_t *tris, const float4 *xs, float3 cm, GeomScratch &gs, bool sph,
-                                         double &vol, double &area)
+__device__ __noinline__ void cell_volume(const uint8_t *faces, const uint32_t *tris, const float4 *xs, float3 cm,
+                                         GeomScratch &gs, bool sph, double &vol, double &area)
 {
     const int t = threadIdx.x, w = t >> 5, l = t & 31;
     const double cx = cm.x, cy = cm.y, cz = cm.z;
@@ -1236,7 +1224,7 @@ __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, 
         if (FUSE && DIV) {
             // With the division decision known: a cell that does not divide
             // takes the next step's half kick and drift here, the two cells of
-            // a division after their placement (k_integrate_divided).
+            // a division after their placement (k_div_apply).
             __syncthreads();
             const bool divides = sm.dflag != 0;   // uniform
             if (FUSE == 2 && !divides && i < NODES) d.Xe[g] = x4;
@@ -1258,7 +1246,9 @@ __device__ __forceinline__ void s2_cells(const Dev &d, int par, const int FUSE, 
             d.CM[a] = make_float4(cm.x, cm.y, cm.z, 0.f);
             d.aabb[pn][2 * a] = lo;
             d.aabb[pn][2 * a + 1] = hi;
-            if (inst != acc_inst) {
+            if (DIV && sm.dflag) {
+                // the boxes of its two cells enter the extents after their placement
+            } else if (inst != acc_inst) {
                 if (acc_inst >= 0) flush_mm(d, acc_inst, pn, acc);
                 acc_inst = inst;
                 acc[0] = lo.x; acc[1] = hi.x; acc[2] = lo.y; acc[3] = hi.y; acc[4] = lo.z; acc[5] = hi.z;
@@ -1311,6 +1301,70 @@ __global__ void __launch_bounds__(SLOTS) k_geom(Dev d, int par)
     }
 }
 
+// calc_sys_CM, src/GPUbounce.cu:2504-2520: the float mean of the first n
+// centres of mass, summed in cell order; recorded as the instance's system
+// centre.
+__device__ __forceinline__ float3 sys_centre(const Dev &d, const InstParams &P, InstState *st, int n)
+{
+    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+    for (int c = 0; c < n; ++c) {
+        const float4 cm = d.CM[P.base + c];
+        sx = __fadd_rn(sx, cm.x);
+        sy = __fadd_rn(sy, cm.y);
+        sz = __fadd_rn(sz, cm.z);
+    }
+    sx = __fdiv_rn(sx, (float)n);
+    sy = __fdiv_rn(sy, (float)n);
+    sz = __fdiv_rn(sz, (float)n);
+    st->syscm[0] = sx;
+    st->syscm[1] = sy;
+    st->syscm[2] = sz;
+    return make_float3(sx, sy, sz);
+}
+
+__device__ __forceinline__ float dist2(float4 cm, float3 o)
+{
+    const float dx = __fsub_rn(cm.x, o.x), dy = __fsub_rn(cm.y, o.y), dz = __fsub_rn(cm.z, o.z);
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+}
+
+// getRmax2, src/GPUbounce.cu:2523-2536: the largest squared distance of the
+// first n centres of mass from the recorded system centre.
+__device__ __forceinline__ float rmax2_from(const Dev &d, const InstParams &P, const InstState *st, int n)
+{
+    const float3 o = make_float3(st->syscm[0], st->syscm[1], st->syscm[2]);
+    float r2 = 0.0f;
+    for (int c = 0; c < n; ++c) {
+        const float v = dist2(d.CM[P.base + c], o);
+        r2 = r2 < v ? v : r2;   // std::max
+    }
+    return r2;
+}
+
+// num_cells_far, src/GPUbounce.cu:1288-1290 and :2538-2565, after the
+// divisions of a step (count_only_internal_cells): the newest div_count cells
+// whose centre of mass lies farther than radius_cutoff x the largest distance
+// from the system's centre are not counted as dividing.  The daughters'
+// centres of mass are still 0 here (computed in their first step), as in the
+// reference.  One thread per instance (k).
+__device__ __forceinline__ void far_count(const Dev &d, int k)
+{
+    const InstParams &P = d.prm[k];
+    InstState *st = &d.st[k];
+    if (!(P.far_r > 0.0f) || !(st->step <= P.div_steps && P.growth > 0.0f)) return;
+    const int n = st->n, nd = st->div_count;
+    if (nd == 0 || n < 50) return;
+    const float3 o = sys_centre(d, P, st, n);
+    const float thr = __fmul_rn(__fmul_rn(P.far_r, P.far_r), rmax2_from(d, P, st, n));
+    int far = 0;
+    for (int c = n - nd; c < n; ++c)
+        if (dist2(d.CM[P.base + c], o) > thr) ++far;
+    if (far) {
+        const int q = atomicAdd(d.n_far, 1);
+        if (q < d.far_cap) d.farlog[q] = make_int4(k, st->step, far, 0);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Division (src/GPUbounce.cu:1210-1286, src/postscriptinit.cu:148-256).
 // D1: one block per instance, dividers in ascending index order, one RANMAR
@@ -1353,6 +1407,16 @@ __device__ void random_vector_dev(S *st, float n[3])
     n[2] = __fsub_rn(1.0f, __fmul_rn(2.0f, __fadd_rn(__fmul_rn(x1, x1), __fmul_rn(x2, x2))));
 }
 
+// Cell a's box of this step (aabb[pn]) into its instance's grid extents.
+__device__ __forceinline__ void add_extents(const Dev &d, InstState *st, int pn, int a)
+{
+    const float4 lo = d.aabb[pn][2 * a], hi = d.aabb[pn][2 * a + 1];
+    int *mm = st->mm[pn];
+    atomicMin(&mm[0], f2o(lo.x)); atomicMax(&mm[1], f2o(hi.x));
+    atomicMin(&mm[2], f2o(lo.y)); atomicMax(&mm[3], f2o(hi.y));
+    atomicMin(&mm[4], f2o(lo.z)); atomicMax(&mm[5], f2o(hi.z));
+}
+
 struct DivRng {
     float u[98];
     float rc, rcd, rcm;
@@ -1365,9 +1429,9 @@ struct DivSmem {
     int base;
 };
 
-// NT threads; k: the instance.
+// NT threads; k: the instance; far: some instance counts internal cells.
 template <int NT>
-__device__ __forceinline__ void div_select(const Dev &d, int par, int k, DivSmem &sm)
+__device__ __forceinline__ void div_select(const Dev &d, int par, int k, bool far, DivSmem &sm)
 {
     InstState *st = &d.st[k];
     const InstParams &P = d.prm[k];
@@ -1403,13 +1467,13 @@ __device__ __forceinline__ void div_select(const Dev &d, int par, int k, DivSmem
                 e.parent = a;
                 e.daughter = P.base + n0 + r;
                 e.inst = k;
-            }
+            } else add_extents(d, st, par ^ 1, a);
         }
         __syncthreads();
     } else {
         // many: ascending compaction of the flags in chunks of NT
         int done = 0;
-        for (int c0 = 0; c0 < n0 && done < ndiv; c0 += NT) {
+        for (int c0 = 0; c0 < n0 && done < total; c0 += NT) {
             const int c = c0 + t;
             const int f = (c < n0) ? (d.divflag[P.base + c] ? 1 : 0) : 0;
             const unsigned b = __ballot_sync(0xffffffffu, f);
@@ -1424,7 +1488,7 @@ __device__ __forceinline__ void div_select(const Dev &d, int par, int k, DivSmem
                 e.parent = P.base + c;
                 e.daughter = P.base + n0 + off;
                 e.inst = k;
-            }
+            } else if (f) add_extents(d, st, par ^ 1, P.base + c);
             int tot = 0;
             for (int q = 0; q < NT / 32; ++q) tot += sm.warp_cnt[q];
             done += tot;
@@ -1447,25 +1511,23 @@ __device__ __forceinline__ void div_select(const Dev &d, int par, int k, DivSmem
         }
         st->n = n0 + ndiv;
         st->rc = sm.rng.rc; st->i97 = sm.rng.i97; st->j97 = sm.rng.j97;
-        for (int q = 0; q < 3; ++q) {
-            st->mm[par ^ 1][2 * q] = f2o(1.0e30f);
-            st->mm[par ^ 1][2 * q + 1] = f2o(-1.0e30f);
-        }
+        if (far) far_count(d, k);
     }
     __syncthreads();
     for (int q = t; q < 98; q += NT) st->u[q] = sm.rng.u[q];
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_div_select(Dev d, int par)
+__global__ void __launch_bounds__(256) k_div_select(Dev d, int par, int far)
 {
     __shared__ DivSmem sm;
-    if (d.flags[1] && (int)blockIdx.x < d.n_inst) div_select<256>(d, par, blockIdx.x, sm);
+    if (d.flags[1] && (int)blockIdx.x < d.n_inst) div_select<256>(d, par, blockIdx.x, far != 0, sm);
 }
 
 // D2: one block per division: the two daughters by half-space projection
 // through CM + n*gap/2 (FP64 geometry), velocities, pressures, stiffness.
-__device__ __forceinline__ void div_apply(const Dev &d, int par, float4 *xs, GeomScratch &gs)
+// With fuse also their next half kick and drift, which S2 gave every other cell.
+__device__ __forceinline__ void div_apply(const Dev &d, int par, bool fuse, float4 *xs, GeomScratch &gs, float *smax)
 {
     const int T = *d.div_total;
     const int pn = par ^ 1;
@@ -1508,6 +1570,7 @@ __device__ __forceinline__ void div_apply(const Dev &d, int par, float4 *xs, Geo
             geom_box(gs, lo, hi);
             d.aabb[pn][2 * a] = lo;
             d.aabb[pn][2 * a + 1] = hi;
+            add_extents(d, &d.st[e.inst], pn, a);
         }
         __syncthreads();
         xs[i] = xb;
@@ -1517,6 +1580,7 @@ __device__ __forceinline__ void div_apply(const Dev &d, int par, float4 *xs, Geo
             geom_box(gs, lo, hi);
             d.aabb[pn][2 * b] = lo;
             d.aabb[pn][2 * b + 1] = hi;
+            add_extents(d, &d.st[e.inst], pn, b);
             d.press[a] = P.minp;
             d.press[b] = P.minp;
             d.E[b] = P.daught_same ? d.E[a] : P.stiff1;
@@ -1536,14 +1600,19 @@ __device__ __forceinline__ void div_apply(const Dev &d, int par, float4 *xs, Geo
             d.FD[gb] = make_float4(0, 0, 0, 0);
         }
         __syncthreads();
+        if (fuse) {   // a thread's own nodes
+            integrate_cell(d, a, smax);
+            integrate_cell(d, b, smax);
+        }
     }
 }
 
-__global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par)
+__global__ void __launch_bounds__(SLOTS) k_div_apply(Dev d, int par, int fuse)
 {
     __shared__ float4 xs[SLOTS];
     __shared__ GeomScratch gs;
-    div_apply(d, par, xs, gs);
+    __shared__ float smax[SLOTS / 32];
+    div_apply(d, par, fuse != 0, xs, gs, smax);
 }
 
 // CoM correction at the end of a step (correct_com, src/GPUbounce.cu:1430-1440
@@ -1611,70 +1680,6 @@ __device__ __forceinline__ void com_shift(const Dev &d)
 }
 
 __global__ void __launch_bounds__(SLOTS) k_com_shift(Dev d) { com_shift(d); }
-
-// calc_sys_CM, src/GPUbounce.cu:2504-2520: the float mean of the first n
-// centres of mass, summed in cell order; recorded as the instance's system
-// centre.
-__device__ __forceinline__ float3 sys_centre(const Dev &d, const InstParams &P, InstState *st, int n)
-{
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    for (int c = 0; c < n; ++c) {
-        const float4 cm = d.CM[P.base + c];
-        sx = __fadd_rn(sx, cm.x);
-        sy = __fadd_rn(sy, cm.y);
-        sz = __fadd_rn(sz, cm.z);
-    }
-    sx = __fdiv_rn(sx, (float)n);
-    sy = __fdiv_rn(sy, (float)n);
-    sz = __fdiv_rn(sz, (float)n);
-    st->syscm[0] = sx;
-    st->syscm[1] = sy;
-    st->syscm[2] = sz;
-    return make_float3(sx, sy, sz);
-}
-
-__device__ __forceinline__ float dist2(float4 cm, float3 o)
-{
-    const float dx = __fsub_rn(cm.x, o.x), dy = __fsub_rn(cm.y, o.y), dz = __fsub_rn(cm.z, o.z);
-    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-}
-
-// getRmax2, src/GPUbounce.cu:2523-2536: the largest squared distance of the
-// first n centres of mass from the recorded system centre.
-__device__ __forceinline__ float rmax2_from(const Dev &d, const InstParams &P, const InstState *st, int n)
-{
-    const float3 o = make_float3(st->syscm[0], st->syscm[1], st->syscm[2]);
-    float r2 = 0.0f;
-    for (int c = 0; c < n; ++c) {
-        const float v = dist2(d.CM[P.base + c], o);
-        r2 = r2 < v ? v : r2;   // std::max
-    }
-    return r2;
-}
-
-// num_cells_far, src/GPUbounce.cu:1288-1290 and :2538-2565, after the
-// divisions of a step (count_only_internal_cells): the newest div_count cells
-// whose centre of mass lies farther than radius_cutoff x the largest distance
-// from the system's centre are not counted as dividing.  The daughters'
-// centres of mass are still 0 here (computed in their first step), as in the
-// reference.  One thread per instance (k).
-__device__ __forceinline__ void far_count(const Dev &d, int k)
-{
-    const InstParams &P = d.prm[k];
-    InstState *st = &d.st[k];
-    if (!(P.far_r > 0.0f) || !(st->step <= P.div_steps && P.growth > 0.0f)) return;
-    const int n = st->n, nd = st->div_count;
-    if (nd == 0 || n < 50) return;
-    const float3 o = sys_centre(d, P, st, n);
-    const float thr = __fmul_rn(__fmul_rn(P.far_r, P.far_r), rmax2_from(d, P, st, n));
-    int far = 0;
-    for (int c = n - nd; c < n; ++c)
-        if (dist2(d.CM[P.base + c], o) > thr) ++far;
-    if (far) {
-        const int q = atomicAdd(d.n_far, 1);
-        if (q < d.far_cap) d.farlog[q] = make_int4(k, st->step, far, 0);
-    }
-}
 
 // Cells softened when growth ends, src/GPUbounce.cu:1340-1429 (duringGrowth
 // off): at the end of step div_time_steps + 2, after the step's grid and
@@ -1754,39 +1759,6 @@ __global__ void __launch_bounds__(SLOTS) k_vol_hist(Dev d, int inst, float lo, f
     }
 }
 
-// G: grid extents of instances that divided this step, from all boxes.
-__device__ __forceinline__ void grid_fix(const Dev &d, int par)
-{
-    const int pn = par ^ 1;
-    const int W = n_work(d);
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < W; w += gridDim.x * blockDim.x) {
-        int a = cell_of(d, w);
-        int inst = inst_of(d, a);
-        if (d.st[inst].div_count == 0) continue;
-        float4 lo = d.aabb[pn][2 * a], hi = d.aabb[pn][2 * a + 1];
-        int *mm = d.st[inst].mm[pn];
-        atomicMin(&mm[0], f2o(lo.x)); atomicMax(&mm[1], f2o(hi.x));
-        atomicMin(&mm[2], f2o(lo.y)); atomicMax(&mm[3], f2o(hi.y));
-        atomicMin(&mm[4], f2o(lo.z)); atomicMax(&mm[5], f2o(hi.z));
-    }
-}
-
-// After the placement of the daughters: the grid extents, with far the
-// internal-cells count, and with fuse the next half kick of the divided cells.
-__device__ __forceinline__ void div_finish(const Dev &d, int par, bool far, bool fuse, float *smax)
-{
-    grid_fix(d, par);
-    if (far && threadIdx.x == 0)
-        for (int k = blockIdx.x; k < d.n_inst; k += gridDim.x) far_count(d, k);
-    if (fuse) integrate_divided(d, smax);
-}
-
-__global__ void __launch_bounds__(SLOTS) k_div_finish(Dev d, int par, int far, int fuse)
-{
-    __shared__ float smax[SLOTS / 32];
-    if (d.flags[1]) div_finish(d, par, far != 0, fuse != 0, smax);
-}
-
 // ---------------------------------------------------------------------------
 // Neighbour-list build (instances whose displacement bound reached the skin,
 // or that divided): every cell's box at the current positions, a table of the
@@ -1802,10 +1774,10 @@ __global__ void __launch_bounds__(SLOTS) k_div_finish(Dev d, int par, int far, i
 // near the cell, the warps test those against a patch of 30 nodes each, and
 // the entries come in their final order (ascending cell, then node).  Bound by
 // the latency of one cell's chain in partial builds (11 us a cell alone on its
-// SM) and by instruction issue in whole ones.  With this form and nb_mark's
-// rule a step of 2500 to 3200 growing cells went from 350 to 237 us (all of it
-// list build), one of 301 from 98 to 69 us; a whole build of 100,000 packed
-// cells takes 1.2 ms against 1.35 with the sort.
+// SM) and by instruction issue in whole ones.  With
+// this form a step of 2500 to 3200 growing cells went from 350 to 237 us (all
+// of it list build), one of 301 from 98 to 69 us; a whole build of 100,000
+// packed cells takes 1.2 ms against 1.35 with the sort.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int bin_coord(float v, float inv)
 {
@@ -1824,55 +1796,6 @@ __device__ __forceinline__ unsigned bin_slot(const InstState &st, int ix, int iy
     h ^= h >> 15;
     h *= 0x9e3779b1u;
     return st.hbase + (h >> (32 - st.hbits));
-}
-
-// B1: boxes at the current positions and the cell table, one warp per cell.
-__device__ __forceinline__ void nb_boxes(const Dev &d)
-{
-    const int W = n_work(d);
-    const int lane = threadIdx.x & 31, nw = SLOTS / 32;
-    const unsigned epoch = *d.epoch;
-    for (int w = blockIdx.x * nw + (threadIdx.x >> 5); w < W; w += gridDim.x * nw) {
-        const int a = cell_of(d, w);
-        const int inst = inst_of(d, a);
-        InstState *st = &d.st[inst];
-        if (!st->rebuild) continue;
-        const float4 *X = d.X + (size_t)a * SLOTS;
-        float lx = 1e30f, ly = 1e30f, lz = 1e30f, hx = -1e30f, hy = -1e30f, hz = -1e30f;
-#pragma unroll
-        for (int k = 0; k < (NODES + 31) / 32; ++k) {
-            const int i = lane + 32 * k;
-            if (i < NODES) {
-                const float4 x = X[i];
-                lx = fminf(lx, x.x); hx = fmaxf(hx, x.x);
-                ly = fminf(ly, x.y); hy = fmaxf(hy, x.y);
-                lz = fminf(lz, x.z); hz = fmaxf(hz, x.z);
-            }
-        }
-        lx = warp_min(lx); ly = warp_min(ly); lz = warp_min(lz);
-        hx = warp_max(hx); hy = warp_max(hy); hz = warp_max(hz);
-        if (lane == 0) {
-            d.nbox[2 * a] = make_float4(lx, ly, lz, 0.f);
-            d.nbox[2 * a + 1] = make_float4(hx, hy, hz, 0.f);
-            if (lx <= hx) {   // some node is a number
-                // a look first: most cells are smaller than one already in
-                const float hq[3] = {0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz)};
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-                    if (__float_as_uint(hq[q]) > __ldcg(&st->hmax[q])) atomicMax(&st->hmax[q], __float_as_uint(hq[q]));
-                const float inv = d.prm[inst].inv_bin;
-                const unsigned b = bin_slot(*st, box_bin(lx, hx, inv), box_bin(ly, hy, inv), box_bin(lz, hz, inv));
-                const unsigned long long old =
-                    atomicExch(&d.bins[b], ((unsigned long long)epoch << 32) | (unsigned)a);
-                d.bnext[a] = (unsigned)(old >> 32) == epoch ? (int)(unsigned)old : -1;
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(SLOTS) k_nb_boxes(Dev d)
-{
-    if (d.flags[0]) nb_boxes(d);
 }
 
 // Gap of two intervals (negative: they overlap).
@@ -1895,47 +1818,116 @@ __device__ __forceinline__ float list_radius(const InstParams &P, bool full, flo
 }
 constexpr float BOX_REACH = 1.0001f;
 
-// B2: the cells to build into d.build, one thread per cell: all cells of whole
-// builds, and those that partial builds concern (the divided ones and those
-// whose boxes come within the list radius of one).
-__device__ __forceinline__ void nb_mark(const Dev &d)
+// B1: boxes at the current positions and the cell table, one warp per cell;
+// and the cells to build into d.build: all cells of whole builds, and those
+// that partial builds concern (the divided ones and those whose boxes come
+// within the list radius of one).  The divided cells' own boxes are not needed
+// for that: they lie within those of their placement (aabb[par], of the step
+// before) and the kick since, which is their distance from their anchors.
+__device__ __forceinline__ void nb_boxes(const Dev &d, int par)
 {
     const int W = n_work(d), T = *d.div_prev;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < W; w += gridDim.x * blockDim.x) {
-        const int a = cell_of(d, w);
+    const int lane = threadIdx.x & 31, nw = SLOTS / 32;
+    const unsigned epoch = *d.epoch;
+    float half[3] = {0.f, 0.f, 0.f};   // largest half extents of this warp's cells (one instance)
+    // the cells of a CTA's warps are listed with one atomic
+    __shared__ int listed[SLOTS / 32];
+    for (int w0 = blockIdx.x * nw; w0 < W; w0 += gridDim.x * nw) {
+        const int w = w0 + (threadIdx.x >> 5);
+        const int a = w < W ? cell_of(d, w) : 0;
         const int inst = inst_of(d, a);
         InstState *st = &d.st[inst];
-        const int rb = st->rebuild;
-        if (rb != 1) {
-            if (rb == 2) d.build[atomicAdd(d.n_build, 1)] = a;
-            d.mark[a] = 0;
-            continue;
-        }
-        const InstParams &P = d.prm[inst];
-        const float4 lo = d.nbox[2 * a], hi = d.nbox[2 * a + 1];
-        const float da = d.cdisp[a];
-        int m = 0;
-        for (int q = 0; q < T; ++q) {
-            const DivEntry &e = d.divtab[q];
-            if (e.inst != inst) continue;
-            const int cs[2] = {e.parent, e.daughter};
+        const int rb = w < W ? st->rebuild : 0;
+        if (lane == 0) listed[threadIdx.x >> 5] = -1;
+        if (rb) {
+            const InstParams &P = d.prm[inst];
+            const float4 *X = d.X + (size_t)a * SLOTS;
+            float lx = 1e30f, ly = 1e30f, lz = 1e30f, hx = -1e30f, hy = -1e30f, hz = -1e30f;
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int c = cs[k];
-                if (a == c) m |= 2;
-                else if (boxes_near(lo, hi, d.nbox[2 * c], d.nbox[2 * c + 1],
-                                    list_radius(P, false, da, d.cdisp[c]) * BOX_REACH))
-                    m |= 1;
+            for (int k = 0; k < (NODES + 31) / 32; ++k) {
+                const int i = lane + 32 * k;
+                if (i < NODES) {
+                    const float4 x = X[i];
+                    lx = fminf(lx, x.x); hx = fmaxf(hx, x.x);
+                    ly = fminf(ly, x.y); hy = fmaxf(hy, x.y);
+                    lz = fminf(lz, x.z); hz = fmaxf(hz, x.z);
+                }
+            }
+            lx = warp_min(lx); ly = warp_min(ly); lz = warp_min(lz);
+            hx = warp_max(hx); hy = warp_max(hy); hz = warp_max(hz);
+            const float4 lo = make_float4(lx, ly, lz, 0.f), hi = make_float4(hx, hy, hz, 0.f);
+            int m = 0;
+            if (rb == 1) {
+                const float da = d.cdisp[a];
+                for (int q = lane; q < T; q += 32) {
+                    const DivEntry &e = d.divtab[q];
+                    if (e.inst != inst) continue;
+                    const int cs[2] = {e.parent, e.daughter};
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const int c = cs[k];
+                        float r = d.cdisp[c];
+                        r += list_radius(P, false, da, r);
+                        float4 pl = d.aabb[par][2 * c], ph = d.aabb[par][2 * c + 1];
+                        if (P.correct_com) {   // the correction moved the nodes, not the boxes
+                            const float *o = st->syscm;
+                            pl = make_float4(pl.x - o[0], pl.y - o[1], pl.z - o[2], 0.f);
+                            ph = make_float4(ph.x - o[0], ph.y - o[1], ph.z - o[2], 0.f);
+                            r += 1e-3f;
+                        }
+                        if (a == c) m |= 2;
+                        else if (boxes_near(lo, hi, pl, ph, r * BOX_REACH)) m |= 1;
+                    }
+                }
+                m = __reduce_or_sync(0xffffffffu, m);
+            }
+            if (lane == 0) {
+                d.nbox[2 * a] = lo;
+                d.nbox[2 * a + 1] = hi;
+                d.mark[a] = (uint8_t)m;
+                if (rb == 2 || m) listed[threadIdx.x >> 5] = a;
+                if (lx <= hx) {   // some node is a number
+                    const float hq[3] = {0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz)};
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        if (d.single) half[q] = fmaxf(half[q], hq[q]);
+                        // a look first: most cells are smaller than one already in
+                        else if (__float_as_uint(hq[q]) > __ldcg(&st->hmax[q])) atomicMax(&st->hmax[q], __float_as_uint(hq[q]));
+                    }
+                    const float inv = P.inv_bin;
+                    const unsigned b = bin_slot(*st, box_bin(lx, hx, inv), box_bin(ly, hy, inv), box_bin(lz, hz, inv));
+                    const unsigned long long old =
+                        atomicExch(&d.bins[b], ((unsigned long long)epoch << 32) | (unsigned)a);
+                    d.bnext[a] = (unsigned)(old >> 32) == epoch ? (int)(unsigned)old : -1;
+                }
             }
         }
-        d.mark[a] = (uint8_t)m;
-        if (m) d.build[atomicAdd(d.n_build, 1)] = a;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int c = lane < nw ? listed[lane] : -1;
+            const unsigned b = __ballot_sync(0xffffffffu, c >= 0);
+            int at = 0;
+            if (lane == 0 && b) at = atomicAdd(d.n_build, __popc(b));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (c >= 0) d.build[at + __popc(b & ((1u << lane) - 1u))] = c;
+        }
+        __syncthreads();
+    }
+    if (d.single) {
+        // one atomic for a CTA: one for each cell of the only instance took 8 us at 3000 cells
+        __shared__ unsigned most[3];
+        if (threadIdx.x < 3) most[threadIdx.x] = 0u;
+        __syncthreads();
+        if (lane == 0)
+            for (int q = 0; q < 3; ++q) atomicMax(&most[q], __float_as_uint(half[q]));
+        __syncthreads();
+        if (threadIdx.x < 3 && most[threadIdx.x]) atomicMax(&d.st[0].hmax[threadIdx.x], most[threadIdx.x]);
     }
 }
 
-__global__ void __launch_bounds__(SLOTS) k_nb_mark(Dev d)
+__global__ void __launch_bounds__(SLOTS) k_nb_boxes(Dev d, int par)
 {
-    if (d.flags[0]) nb_mark(d);
+    if (d.flags[0]) nb_boxes(d, par);
 }
 
 constexpr int NBW = SLOTS / 32;   // warps of a CTA, and cells whose nodes are staged together
@@ -2153,7 +2145,7 @@ __device__ __forceinline__ void list_stats(const Dev &d, ListSmem &sm)
     if (d.halo_stats) atomicMax(&st->max_halo, sm.max_halo);
 }
 
-// B3: the lists of cell a, with the radius of whole builds (full) or with the
+// B2: the lists of cell a, with the radius of whole builds (full) or with the
 // cells' displacements.  The whole CTA; its warps take a patch of 30
 // neighbouring nodes each.  False, without full only, if some node has more
 // entries than it has room for.
@@ -2413,9 +2405,7 @@ __global__ void __launch_bounds__(SLOTS, 4) k_steps(Dev d, int par, int n, int n
         const int fuse = com ? 0 : end && last ? 2 : 1;
         const auto next = [&] { if (!end) step_begin<SLOTS>(d, par); };
         if (d.flags[0]) {
-            nb_boxes(d);
-            if (!grid_sync(d, bar)) return;
-            nb_mark(d);
+            nb_boxes(d, par);
             if (!grid_sync(d, bar)) return;
             nb_lists(d, sm.lists);
             if (!grid_sync(d, bar)) return;
@@ -2435,11 +2425,9 @@ __global__ void __launch_bounds__(SLOTS, 4) k_steps(Dev d, int par, int n, int n
             }))
             return;
         if (div && d.flags[1]) {
-            for (int q = blockIdx.x; q < d.n_inst; q += gridDim.x) div_select<SLOTS>(d, par, q, sm.div);
+            for (int q = blockIdx.x; q < d.n_inst; q += gridDim.x) div_select<SLOTS>(d, par, q, far != 0, sm.div);
             if (!grid_sync(d, bar)) return;
-            div_apply(d, par, sm.s2.xs, sm.s2.gs);
-            if (!grid_sync(d, bar)) return;
-            div_finish(d, par, far != 0, fuse != 0, sm.s2.smax);
+            div_apply(d, par, fuse != 0, sm.s2.xs, sm.s2.gs, sm.s2.smax);
             if (!grid_sync(d, bar, [&] {
                     if (com) centres();
                     else next();

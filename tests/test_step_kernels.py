@@ -176,13 +176,15 @@ def test_forces_of_bent_and_crowded_cells(mesh, make, arg):
     sim.close()
 
 
-@pytest.mark.parametrize("skin", [0.25, 0.35])
-def test_crowded_partial_builds_fall_back(mesh, skin):
+@pytest.mark.parametrize("skin,over", [(0.25, {}), (0.35, {}), (0.2, {"correct_com": 1})])
+def test_partial_builds_do_not_change_results(mesh, skin, over):
     """A growing colony with a wide list skin against the default one, bit for
     bit.  At 0.35 the radius of a partial build around a division gives some
     node more entries than it has room for (a whole build stays below): the
-    cell takes the smaller radius and the instance is rebuilt in the next step."""
-    p, st = _growing(64)
+    cell takes the smaller radius and the instance is rebuilt in the next step.
+    With the centre-of-mass correction the boxes that a division's neighbours are
+    found by lie apart from the nodes."""
+    p, st = _growing(64, **over)
     topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
     got = []
     for s in (0.1, skin):
