@@ -220,9 +220,9 @@ __device__ __forceinline__ void sincos_small(double x, double &s, double &c)
 }
 
 // One arm of a vertex: the exact FP64 difference p of two node positions,
-// its squared length, length and inverse squared length (from one rsqrt).
+// its squared length, length, and inverse length and its square (from one rsqrt).
 struct Arm {
-    double x, y, z, r2, len, ir2;
+    double x, y, z, r2, len, ir2, ir;
 };
 
 __device__ __forceinline__ Arm make_arm(const double3 &to, const double3 &from)
@@ -235,6 +235,7 @@ __device__ __forceinline__ Arm make_arm(const double3 &to, const double3 &from)
     const double r = rsqrt_nr(a.r2);
     a.len = a.r2 * r;
     a.ir2 = r * r;
+    a.ir = r;
     return a;
 }
 
@@ -953,47 +954,24 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         if (wn < W) prefetch_cell(d, cell_of(d, wn));
         const float3 x = f3(x4);
         const float3 v = f3(v4);
-        // bond angles: thread = vertex, three angles each
-        if (P.angles && i < NODES) {
-            const double3 xi = sm.xd[i];
-            const Arm pa = make_arm(sm.xd[n0], xi), pb = make_arm(sm.xd[n1], xi), pc = make_arm(sm.xd[n2], xi);
-            const double2 *cs0 = d.topo.cs0 + 3 * i;
-            const float4 th = __ldg(&d.topo.th0[i]);
-            // angles (n0, n1), (n1, n2), (n0, n2); arm ends summed by destination
-            double3 F01p, F01q, F12p, F12q, F02p, F02q;
-            double2 t0 = __ldg(&cs0[0]);
-            angle_term(pa, pb, th.x, t0.x, t0.y, F01p, F01q);
-            t0 = __ldg(&cs0[1]);
-            angle_term(pb, pc, th.y, t0.x, t0.y, F12p, F12q);
-            t0 = __ldg(&cs0[2]);
-            angle_term(pa, pc, th.z, t0.x, t0.y, F02p, F02q);
-            const int o = i * 3;
-            sm.arm.x[o] = F01p.x + F02p.x; sm.arm.y[o] = F01p.y + F02p.y; sm.arm.z[o] = F01p.z + F02p.z;
-            sm.arm.x[o + 1] = F01q.x + F12p.x; sm.arm.y[o + 1] = F01q.y + F12p.y; sm.arm.z[o + 1] = F01q.z + F12p.z;
-            sm.arm.x[o + 2] = F12q.x + F02q.x; sm.arm.y[o + 2] = F12q.y + F02q.y; sm.arm.z[o + 2] = F12q.z + F02q.z;
-        }
-        __syncthreads();
         // The node force is accumulated in FP64: its terms (pressure up
         // to ~1e3, stiff contact repulsion up to ~1e4) can cancel to a
         // net force orders of magnitude smaller, and the sum is rounded to
         // float once, as the reference stores it.
         double FX = 0.0, FY = 0.0, FZ = 0.0;
         if (i < NODES) {
-            if (isnan(x.x) || isnan(x.y) || isnan(x.z)) atomic_or_err(&d.st[inst], CS3D_ERRBIT_NAN);
-            // springs, src/propagate.cu:298-314:
+            const double3 xi = sm.xd[i];
+            const Arm pa = make_arm(sm.xd[n0], xi), pb = make_arm(sm.xd[n1], xi), pc = make_arm(sm.xd[n2], xi);
+            // springs, src/propagate.cu:298-314, along the angles' arms:
             // k (R - R0) / R0 * d / R = k (1/R0 - 1/R) d
             const double stiff = d.E[a];
-            const int nbr[3] = {n0, n1, n2};
-            const double3 xi = sm.xd[i];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                // exact FP64 differences of the float positions
-                const double3 xn = sm.xd[nbr[k]];
-                const double ex = xn.x - xi.x, ey = xn.y - xi.y, ez = xn.z - xi.z;
-                const double iR = rsqrt_nr(ex * ex + ey * ey + ez * ez);
-                const double c = stiff * (__ldg(&d.topo.r0i[3 * i + k]) - iR);
-                FX += c * ex; FY += c * ey; FZ += c * ez;
-            }
+            const auto spring = [&](const Arm &p, int k) {
+                const double c = stiff * (__ldg(&d.topo.r0i[3 * i + k]) - p.ir);
+                FX += c * p.x; FY += c * p.y; FZ += c * p.z;
+            };
+            spring(pa, 0);
+            spring(pb, 1);
+            spring(pc, 2);
             // internal pressure, src/propagate.cu:318-330 (CM of the previous step)
             {
                 const float4 cm = d.CM[a];
@@ -1001,6 +979,27 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
                 const double c = 3.0 * (double)sm.press * rsqrt_nr(rx * rx + ry * ry + rz * rz);
                 FX += c * rx; FY += c * ry; FZ += c * rz;
             }
+            // bond angles: thread = vertex, three angles each
+            if (P.angles) {
+                const double2 *cs0 = d.topo.cs0 + 3 * i;
+                const float4 th = __ldg(&d.topo.th0[i]);
+                // angles (n0, n1), (n1, n2), (n0, n2); arm ends summed by destination
+                double3 F01p, F01q, F12p, F12q, F02p, F02q;
+                double2 t0 = __ldg(&cs0[0]);
+                angle_term(pa, pb, th.x, t0.x, t0.y, F01p, F01q);
+                t0 = __ldg(&cs0[1]);
+                angle_term(pb, pc, th.y, t0.x, t0.y, F12p, F12q);
+                t0 = __ldg(&cs0[2]);
+                angle_term(pa, pc, th.z, t0.x, t0.y, F02p, F02q);
+                const int o = i * 3;
+                sm.arm.x[o] = F01p.x + F02p.x; sm.arm.y[o] = F01p.y + F02p.y; sm.arm.z[o] = F01p.z + F02p.z;
+                sm.arm.x[o + 1] = F01q.x + F12p.x; sm.arm.y[o + 1] = F01q.y + F12p.y; sm.arm.z[o + 1] = F01q.z + F12p.z;
+                sm.arm.x[o + 2] = F12q.x + F02q.x; sm.arm.y[o + 2] = F12q.y + F02q.y; sm.arm.z[o + 2] = F12q.z + F02q.z;
+            }
+        }
+        __syncthreads();
+        if (i < NODES) {
+            if (isnan(x.x) || isnan(x.y) || isnan(x.z)) atomic_or_err(&d.st[inst], CS3D_ERRBIT_NAN);
             // bond angles, src/propagate.cu:81-181: the vertex terms (minus
             // the arm forces of the angles at i) and the arm terms (the arm
             // forces that the angles at the three neighbours send to i)
