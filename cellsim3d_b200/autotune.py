@@ -1,7 +1,7 @@
 """Neighbour-list skin autotuner by population range.
 
-The list skin (the margin of the list radius over the attraction range, and
-with it the edge of the node-hash bins) trades the length of the contact
+The list skin (the margin of the list radius over the attraction range)
+trades the length of the contact
 lists that every step sweeps against the frequency of list rebuilds.  The
 best value depends on how fast the nodes move and how densely the cells
 pack, and both change as a colony grows.  The skin changes no result: the

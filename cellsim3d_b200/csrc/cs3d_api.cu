@@ -484,7 +484,9 @@ bool in_one_kernel(const cs3d_ctx *c) { return c->grid_steps > 0 && c->n_now <= 
 constexpr int STEPS_PER_LAUNCH = 256;
 
 // n steps from step s on in one cooperative launch; the state is kicked.
-int launch_steps(cs3d_ctx *c, long long s, int n, bool last)
+// Where the device has no room for all CTAs at once (a share of it, under MPS),
+// the context goes back to the launch sequence: *fits is false.
+int launch_steps(cs3d_ctx *c, long long s, int n, bool last, bool *fits)
 {
     Dev d = c->d;
     int par = (int)((s - 1) & 1);
@@ -494,7 +496,15 @@ int launch_steps(cs3d_ctx *c, long long s, int n, bool last)
     // as many CTAs as the cells may become: one without a cell only waits
     const int grid = std::min(c->grid_steps, c->cap_total);
     void *args[] = {&d, &par, &n, &n_div, &is_last, &com, &far};
-    CK(cudaLaunchCooperativeKernel((const void *)k_steps, dim3(grid), dim3(SLOTS), args, sizeof(StepsSmem), c->stream));
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel((const void *)k_steps, dim3(grid), dim3(SLOTS), args, sizeof(StepsSmem), c->stream);
+    *fits = e != cudaErrorCooperativeLaunchTooLarge;
+    if (!*fits) {
+        cudaGetLastError();
+        c->grid_steps = 0;
+        return CS3D_OK;
+    }
+    CK(e);
     c->launches_per_step = 1;
     return CS3D_OK;
 }
@@ -962,8 +972,11 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
             if (k1) {
                 k_integrate<<<c->grid_s2, SLOTS, 0, c->stream>>>(c->d);
                 CK(cudaGetLastError());
+                k1 = false;
             }
-            if ((rc = launch_steps(c, s, m, last))) return rc;
+            bool fits = true;
+            if ((rc = launch_steps(c, s, m, last, &fits))) return rc;
+            if (!fits) { --k; continue; }   // the same step again, by the sequence
             c->host_step = s + m - 1;
             k1 = c->any_com;
             c->prekicked = last && !c->any_com;

@@ -97,7 +97,8 @@ __device__ __forceinline__ int inst_of(const Dev &d, int a) { return d.single ? 
 // Cells of a phase dealt out to the CTAs one by one: a CTA begins with the
 // cell of its index and draws the next one while it works.  A cell next to a
 // division takes three times as long as another, so that with a fixed stride
-// the last CTA of S1 ended 60 % after the mean one (2500 growing cells).
+// the last CTA of S1 ended 60 % after the mean one (2500 growing cells); S1
+// takes the newest cells first, a further 2 % of the step.
 // next[]: two words of the CTA's shared memory; the counter is zero at the
 // start of the phase (step_begin).
 struct Dealer {
@@ -925,7 +926,8 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
     const float sgn = (float)(int8_t)(nnp >> 24);
     Dealer deal(&d.deal[DEAL_S1], sm.next);
     while (deal.w < W) {
-        const int a = cell_of(d, deal.w);
+        // the newest cells first: fresh daughters take longest
+        const int a = cell_of(d, W - 1 - deal.w);
         deal.draw();
         const int inst = inst_of(d, a);
         const InstParams &P = d.prm[inst];
@@ -951,7 +953,7 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         __syncthreads();
         slots_boxes(d, P, par, sm.sd, nc);
         const int wn = sm.next[deal.turn];
-        if (wn < W) prefetch_cell(d, cell_of(d, wn));
+        if (wn < W) prefetch_cell(d, cell_of(d, W - 1 - wn));
         const float3 x = f3(x4);
         const float3 v = f3(v4);
         // The node force is accumulated in FP64: its terms (pressure up

@@ -48,7 +48,7 @@ extern "C" {
 #define CS3D_ERRBIT_ENTRY_OVERFLOW 0x008u  /* > CS3D_MAX_ENTRIES contact nodes or > CS3D_MAX_DIS pairs for one node */
 #define CS3D_ERRBIT_NONFINITE_VOL  0x010u  /* src/volume.cu:134-139 */
 #define CS3D_ERRBIT_BAD_NORMAL     0x020u  /* |n| != 1, src/postscriptinit.cu:215-219 */
-#define CS3D_ERRBIT_GRID_OVERFLOW  0x040u  /* reserved, never raised (the node hash cannot overflow) */
+#define CS3D_ERRBIT_GRID_OVERFLOW  0x040u  /* reserved, never raised (the cell table cannot overflow) */
 #define CS3D_ERRBIT_PAIR_OVERFLOW  0x080u  /* pair-recording buffer full */
 #define CS3D_ERRBIT_HALO_OVERFLOW  0x100u  /* reserved, never raised */
 #define CS3D_ERRBIT_SOFT_CELLS     0x200u  /* more distinct softer cells requested than cell indices
@@ -314,9 +314,9 @@ int cs3d_get_state(cs3d_ctx *ctx, int inst, int *n_cells, float *X, float *Y, fl
 /* Start reading instance inst back without waiting for it, so that the next
  * cs3d_step overlaps the device-to-host copy (the reference reads each frame
  * back on its step loop's thread and the GPU idles meanwhile,
- * src/GPUbounce.cu:1443-1475, WriteBinaryTraj :2446-2477).  The cell count is
- * read first (a short synchronous read) and stored in *n_cells; the arrays
- * are then gathered on the context's stream into one of two device staging
+ * src/GPUbounce.cu:1443-1475, WriteBinaryTraj :2446-2477).  The cell count
+ * (known on the host since the last step) is stored in *n_cells; the arrays
+ * are gathered on the context's stream into one of two device staging
  * slots (slot 0 or 1) and copied to the caller's buffers on a separate copy
  * stream, one cudaMemcpyAsync per array.  Output pointers may be NULL; they
  * should be page-locked (cs3d_host_alloc) for the copy to be asynchronous.
@@ -408,9 +408,8 @@ int cs3d_last_error(cs3d_ctx *ctx, int inst, uint32_t *bits);
  * [5] max distinct contact-candidate nodes (of other cells) per cell seen
  * (counted only with CS3D_OPT_HALO_STATS, else 0),
  * [6] cell neighbour lists built (cumulative), [7] of the rebuilds [1], those
- * that only the rule for dividing instances called for (a division in the
- * step and a node more than a quarter of the skin from its anchor, with no
- * node past half the skin). */
+ * that only the rule for dividing instances called for (more than one cell in
+ * 16 divided in the step, with no other cause). */
 int cs3d_get_stats(cs3d_ctx *ctx, long long *stats, int n);
 
 /* Profiling pass: n_steps steps launched kernel by kernel (not as a graph)
