@@ -502,14 +502,12 @@ __device__ __forceinline__ double3 sweep_s2(const Dev &d, const int *cell, int a
 // x_N1)).  The projection is linear in v_ij, so the sweeps sum the velocity
 // differences alone (S) and this applies it once: S - (S . n) n.  The normal
 // is formed in FP64 from exact differences of the float positions.
-__device__ __forceinline__ double3 as_d3(const double3 &a) { return a; }
 __device__ __forceinline__ double3 as_d3(const float4 &a) { return make_double3(a.x, a.y, a.z); }
 
-// xd: the cell's positions (FP64 copies, or the float4 originals).
-template <typename T>
-__device__ __forceinline__ double3 tangential(const T *xd, int n0, int n1, int n2, float sgn, double3 S)
+// xs: the cell's positions.
+__device__ __forceinline__ double3 tangential(const float4 *xs, int n0, int n1, int n2, float sgn, double3 S)
 {
-    const double3 p0 = as_d3(xd[n0]), p1 = as_d3(xd[n1]), p2 = as_d3(xd[n2]);
+    const double3 p0 = as_d3(xs[n0]), p1 = as_d3(xs[n1]), p2 = as_d3(xs[n2]);
     const double ax = p1.x - p0.x, ay = p1.y - p0.y, az = p1.z - p0.z;
     const double bx = p2.x - p0.x, by = p2.y - p0.y, bz = p2.z - p0.z;
     const double cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
@@ -521,18 +519,17 @@ __device__ __forceinline__ double3 tangential(const T *xd, int n0, int n1, int n
 
 // Dissipative force, src/propagate.cu:546-658: bond damping with the three
 // neighbours, tangential friction sum vt, viscous drag, on the cell's
-// velocities (vd: FP64 copies or the float4 originals).  FP64: the damping
+// velocities vs.  FP64: the damping
 // term is a sum of velocity differences that can cancel.
-template <typename T>
-__device__ __forceinline__ float3 dis_force(const InstParams &P, const T *vd, int i, int n0, int n1, int n2,
+__device__ __forceinline__ float3 dis_force(const InstParams &P, const float4 *vs, int i, int n0, int n1, int n2,
                                            double3 vt)
 {
-    const double3 v = as_d3(vd[i]);
+    const double3 v = as_d3(vs[i]);
     double dx = 0.0, dy = 0.0, dz = 0.0;
     const int nbr[3] = {n0, n1, n2};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double3 vn = as_d3(vd[nbr[k]]);
+        const double3 vn = as_d3(vs[nbr[k]]);
         dx += v.x - vn.x; dy += v.y - vn.y; dz += v.z - vn.z;
     }
     const double gi = P.gint, ge = P.gext, go = P.go;
@@ -905,8 +902,11 @@ __device__ __forceinline__ void prefetch_cell(const Dev &d, int a)
 }
 
 struct S1Smem {
-    double3 xd[SLOTS];   // FP64 copies of the positions and velocities: the
-    double3 vd[SLOTS];   // FP64 terms read them without conversions
+    // The cell's positions and velocities as floats, converted where they are
+    // read: with FP64 copies the gathers of the neighbours kept the L1 pipe 70 %
+    // busy, with floats the conversions share the XU pipe's 32 % (S1 of 100,000
+    // packed cells 1.66 -> 1.61 ms; with positions in both forms 1.69).
+    float4 xs[SLOTS], vs[SLOTS];
     SlotData sd;
     union {                         // the angles' arms are read before the sweep begins: the
         SweepSmem sweep[SLOTS / 32];  // room is worth more as L1 (S1 of 100,000 packed
@@ -941,8 +941,8 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         for (int q = 0; q < EPRE / 2; ++q)
             pre[q] = (uint32_t)d.ent[((size_t)a * MAXE + 2 * q) * SLOTS + i] |
                      ((uint32_t)d.ent[((size_t)a * MAXE + 2 * q + 1) * SLOTS + i] << 16);
-        sm.xd[i] = make_double3(x4.x, x4.y, x4.z);
-        sm.vd[i] = make_double3(v4.x, v4.y, v4.z);
+        sm.xs[i] = x4;
+        sm.vs[i] = v4;
         slots_load(d, a, &d.st[inst], par, sm.sd);
         if (i == 128) {
             // this step's PressureUpdate (none before the initial forces)
@@ -962,8 +962,9 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         // float once, as the reference stores it.
         double FX = 0.0, FY = 0.0, FZ = 0.0;
         if (i < NODES) {
-            const double3 xi = sm.xd[i];
-            const Arm pa = make_arm(sm.xd[n0], xi), pb = make_arm(sm.xd[n1], xi), pc = make_arm(sm.xd[n2], xi);
+            const double3 xi = as_d3(x4);
+            const Arm pa = make_arm(as_d3(sm.xs[n0]), xi), pb = make_arm(as_d3(sm.xs[n1]), xi),
+                      pc = make_arm(as_d3(sm.xs[n2]), xi);
             // springs, src/propagate.cu:298-314, along the angles' arms:
             // k (R - R0) / R0 * d / R = k (1/R0 - 1/R) d
             const double stiff = d.E[a];
@@ -1018,7 +1019,7 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
         double3 vsum = make_double3(0.0, 0.0, 0.0);
         const int nd = sweep_s1<COOP>(d, P, sm.sd, sm.sweep[i >> 5], a, i, x, v, ne, pre, FX, FY, FZ, vsum);
         if (i < NODES) {
-            const double3 vt = tangential(sm.xd, n0, n1, n2, sgn, vsum);
+            const double3 vt = tangential(sm.xs, n0, n1, n2, sgn, vsum);
             if (nd > MAXD) atomic_or_err(&d.st[inst], CS3D_ERRBIT_ENTRY_OVERFLOW);
             // rigid box walls, src/propagate.cu:474-510 (float gap tests)
             if (P.rigid) {
@@ -1033,7 +1034,7 @@ __device__ __forceinline__ void s1_cells(const Dev &d, int par, S1Smem &sm)
                 if (g1 < P.thresh) FZ += -wk * ((double)g1 - th);
                 if (g2 < P.thresh) FZ += wk * ((double)g2 - th);
             }
-            const float3 fd = dis_force(P, sm.vd, i, n0, n1, n2, vt);
+            const float3 fd = dis_force(P, sm.vs, i, n0, n1, n2, vt);
             d.FC[g] = make_float4((float)FX, (float)FY, (float)FZ, 0.f);
             d.ndis[g] = (uint8_t)(nd < MAXD ? nd : MAXD);
             if (INIT) {
