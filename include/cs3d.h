@@ -404,7 +404,8 @@ int cs3d_last_error(cs3d_ctx *ctx, int inst, uint32_t *bits);
 
 /* Counters of this library's neighbour lists (no counterpart in the
  * reference): [0] steps, [1] neighbour-list rebuilds, [2] max entries per node
- * seen, [3] max candidate cells per cell seen, [4] kernel launches per step,
+ * seen, [3] max candidate cells per cell seen, [4] kernel launches per step
+ * (1 where the steps share one launch),
  * [5] max distinct contact-candidate nodes (of other cells) per cell seen
  * (counted only with CS3D_OPT_HALO_STATS, else 0),
  * [6] cell neighbour lists built (cumulative), [7] of the rebuilds [1], those
