@@ -41,7 +41,6 @@ struct cs3d_ctx {
     std::vector<long long> soften_steps;  // steps whose end softens cells (stiffness schedule)
     float skin = 0.1f;
     int grid_cells = 0;            // blocks of the per-cell kernels
-    int grid_flat = 0;             // blocks of the per-thread kernels
     int grid_lists = 0;            // blocks of the neighbour lists
     int grid_boxes = 0;            // blocks of the cell boxes (a warp per cell)
     int grid_s2 = 0;               // blocks of S2 and the integrator
@@ -759,7 +758,6 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_s1<false>, SLOTS, sizeof(S1Smem));
     c->grid_cells = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ, 1)));
-    c->grid_flat = std::max(1, std::min((c->cap_total + 255) / 256 + 1, c->nsm * 8));
     int occ_nl = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_nl, k_nb_lists, SLOTS, 0);
     c->grid_lists = std::max(1, std::min(c->cap_total, c->nsm * std::max(occ_nl, 1)));
