@@ -1882,8 +1882,10 @@ __device__ __forceinline__ void nb_boxes(const Dev &d, int par)
                 d.nbox[2 * a + 1] = hi;
                 d.mark[a] = (uint8_t)m;
                 if (rb == 2 || m) listed[threadIdx.x >> 5] = a;
-                if (lx <= hx) {   // some node is a number
-                    const float hq[3] = {0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz)};
+                if (lx <= hx && ly <= hy && lz <= hz) {   // some node is a number, along each axis
+                    // 0 for a cell at infinity (a NaN here would be the largest of all)
+                    const float hq[3] = {fmaxf(0.5f * (hx - lx), 0.0f), fmaxf(0.5f * (hy - ly), 0.0f),
+                                         fmaxf(0.5f * (hz - lz), 0.0f)};
 #pragma unroll
                     for (int q = 0; q < 3; ++q) {
                         if (d.single) half[q] = fmaxf(half[q], hq[q]);
@@ -2094,6 +2096,10 @@ __device__ __forceinline__ void cells_in_reach(const Dev &d, const InstParams &P
     const int x0 = bin_coord(lo.x - ex, inv), y0 = bin_coord(lo.y - ey, inv), z0 = bin_coord(lo.z - ez, inv);
     const long long nx = bin_coord(hi.x + ex, inv) - x0 + 1ll, ny = bin_coord(hi.y + ey, inv) - y0 + 1ll,
                     nz = bin_coord(hi.z + ez, inv) - z0 + 1ll;
+    // A cell whose nodes are all NaN along an axis has no box (lo 1e30, hi
+    // -1e30) and reaches nothing: the bins of its ranges come out negative,
+    // and their product wraps to some 1e9.
+    if (nx <= 0 || ny <= 0 || nz <= 0) return;
     if (nx > 64 || ny > 64 || nz > 64 || nx * ny * nz > 4096) {   // some cell is far larger than the mesh at rest
         if (t == 0) sm.n = MAXB + 1;
         return;

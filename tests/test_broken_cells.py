@@ -1,0 +1,71 @@
+"""A cell that is broken (NaN or infinite nodes) raises its error and leaves the
+cells that do not touch it as they are without it."""
+import numpy as np
+import pytest
+
+import cellsim3d_b200 as cs
+from cellsim3d_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+NAN = 0x001
+
+
+def _cells(mesh, k=3, spacing=2.15):
+    """k^3 cells in contact, [n, 192, 3] float32, and their box."""
+    xyz = W.centred(W.scaled_xyz(mesh))
+    c = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3) * spacing + 2.0
+    x = np.zeros((len(c), 192, 3), np.float32)
+    x[:, :180] = xyz[None] + c[:, None].astype(np.float32)
+    return x, float(k * spacing + 4.0)
+
+
+def _run(mesh, x, box, steps=2, beside=None, **over):
+    """Initial forces, then forces, state and cell data after some steps, and
+    the error bits; beside: the cells of a second instance."""
+    p = W.base_params(box_len=(box, box, box), growth_rate=0.0)
+    p.update(over)
+    rest = np.zeros((192, 3), np.float32)
+    rest[:180] = W.centred(W.scaled_xyz(mesh))
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), *[np.ascontiguousarray(rest[:, q]) for q in range(3)])
+    xs = [x] if beside is None else [x, beside]
+    sim = cs.Ensemble([p] * len(xs), topo, [len(y) for y in xs])
+    for k, y in enumerate(xs):
+        sim.load_state(k, *[np.ascontiguousarray(y[..., q].reshape(-1)) for q in range(3)], n_cells=len(y))
+    out = [sim.forces()]
+    sim.step(steps, raise_on_error=False)
+    out += [sim.forces(), sim.state(), sim.cells()]
+    err = sim.last_error()
+    sim.close()
+    return out, err
+
+
+def _same(a, b, n, keep):
+    """The per-node and per-cell arrays of the n cells `keep` picks from a, against all of b's."""
+    for x, y in zip(a, b):
+        for k in x:
+            if k == "n":
+                continue
+            u = np.asarray(x[k]).reshape(n, -1)[keep]
+            v = np.asarray(y[k]).reshape(len(u), -1)
+            assert np.array_equal(u, v), k
+
+
+@pytest.mark.parametrize("axes", [(0, 1, 2), (0,), (1,), (2,), (0, 2)])
+@pytest.mark.parametrize("ensemble", [0, 1])
+def test_cell_without_numbers_along_an_axis(mesh, axes, ensemble):
+    """Forces, states and cell data of the others bit for bit, beside a cell
+    whose nodes are all NaN along some axes (it has no box there), in the lists
+    built at the load and in those of every step that follow from the NaN."""
+    x, box = _cells(mesh)
+    beside = x if ensemble else None
+    want, err = _run(mesh, x, box, beside=beside)
+    assert err == 0
+    n = len(x) + 1
+    broken = x[13:14].copy()
+    broken[..., list(axes)] = np.nan
+    y = np.concatenate([x[:13], broken, x[13:]])
+    got, err = _run(mesh, y, box, beside=beside)
+    assert err & NAN
+    keep = np.arange(n) != 13
+    _same(got, want, n, keep)
