@@ -448,10 +448,14 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
                 mine &= mine - 1u;
                 if (nd < MAXD) dl[(size_t)nd * SLOTS] = (uint16_t)ss.item[b + q];
                 ++nd;
+                // 0 also where the pair is a dissipative one only: at the cut-off,
+                // or with a node that is no number, which must not get into F
                 const double k = ss.res[0][q];
-                FX = fma(k, ss.res[1][q], FX);
-                FY = fma(k, ss.res[2][q], FY);
-                FZ = fma(k, ss.res[3][q], FZ);
+                if (k != 0.0) {
+                    FX = fma(k, ss.res[1][q], FX);
+                    FY = fma(k, ss.res[2][q], FY);
+                    FZ = fma(k, ss.res[3][q], FZ);
+                }
                 vsum.x += ss.res[4][q]; vsum.y += ss.res[5][q]; vsum.z += ss.res[6][q];
             }
             __syncwarp();

@@ -69,3 +69,55 @@ def test_cell_without_numbers_along_an_axis(mesh, axes, ensemble):
     assert err & NAN
     keep = np.arange(n) != 13
     _same(got, want, n, keep)
+
+
+def test_nan_neighbour_leaves_the_conservative_force(mesh):
+    """Two cells in contact, one of which has a NaN velocity at a node that
+    touches nothing: in the first step the node and its three bond neighbours
+    have NaN positions, listed as contacts of the other cell's nodes.  Their
+    pairs take no part in the conservative force, which is that of the run
+    without the NaN less the forces of those pairs, to the rounding of the two
+    float results."""
+    p = W.base_params(box_len=(20.0, 20.0, 20.0), growth_rate=0.0, use_rigid_box=0)
+    st = W.state(np.array([[5.0, 5.0, 5.0], [7.1, 5.1, 5.05]], np.float32))
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
+    nn = np.asarray(mesh["nn"])[:, :180].T
+
+    def run(node=None):
+        sim = cs.Simulation(p, topo, 2)
+        sim.set_option(cs.OPT_RECORD_PAIRS, 1)
+        sim.set_option(cs.OPT_PAIR_CAPACITY, 1 << 16)
+        v = [np.zeros(2 * 192, np.float32) for _ in range(3)]
+        if node is not None:
+            v[0][192 + node] = np.nan
+        sim.load_state(st["X"], st["Y"], st["Z"], *v, n_cells=2)
+        first = sim.pairs(0)
+        sim.step(1, raise_on_error=False)
+        f = sim.forces()
+        s = sim.state()
+        sim.close()
+        return (first, np.stack([f["FC" + k] for k in "XYZ"], -1)[:180].astype(np.float64),
+                np.stack([s[k] for k in "XYZ"], -1).astype(np.float64))
+
+    pairs, want, x = run()
+    touching = set(pairs[pairs[:, 0] == 1][:, 1].tolist())
+    # a node next to a touching one that touches nothing itself
+    node = next(m for m in range(180) if m not in touching and touching & set(nn[m].tolist()))
+    gone = {node} | set(nn[node].tolist())
+    _, got, y = run(node)
+    assert np.isnan(y[192 + np.array(sorted(gone)), 0]).all() and np.isfinite(y[:180]).all()
+    assert np.isfinite(got).all()
+    lost = np.zeros((180, 3))
+    for a, i, _, j in pairs:
+        if a == 0 and j in gone:
+            d = x[i] - x[192 + j]
+            r = np.linalg.norm(d)
+            assert r < p["attraction_range"] - 1e-4 and abs(r - p["repulsion_range"]) > 1e-4
+            e = p["youngs_mod"]
+            k = -p["attraction_strength"] * e * (p["attraction_range"] - r)
+            if r < p["repulsion_range"]:
+                k += p["repulsion_strength"] * e * (p["repulsion_range"] - r)
+            lost[i] += k * d / r
+    assert (np.abs(lost).max(1) > 0).any()
+    tol = 2.0 ** -23 * (np.abs(want).max(1) + np.abs(got).max(1) + np.abs(lost).max(1))[:, None]
+    assert (np.abs(want - lost - got) <= tol).all()
