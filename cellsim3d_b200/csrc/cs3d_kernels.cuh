@@ -262,8 +262,8 @@ __device__ __forceinline__ void angle_term(const Arm &p, const Arm &q, float th0
 // boxes and stale insertion bin ranges.
 struct SlotData {
     int cell[MAXC];
-    float4 lo[MAXC], hi[MAXC];
-    int4 range[MAXC];   // lowest and highest bin as 16-bit numbers, low | high << 16, by axis
+    float4 lo[MAXC], hi[MAXC];   // w: lowest, highest bin along z (int bits)
+    int4 range[MAXC];            // lowest and highest bin along x and y
     float mn[3];
     int div[3];
 };
@@ -294,14 +294,15 @@ __device__ __forceinline__ void slots_boxes(const Dev &d, const InstParams &P, i
     if (t < nc) {
         int c = sd.cell[t];
         float4 lo = d.aabb[par][2 * c], hi = d.aabb[par][2 * c + 1];
-        sd.lo[t] = lo;
-        sd.hi[t] = hi;
         int st, en;
         int4 rg;
-        bin_range_axis(lo.x, hi.x, P.ra, sd.mn[0], sd.div[0], st, en); rg.x = (st & 0xffff) | en << 16;
-        bin_range_axis(lo.y, hi.y, P.ra, sd.mn[1], sd.div[1], st, en); rg.y = (st & 0xffff) | en << 16;
-        bin_range_axis(lo.z, hi.z, P.ra, sd.mn[2], sd.div[2], st, en); rg.z = (st & 0xffff) | en << 16;
-        rg.w = 0;
+        bin_range_axis(lo.x, hi.x, P.ra, sd.mn[0], sd.div[0], rg.x, rg.y);
+        bin_range_axis(lo.y, hi.y, P.ra, sd.mn[1], sd.div[1], rg.z, rg.w);
+        bin_range_axis(lo.z, hi.z, P.ra, sd.mn[2], sd.div[2], st, en);
+        lo.w = __int_as_float(st);
+        hi.w = __int_as_float(en);
+        sd.lo[t] = lo;
+        sd.hi[t] = hi;
         sd.range[t] = rg;
     }
 }
@@ -324,8 +325,9 @@ __device__ __forceinline__ NodeBins node_bins(const SlotData &sd, float3 x)
 __device__ __forceinline__ bool slot_ok(const SlotData &sd, const InstParams &P, float3 x, NodeBins nb, int s)
 {
     const int4 g = sd.range[s];
-    return nb.b0 >= (short)g.x && nb.b0 <= g.x >> 16 && nb.b1 >= (short)g.y && nb.b1 <= g.y >> 16 &&
-           nb.b2 >= (short)g.z && nb.b2 <= g.z >> 16 && aabb_keep(sd.lo[s], sd.hi[s], x.x, x.y, x.z, P.ra2);
+    const float4 lo = sd.lo[s], hi = sd.hi[s];
+    return nb.b0 >= g.x && nb.b0 <= g.y && nb.b1 >= g.z && nb.b1 <= g.w && nb.b2 >= __float_as_int(lo.w) &&
+           nb.b2 <= __float_as_int(hi.w) && aabb_keep(lo, hi, x.x, x.y, x.z, P.ra2);
 }
 
 // ---------------------------------------------------------------------------
@@ -886,8 +888,8 @@ struct ArmForces {
 
 // The next cell's nodes and first entries towards L2: a system of more than
 // some 20,000 cells does not stay there between steps.  With the bins of a
-// node by multiplication (div_dl), a candidate's bin range in one word an
-// axis and the cell's set-up spread over the warps: S1 of 100,000 packed
+// node by multiplication (div_dl), a candidate's bin ranges in two 16-byte
+// words with its box and the cell's set-up spread over the warps: S1 of 100,000 packed
 // cells 1.86 -> 1.68 ms, of 3000 growing ones 85 -> 80 us.
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void prefetch_cell(const Dev &d, int a)

@@ -121,3 +121,19 @@ def test_nan_neighbour_leaves_the_conservative_force(mesh):
     assert (np.abs(lost).max(1) > 0).any()
     tol = 2.0 ** -23 * (np.abs(want).max(1) + np.abs(got).max(1) + np.abs(lost).max(1))[:, None]
     assert (np.abs(want - lost - got) <= tol).all()
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("far", [-9.0e4, -1.0e5, -4.0e5])
+def test_contacts_of_a_wide_system(mesh, axis, far):
+    """The cells of a cluster bit for bit with a lone cell so far below them
+    that their grid bins number more than 16 bits hold (32767 bins of 2.9)."""
+    x, box = _cells(mesh)
+    want, err = _run(mesh, x, box, use_rigid_box=0)
+    assert err == 0
+    n = len(x) + 1
+    lone = x[:1].copy()
+    lone[:, :180, axis] += np.float32(far)
+    got, err = _run(mesh, np.concatenate([x[:13], lone, x[13:]]), box, use_rigid_box=0)
+    assert err == 0
+    _same(got, want, n, np.arange(n) != 13)
