@@ -184,14 +184,17 @@ __device__ __forceinline__ int grid_div(float mn, float mx)
 }
 
 // x / DL, correctly rounded: the product with the rounded reciprocal, corrected
-// once by the exact remainder (three operations; a division takes a dozen and
-// a branch).  Equal to the IEEE quotient for every float of magnitude 2^-30 to
-// 2^34, checked over all of them; only the integer part is used.
+// once by the exact remainder (Markstein's method, as div_m; three operations,
+// where a division takes a dozen and a branch).  Equal to the IEEE quotient for
+// every float of magnitude 2^-30 to 2^34, checked over all of them, and for
+// infinities and NaN, whose remainder is no number; only the integer part is
+// used.
 __device__ __forceinline__ float div_dl(float x)
 {
     constexpr float r = 1.0f / DL;
     const float q = __fmul_rn(x, r);
-    return __fmaf_rn(__fmaf_rn(-q, DL, x), r, q);
+    const float e = __fmaf_rn(-q, DL, x);
+    return e == e ? __fmaf_rn(e, r, q) : q;
 }
 
 // Node bin along one axis, src/propagate.cu:360-370.

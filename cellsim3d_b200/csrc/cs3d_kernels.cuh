@@ -762,12 +762,14 @@ struct GeomScratch {
     double fc[CS3D_FACES][3];   // face centres relative to the cell's centre of mass
 };
 
-// t / 180, correctly rounded as div_m.
+// t / 180, correctly rounded by Markstein's method as div_m; an infinity stays
+// one (its remainder is no number).
 __device__ __forceinline__ double div_nodes(double t)
 {
     constexpr double r = 1.0 / NODES;
     const double q = t * r;
-    return fma(fma(-q, (double)NODES, t), r, q);
+    const double e = fma(-q, (double)NODES, t);
+    return e == e ? fma(e, r, q) : q;
 }
 
 // Centre of mass (FP64 sum, src/centermass.cu:8-50) and bounding box

@@ -137,3 +137,55 @@ def test_contacts_of_a_wide_system(mesh, axis, far):
     got, err = _run(mesh, np.concatenate([x[:13], lone, x[13:]]), box, use_rigid_box=0)
     assert err == 0
     _same(got, want, n, np.arange(n) != 13)
+
+
+@pytest.mark.parametrize("ensemble", [0, 1])
+def test_cell_at_infinity(mesh, ensemble):
+    """A cell at +inf in x: its box and centre of mass are there, and the
+    others' forces, states and cell data are those without it, bit for bit."""
+    x, box = _cells(mesh)
+    beside = x if ensemble else None
+    want, _ = _run(mesh, x, box, beside=beside, use_rigid_box=0)
+    n = len(x) + 1
+    far = x[13:14].copy()
+    far[:, :180, 0] = np.inf
+    got, err = _run(mesh, np.concatenate([x[:13], far, x[13:]]), box, beside=beside, use_rigid_box=0)
+    assert err & NAN   # its forces are no numbers, and so its positions after a step
+    _same(got, want, n, np.arange(n) != 13)
+
+
+def test_centre_of_mass_of_an_infinite_node(mesh):
+    """Centres of mass and boxes as float64 sums give them, with one node of one cell at -inf, at the load."""
+    x, box = _cells(mesh, k=2)
+    x[5, 17, 1] = -np.inf
+    out, _ = _run(mesh, x, box, steps=0, use_rigid_box=0)
+    cells = out[-1]
+    cm = (x[:, :180].astype(np.float64).sum(1) / 180.0).astype(np.float32)
+    assert np.isneginf(cells["cm"][5, 1]) and np.isneginf(cm[5, 1])
+    # the float64 sums differ by their order, so that the floats may differ by one
+    ok = np.isfinite(cm)
+    assert ok.sum() == cm.size - 1
+    assert np.allclose(cells["cm"][ok], cm[ok], rtol=2.0 ** -23, atol=0)
+    assert np.array_equal(cells["aabb"][:, 0::2], x[:, :180].min(1))
+    assert np.array_equal(cells["aabb"][:, 1::2], x[:, :180].max(1))
+
+
+def test_grid_of_a_system_that_reaches_minus_infinity(mesh):
+    """With a cell at -inf along an axis every node's bin is the last one and
+    every box's range begins past it (float to int conversion saturates, as in
+    the reference's grid), so that no pair counts."""
+    x, box = _cells(mesh, k=2)
+    rest = np.zeros((192, 3), np.float32)
+    rest[:180] = W.centred(W.scaled_xyz(mesh))
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), *[np.ascontiguousarray(rest[:, q]) for q in range(3)])
+    far = x[:1].copy()
+    far[:, :180, 2] = -np.inf
+    counts = []
+    for y in (x, np.concatenate([x, far])):
+        sim = cs.Simulation(W.base_params(box_len=(box, box, box), growth_rate=0.0), topo, len(y))
+        sim.set_option(cs.OPT_RECORD_PAIRS, 1)
+        sim.set_option(cs.OPT_PAIR_CAPACITY, 1 << 16)
+        sim.load_state(*[np.ascontiguousarray(y[..., q].reshape(-1)) for q in range(3)], n_cells=len(y))
+        counts.append(len(sim.pairs(1)))
+        sim.close()
+    assert counts[0] > 0 and counts[1] == 0
