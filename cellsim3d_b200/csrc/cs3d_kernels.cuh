@@ -809,12 +809,14 @@ __device__ __forceinline__ void geom_box(const GeomScratch &gs, float4 &lo, floa
     }
 }
 
-// sqrt(x) to within an ulp or so (0 for x below 1e-280, where no triangle of a
-// cell is): the approximate inverse root refined once, then Heron's step.
+// sqrt(x) to within an ulp: the approximate inverse root, refined once (to 1e-12),
+// then Heron's step by the exact remainder.  Zero, values that the approximation
+// does not reach and those that are no finite numbers take the full root.
 __device__ __forceinline__ double sqrt_full(double x)
 {
+    if (!(x > 1e-280 && x < 1e280)) return sqrt(x);
     const double r = rsqrt_nr(x), s = x * r;
-    return x > 1e-280 ? fma(0.5 * r, fma(-s, s, x), s) : 0.0;
+    return fma(0.5 * r, fma(-s, s, x), s);
 }
 
 // Volume, area and the division test, src/volume.cu:5-163, in FP64.  Each

@@ -189,3 +189,24 @@ def test_grid_of_a_system_that_reaches_minus_infinity(mesh):
         counts.append(len(sim.pairs(1)))
         sim.close()
     assert counts[0] > 0 and counts[1] == 0
+
+
+def test_area_and_volume_of_a_broken_cell(mesh):
+    """The division test of a cell with a NaN node stores a volume and an area
+    that are no numbers and raises its bit; those of a cell that does not touch it are
+    those of the run without the NaN."""
+    x, box = _cells(mesh, k=2)
+    got = []
+    for node in (None, 17):
+        y = x.copy()
+        if node is not None:
+            y[5, node] = np.nan
+        out, err = _run(mesh, y, box, steps=1, growth_rate=0.002, division_vol=1e3)
+        got.append(out[-1])
+    assert err & NAN and err & 0x010
+    for k in ("volume", "area"):
+        assert np.isnan(got[1][k][5]) and np.isfinite(got[0][k]).all() and (got[0][k] > 0).all()
+    far = (np.abs(x[:, 0] - x[5, 0]) > 1.0).sum(1) == 3   # the one that does not touch it
+    assert far.sum() == 1
+    for k in ("volume", "area"):
+        assert np.array_equal(got[0][k][far], got[1][k][far])
