@@ -1604,6 +1604,9 @@ __device__ __forceinline__ void div_apply(const Dev &d, int par, bool fuse, floa
             d.V[gb] = d.V[ga];
             d.FC[gb] = make_float4(0, 0, 0, 0);
             d.FD[gb] = make_float4(0, 0, 0, 0);
+            // no random force before the daughter's first step: the slot may hold
+            // that of a cell of an earlier load
+            d.FR[gb] = make_float4(0, 0, 0, 0);
         }
         __syncthreads();
         if (fuse) {   // a thread's own nodes

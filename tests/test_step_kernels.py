@@ -198,3 +198,30 @@ def test_partial_builds_do_not_change_results(mesh, skin, over):
     assert np.array_equal(ea, eb)
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n", [8, 160])
+@pytest.mark.parametrize("com", [0, 1])
+def test_reloaded_context_repeats_the_run(mesh, n, com):
+    """With noise, growth and divisions: a load into a context that has already
+    run gives the states, forces and events of a fresh context, bit for bit
+    (a daughter's slot keeps nothing of the cell it held before), with the steps
+    in one kernel (8 cells) and as a launch sequence (160)."""
+    p, st = _growing(n, add_rands=1, rand_scale_factor=0.5, rand_seed=5, correct_com=com)
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
+    rng = cs.Ranmar(p["rng_ij"], p["rng_kl"])
+    got = []
+    for passes in (1, 2):
+        sim = cs.Simulation(p, topo, 3 * n)
+        for _ in range(passes):
+            known = len(sim.events())
+            sim.load_state(st["X"], st["Y"], st["Z"], n_cells=n)
+            sim.set_rng(rng)
+            sim.step(10)
+        got.append((sim.state(), sim.forces(), sim.random_force(), sim.events()[known:]))
+        sim.close()
+    (a, fa, ra, ea), (b, fb, rb, eb) = got
+    assert a["n"] == b["n"] > n and len(ea) == a["n"] - n and len(eb) == len(ea)
+    for u, v in ((a, b), (fa, fb), (ra, rb)):
+        for k in u:
+            assert np.array_equal(u[k], v[k]), k
