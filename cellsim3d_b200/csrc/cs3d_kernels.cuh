@@ -2163,7 +2163,7 @@ __device__ __forceinline__ void list_stats(const Dev &d, ListSmem &sm)
 // B2: the lists of cell a, with the radius of whole builds (full) or with the
 // cells' displacements.  The whole CTA; its warps take a patch of 30
 // neighbouring nodes each.  False, without full only, if some node has more
-// entries than it has room for.
+// entries than it has room for, or the cell more candidates.
 __device__ __forceinline__ bool nb_cell(const Dev &d, int a, int node, unsigned epoch, bool full, ListSmem &sm)
 {
     const int t = threadIdx.x, wid = t >> 5, lane = t & 31;
@@ -2255,7 +2255,7 @@ __device__ __forceinline__ bool nb_cell(const Dev &d, int a, int node, unsigned 
             }
         }
     }
-    if (!full && __syncthreads_or(e.cnt > MAXE)) return false;
+    if (!full && __syncthreads_or(e.cnt > MAXE || nslot > MAXC)) return false;
     if (real) {
         d.nent[g] = (uint8_t)(e.cnt < MAXE ? e.cnt : MAXE);
         // new anchors, except for the neighbours of divided cells: other
@@ -2290,8 +2290,8 @@ __device__ __forceinline__ bool nb_cell(const Dev &d, int a, int node, unsigned 
 }
 
 // The listed cells.  Where a partial build's radius gives a node more entries
-// than it has room for (cells far from their anchors in a crowd), the cell's
-// lists are built with the radius of a whole build, which covers this step, and
+// than it has room for, or the cell more candidates (cells far from their
+// anchors in a crowd), the cell's lists are built with the radius of a whole build, which covers this step, and
 // the instance is rebuilt whole in the next one.
 __device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
 {

@@ -225,3 +225,64 @@ def test_reloaded_context_repeats_the_run(mesh, n, com):
     for u, v in ((a, b), (fa, fb), (ra, rb)):
         for k in u:
             assert np.array_equal(u[k], v[k]), k
+
+
+def _crowd_around(xyz, near, far):
+    """A large flat cell, a cell inside it and others outside, each at a gap from
+    a node of the large one: 115 at `near`, 35 at `far`."""
+    from scipy.spatial import cKDTree
+    axes = np.array([18.0, 18.0, 8.0])
+    big = xyz * axes
+    tree = cKDTree(big)
+    cells = [big, xyz * 1.3]
+    for q, i in enumerate(np.random.default_rng(1).permutation(180)[:150]):
+        gap = near if q < 115 else far
+        out = big[i] / axes ** 2
+        out /= np.linalg.norm(out)
+        lo, hi = 0.0, 3.0
+        for _ in range(60):
+            mid = 0.5 * (lo + hi)
+            if tree.query(xyz * 0.9 + big[i] + out * mid)[0].min() < gap:
+                lo = mid
+            else:
+                hi = mid
+        cells.append(xyz * 0.9 + big[i] + out * hi)
+    return np.stack(cells)
+
+
+def test_partial_build_with_more_candidates_than_slots(mesh):
+    """A cell with 115 others within the list radius and 35 more within that of
+    a partial build, which adds the distances from the anchors: 150 are more
+    candidates than there are slots.  All cells drift at one velocity and the
+    one inside divides in the first step.  The steps run, and their states are
+    those with a skin so small that every build is a whole one."""
+    from scipy.spatial import cKDTree
+    xyz = W.centred(W.scaled_xyz(mesh)).astype(np.float64)
+    x = _crowd_around(xyz, 0.35, 0.45)
+    # 0.3 and a skin of 0.1; two steps of 0.02 and less than half the skin
+    gaps = np.array([cKDTree(x[0]).query(c)[0].min() for c in x[2:]])
+    assert (gaps < 0.39).sum() == 115 and (gaps < 0.475).sum() == 150 and gaps.min() > 0.31
+    n = len(x)
+    st = _pack((x + 30.0).astype(np.float32))
+    v = np.zeros(n * 192, np.float32)
+    u = v.reshape(n, 192)
+    u[:, :180] = 200.0
+    p = W.base_params(box_len=(60.0, 60.0, 60.0), use_rigid_box=0, constrain_angles=0, youngs_mod=1e-3,
+                      stiffness1=1e-6, internal_damping=0.0, viscotic_damping=0.0, gamma_visc=0.0, max_pressure=0.0,
+                      min_pressure=0.0, growth_rate=1e-9, division_vol=6.0)
+    rest = np.zeros((192, 3), np.float32)
+    rest[:180] = xyz
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), *[np.ascontiguousarray(rest[:, q]) for q in range(3)])
+    got = []
+    for skin in (0.1, 0.03):
+        sim = cs.Simulation(p, topo, n + 8)
+        sim.set_option(cs.OPT_SKIN, int(round(skin * 1e6)))
+        sim.load_state(st["X"], st["Y"], st["Z"], v, v * 0, v * 0, n_cells=n)
+        sim.step(4)
+        got.append((sim.state(), sim.events(), sim.forces()))
+        sim.close()
+    (a, ea, fa), (b, eb, fb) = got
+    assert np.array_equal(ea, eb) and ea.tolist() == [[1, 1, n]]
+    for s, t in ((a, b), (fa, fb)):
+        for k in s:
+            assert np.array_equal(s[k], t[k]), k
