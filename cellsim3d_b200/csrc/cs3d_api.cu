@@ -706,7 +706,7 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     AL(d.dlist, (size_t)c->cap_total * MAXD * SLOTS); AL(d.ndis, nodes);
     AL(d.Xb, nodes);
     AL(d.ent, (size_t)c->cap_total * MAXE * SLOTS); AL(d.nent, nodes);
-    AL(d.nbox, 2 * (size_t)c->cap_total); AL(d.bins, bins); AL(d.bnext, c->cap_total); AL(d.epoch, 1);
+    AL(d.nbox, 2 * (size_t)c->cap_total); AL(d.bins, bins); AL(d.bnext, c->cap_total); AL(d.large, c->cap_total); AL(d.epoch, 1);
     AL(d.cdisp, c->cap_total); AL(d.build, c->cap_total); AL(d.n_build, 1); AL(d.mark, c->cap_total);
     AL(d.divtab, c->cap_total); AL(d.div_total, 1); AL(d.div_prev, 1); AL(d.flagged, c->cap_total);
     AL(d.events, d.ev_cap); AL(d.n_events, 1);
@@ -1363,7 +1363,7 @@ int cs3d_get_stats(cs3d_ctx *c, long long *stats, int n)
     std::vector<InstState> st(c->n_inst);
     CK(cudaMemcpyAsync(st.data(), c->d.st, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    long long v[8] = {c->host_step, 0, 0, 0, c->launches_per_step, 0, 0, 0};
+    long long v[9] = {c->host_step, 0, 0, 0, c->launches_per_step, 0, 0, 0, 0};
     for (auto &q : st) v[5] = std::max<long long>(v[5], q.max_halo);
     for (auto &q : st) {
         v[1] += q.rebuilds;
@@ -1371,8 +1371,9 @@ int cs3d_get_stats(cs3d_ctx *c, long long *stats, int n)
         v[3] = std::max<long long>(v[3], q.max_cand);
         v[6] += q.built;
         v[7] += q.rebuilds_div;
+        v[8] += q.searches;
     }
-    for (int k = 0; k < n && k < 8; ++k) stats[k] = v[k];
+    for (int k = 0; k < n && k < 9; ++k) stats[k] = v[k];
     return CS3D_OK;
 }
 
@@ -1407,7 +1408,7 @@ struct StaticScratch {
     float4 aabb0[2 * SCAP], aabb1[2 * SCAP];
     float4 nbox[2 * SCAP];
     unsigned long long bins[SBINS];
-    int bnext[SCAP];
+    int bnext[SCAP], large[SCAP];
     unsigned epoch;
     float cdisp[SCAP];
     int build[SCAP], n_build;
@@ -1460,7 +1461,7 @@ Dev static_dev(StaticScratch *s)
     d.cand = s->cand; d.ncand = s->ncand;
     d.dlist = s->dlist; d.ndis = s->ndis;
     d.ent = s->ent; d.nent = s->nent;
-    d.nbox = s->nbox; d.bins = s->bins; d.bnext = s->bnext; d.epoch = &s->epoch;
+    d.nbox = s->nbox; d.bins = s->bins; d.bnext = s->bnext; d.large = s->large; d.epoch = &s->epoch;
     d.cdisp = s->cdisp; d.build = s->build; d.n_build = &s->n_build; d.mark = s->mark;
     d.divtab = s->divtab; d.div_total = &s->div_total; d.div_prev = &s->div_prev; d.flagged = s->flagged;
     d.events = s->events; d.n_events = &s->n_events; d.ev_cap = SEVENTS;

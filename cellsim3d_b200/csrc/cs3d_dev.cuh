@@ -13,6 +13,7 @@ constexpr int NODES = CS3D_NODES;      // real nodes per cell
 constexpr int MAXC = CS3D_MAX_CAND;    // contact-candidate cells per cell
 constexpr int MAXE = CS3D_MAX_ENTRIES; // contact-candidate nodes per node
 constexpr int MAXD = CS3D_MAX_DIS;     // dissipative pairs per node
+constexpr int LEVELS = 12;             // size classes of the list build's cell table
 constexpr float DL = 2.9f;             // reference grid spacing, src/GPUbounce.cu:756
 
 // Per-instance constants (uploaded once).
@@ -65,8 +66,11 @@ struct InstState {
     int max_entries, max_cand, max_halo;
     unsigned hbase;        // first bin of this instance's slice of the cell table
     int hbits;             // log2 of the slice size (0: not rebuilding)
-    unsigned hmax[3];      // largest half extent of its cells' boxes at this build (float bits)
+    unsigned hmax[LEVELS][3];  // largest half extent of the table's boxes at this build (float bits), by size class
+    int top;               // highest class in the table
+    int n_large, n_giant;  // cells in its list (d.large): large ones, and those of no class
     int built;             // cells whose lists were built (cumulative)
+    int searches;          // of those, the ones for which all cells were looked at
     int rebuilds;
     int rebuilds_div;      // of those, the ones only the rule for dividing instances called for
     float syscm[3];        // the reference's system centre of mass as of its last
@@ -135,6 +139,7 @@ struct Dev {
     float4 *nbox;       // [2*cell] lo, hi
     unsigned long long *bins;
     int *bnext;         // [cell]
+    int *large;         // [cell] by instance: large cells from its base on, those of no class from its end back
     float *cdisp;       // [cell] largest distance of its nodes from their anchors
     int *build;         // cells of this step's partial builds
     int *n_build;

@@ -410,7 +410,9 @@ int cs3d_last_error(cs3d_ctx *ctx, int inst, uint32_t *bits);
  * (counted only with CS3D_OPT_HALO_STATS, else 0),
  * [6] cell neighbour lists built (cumulative), [7] of the rebuilds [1], those
  * that only the rule for dividing instances called for (more than one cell in
- * 16 divided in the step, with no other cause). */
+ * 16 divided in the step, with no other cause), [8] of the lists [6], those for
+ * which all cells of the instance were looked at (a cell far larger than the
+ * mesh at rest, or one with more than 192 others in reach). */
 int cs3d_get_stats(cs3d_ctx *ctx, long long *stats, int n);
 
 /* Profiling pass: n_steps steps launched kernel by kernel (not as a graph)

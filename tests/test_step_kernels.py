@@ -286,3 +286,74 @@ def test_partial_build_with_more_candidates_than_slots(mesh):
     for s, t in ((a, b), (fa, fb)):
         for k in s:
             assert np.array_equal(s[k], t[k]), k
+
+
+def _small_and_large(mesh, scales, small, deep):
+    """Small cells on a lattice and large ones past one of its corners each, in contact with a few."""
+    rng = np.random.default_rng(23)
+    xyz = W.centred(W.scaled_xyz(mesh)).astype(np.float64)
+    k = int(np.ceil(small ** (1.0 / 3.0)))
+    c = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3)[:small] * 1.15
+    c = c + rng.uniform(-0.05, 0.05, c.shape)
+    x = [xyz * 0.5 + p for p in c]
+    for q, s in enumerate(scales):
+        turn = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        out = np.array([1.0 if q >> b & 1 else -1.0 for b in range(3)])
+        at = np.where(out > 0, c.max(0), 0.0) + out / np.sqrt(3.0) * (s - deep)
+        x.insert(len(x) // (q + 2), xyz @ turn * s + at)
+    return (np.stack(x) + 40.0).astype(np.float32)
+
+
+def _check_pairs(mesh, x):
+    """Contact pairs of the cells x against a search over all nodes; the context's counters."""
+    n = len(x)
+    st = _pack(x)
+    p = W.base_params(box_len=(400.0, 400.0, 400.0), growth_rate=0.0, use_rigid_box=0)
+    rest = np.zeros((192, 3), np.float32)
+    rest[:180] = W.centred(W.scaled_xyz(mesh))
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), *[np.ascontiguousarray(rest[:, q]) for q in range(3)])
+    sim = cs.Simulation(p, topo, n)
+    sim.set_option(cs.OPT_RECORD_PAIRS, 1)
+    sim.set_option(cs.OPT_PAIR_CAPACITY, 1 << 21)
+    sim.load_state(st["X"], st["Y"], st["Z"], n_cells=n)
+    sim.forces()
+    got = sim.pairs(0).astype(np.int64)
+    got = np.sort((got[:, 0] * 180 + got[:, 1]) * (n * 180) + got[:, 2] * 180 + got[:, 3])
+    want = _pairs_within(x.astype(np.float64), float(np.float32(p["attraction_range"])))
+    assert np.array_equal(got, want)
+    s = sim.stats()
+    sim.close()
+    return s
+
+
+@pytest.mark.parametrize("scales,small,deep,searches", [((3.0, 3.2, 3.4, 3.6), 300, 0.8, 0), ((8.6,), 190, 2.5, 0),
+                                                        ((14.0,), 400, 0.8, 1), ((4.0, 5.0, 14.0), 400, 0.8, 1),
+                                                        ((12.0,) * 6, 729, 0.8, 6)])
+def test_list_build_with_several_large_cells(mesh, scales, small, deep, searches):
+    """Contact pairs against a search over all nodes, with cells on both sides
+    of the largest that the table of the cells takes, and with 129 to 192 and
+    more boxes in reach of one.  The small cells find theirs through the table all
+    the same: only a large cell looks at all the others."""
+    x = _small_and_large(mesh, scales, small, deep)
+    s = _check_pairs(mesh, x)
+    assert s["full_searches"] == searches and s["lists_built"] == len(x)
+    lo, hi = x[:, :180].min(1) - 0.2, x[:, :180].max(1) + 0.2
+    reach = [(np.all((lo <= hi[a]) & (hi >= lo[a]), axis=1)).sum() - 1 for a in range(len(x))]
+    if small == 190:
+        assert 128 < max(reach) <= 192
+
+
+def test_list_build_with_cells_of_three_sizes(mesh):
+    """Contact pairs against a search over all nodes where more cells than the
+    list of large ones holds are 4 and 8 times the size of the others, lattice
+    beside lattice: the size classes of the table."""
+    rng = np.random.default_rng(31)
+    xyz = W.centred(W.scaled_xyz(mesh)).astype(np.float64)
+    x, right = [], 0.0
+    for scale, m in ((0.9, (5, 10, 10)), (8.0, (4, 5, 5)), (3.8, (4, 5, 5)), (0.6, (3, 8, 8))):
+        c = np.stack(np.meshgrid(*[np.arange(k) for k in m], indexing="ij"), -1).reshape(-1, 3) * (2.0 * scale + 0.1)
+        c = c + rng.uniform(-0.02, 0.02, c.shape) + [right + scale, 0.0, 0.0]
+        x += [xyz * scale + p for p in c]
+        right = c[:, 0].max() + scale + 0.1
+    x = (np.stack(x)[rng.permutation(len(x))] + 10.0).astype(np.float32)
+    assert _check_pairs(mesh, x)["full_searches"] == 0
