@@ -578,6 +578,15 @@ unsigned take_states(cs3d_ctx *c)
     return bits;
 }
 
+// Whether some instance has been left half way through a step that gave up and
+// not been loaded since.
+bool torn(const cs3d_ctx *c)
+{
+    for (const InstState &st : c->hst)
+        if (st.err & CS3D_ERRBIT_SYNC) return true;
+    return false;
+}
+
 int read_errors(cs3d_ctx *c, unsigned *any)
 {
     if (int rc = fetch_states(c)) return rc;
@@ -687,6 +696,7 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
     d.ev_cap = std::max(1 << 16, 2 * c->cap_total);
     d.far_cap = d.ev_cap;
     d.pair_cap = 1;
+    d.polls = SYNC_POLLS;
     Arena ar;
     const auto lay_out = [&] {
         ar.at = 0;
@@ -828,6 +838,10 @@ int cs3d_set_option(cs3d_ctx *c, int option, long long value)
     case CS3D_OPT_HALO_STATS:
         c->d.halo_stats = value ? 1 : 0;
         break;
+    case CS3D_OPT_SYNC_POLLS:
+        if (value < 0 || value > UINT32_MAX) return CS3D_E_ARG;
+        c->d.polls = (unsigned)value;
+        return CS3D_OK;  // the graphs have no barriers
     case CS3D_OPT_PAIR_CAPACITY: {
         if (value < 1) return CS3D_E_ARG;
         int4 *p = nullptr;
@@ -914,6 +928,7 @@ int cs3d_load_state(cs3d_ctx *c, int inst, int n, const float *X, const float *Y
         if (int rc = wait_stream(c)) return rc;
     c->n_now += n - c->hn[inst];
     c->hn[inst] = n;
+    c->hst[inst].err = 0u;
     c->need_init = true;
     return CS3D_OK;
 }
@@ -950,6 +965,7 @@ int cs3d_get_rng(cs3d_ctx *c, int inst, cs3d_rng *r)
 int cs3d_step(cs3d_ctx *c, int n_steps)
 {
     if (!c || n_steps < 0) return CS3D_E_ARG;
+    if (torn(c)) return CS3D_E_DEVICE_FLAGS;
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;
@@ -982,6 +998,7 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
             // the cells may have outgrown the kernel
             unsigned bits = 0;
             if (!last && (rc = read_errors(c, &bits))) return rc;
+            if (bits & CS3D_ERRBIT_SYNC) return CS3D_E_DEVICE_FLAGS;
             continue;
         }
         // S2 integrates the next step unless the step shifts or softens
@@ -1004,6 +1021,10 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
     unsigned bits = 0;
     if ((rc = read_errors(c, &bits))) return rc;
     CK(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
+    if (bits & CS3D_ERRBIT_SYNC) {
+        c->prekicked = false;
+        return CS3D_E_DEVICE_FLAGS;
+    }
     if (bits & CS3D_ERRBIT_CAPACITY) return CS3D_E_CAPACITY;
     if (bits) return CS3D_E_DEVICE_FLAGS;
     return CS3D_OK;
@@ -1013,6 +1034,7 @@ int cs3d_profile_step(cs3d_ctx *c, int n_steps, float *kernel_ms, char *names, i
                       int max_kernels, int *n_kernels)
 {
     if (!c || n_steps <= 0 || !n_kernels) return CS3D_E_ARG;
+    if (torn(c)) return CS3D_E_DEVICE_FLAGS;
     cudaSetDevice(c->device);
     int rc = ensure_init(c);
     if (rc) return rc;

@@ -159,6 +159,7 @@ struct Dev {
     int *flags;         // [0] any rebuild, [1] any division
     int *deal;          // counters of the cells dealt out, by phase (Dealer)
     unsigned *bar;      // [0] arrivals, [1] barriers passed (k_steps; zero at its launch)
+    unsigned polls;     // looks at a barrier before a CTA gives up
     int4 *pairs;        // (cell_a<<8 | node_i, cell_b<<8 | node_j, kind, 0)
     unsigned long long *n_pairs;
     long long pair_cap;

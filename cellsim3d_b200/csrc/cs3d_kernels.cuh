@@ -735,6 +735,8 @@ __global__ void __launch_bounds__(256) k_init_begin(Dev d)
         st->ds = 0.0f;
         st->force_rebuild = 0;
         st->disp_step = 0u;
+        st->flagged = 0;   // not zero after a step left half done
+        st->div_count = 0;
         for (int p = 0; p < 2; ++p)
             for (int q = 0; q < 3; ++q) {
                 st->mm[p][2 * q] = f2o(1.0e30f);
@@ -2411,16 +2413,19 @@ union StepsSmem {
     float com[3][SLOTS];
 };
 
-// Waits at most this many polls (about a microsecond each) for the other CTAs.
+// Polls for the other CTAs at a barrier (about a microsecond each) by default.
 constexpr unsigned SYNC_POLLS = 1u << 22;
 
 // Polls until *p >= v.  Relaxed loads: an acquiring one empties the SM's L1,
 // which the CTAs still at work beside this one need (S1 of 440 cells took 38 us
 // beside acquiring polls, 24 without).  False if the others did not come: the
-// CTA must return.  One thread.
+// CTA must return.  It has counted itself in, so that those still to come pass
+// this barrier, do the next phase's work among themselves and give up at its
+// end, where the arrivals no longer add up.  Nothing of that state is stepped
+// again: the host refuses until the instances are loaded.  One thread.
 __device__ __forceinline__ bool poll_until(const Dev &d, const unsigned *p, unsigned v)
 {
-    for (unsigned polls = 0; polls < SYNC_POLLS; ++polls) {
+    for (unsigned polls = 0; polls < d.polls; ++polls) {
         unsigned u;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(u) : "l"(p) : "memory");
         if (u >= v) {
@@ -2429,7 +2434,7 @@ __device__ __forceinline__ bool poll_until(const Dev &d, const unsigned *p, unsi
         }
         __nanosleep(20);
     }
-    atomic_or_err(&d.st[0], CS3D_ERRBIT_SYNC);
+    for (int k = 0; k < d.n_inst; ++k) atomic_or_err(&d.st[k], CS3D_ERRBIT_SYNC);
     return false;
 }
 

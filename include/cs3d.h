@@ -53,7 +53,8 @@ extern "C" {
 #define CS3D_ERRBIT_HALO_OVERFLOW  0x100u  /* reserved, never raised */
 #define CS3D_ERRBIT_SOFT_CELLS     0x200u  /* more distinct softer cells requested than cell indices
                                               exist (the reference loops forever, src/GPUbounce.cu:1364-1384) */
-#define CS3D_ERRBIT_SYNC           0x400u  /* the blocks of a step kernel lost one another (never seen) */
+#define CS3D_ERRBIT_SYNC           0x400u  /* the blocks of a step kernel lost one another (never seen): the step was
+                                              left half done, and cs3d_step refuses until every instance is loaded again */
 
 #define CS3D_MAX_CAND     128   /* contact-candidate cells per cell */
 #define CS3D_MAX_ENTRIES   64   /* contact-candidate nodes per node */
@@ -383,6 +384,9 @@ int cs3d_get_grid(cs3d_ctx *ctx, int inst, float minmax[6], int divs[3]);
 #define CS3D_OPT_HALO_STATS    5   /* value 0/1: count the distinct contact-candidate nodes of each cell
                                       at every list build (cs3d_get_stats [5]); off by default, as the
                                       count costs the build a shared-memory atomic per entry */
+#define CS3D_OPT_SYNC_POLLS    6   /* value = times (2^22 by default, some seconds) that a block of a step kernel
+                                      looks whether the others have come to a barrier before it gives up with
+                                      CS3D_ERRBIT_SYNC */
 int cs3d_set_option(cs3d_ctx *ctx, int option, long long value);
 
 /* Contact pairs recorded during the last force evaluation (requires

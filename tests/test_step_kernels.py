@@ -357,3 +357,59 @@ def test_list_build_with_cells_of_three_sizes(mesh):
         right = c[:, 0].max() + scale + 0.1
     x = (np.stack(x)[rng.permutation(len(x))] + 10.0).astype(np.float32)
     assert _check_pairs(mesh, x)["full_searches"] == 0
+
+
+SYNC = 0x400
+
+
+@pytest.mark.parametrize("instances,com", [(1, 0), (1, 1), (2, 0)])
+@pytest.mark.parametrize("done", [0, 3])
+def test_steps_that_give_up_at_a_barrier(mesh, instances, com, done):
+    """Blocks that look for the others 0 times give up at the first barrier of a
+    launch: the step ends with SYNC, and further ones (also profiled, also with
+    the limit back at its default) are refused until every instance is loaded
+    again.  Then the run is that of a fresh context, bit for bit, divisions
+    included."""
+    p, st = _growing(8, correct_com=com)
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
+
+    def load(ens, k):
+        ens.load_state(k, st["X"], st["Y"], st["Z"], n_cells=8)
+        ens.set_rng(k, cs.Ranmar(p["rng_ij"], p["rng_kl"]))
+
+    got = []
+    for give_up in (0, 1):
+        ens = cs.Ensemble([p] * instances, topo, [40] * instances)
+        for k in range(instances):
+            load(ens, k)
+        if give_up:
+            ens.step(done)
+            ens.set_option(cs.OPT_SYNC_POLLS, 0)
+            assert ens.step(600, raise_on_error=False) == -7
+            assert all(ens.last_error(k) & SYNC for k in range(instances))
+            ens.set_option(cs.OPT_SYNC_POLLS, 1 << 22)
+            for k in range(instances):
+                assert ens.step(1, raise_on_error=False) == -7
+                with pytest.raises(cs.CS3DError):
+                    ens.profile_step(1)
+                load(ens, k)
+            assert ens.last_error(-1) == 0
+        known = [len(ens.events(k)) for k in range(instances)]
+        ens.step(20)
+        assert ens.stats()["launches_per_step"] == 1
+        got.append([(ens.state(k), ens.forces(k), len(ens.events(k)) - known[k]) for k in range(instances)])
+        ens.close()
+    for (a, fa, ea), (b, fb, eb) in zip(*got):
+        assert a["n"] == b["n"] == 8 + ea == 8 + eb > 8
+        for u, v in ((a, b), (fa, fb)):
+            for k in u:
+                assert np.array_equal(u[k], v[k]), k
+
+
+def test_barrier_limit_option_is_checked(mesh):
+    p, st = _growing(1)
+    sim = _sim(p, st, mesh)
+    for bad in (-1, 1 << 32):
+        with pytest.raises(cs.CS3DError):
+            sim.set_option(cs.OPT_SYNC_POLLS, bad)
+    sim.close()
