@@ -334,6 +334,7 @@ def run_cs3d(args, world, rank, local):
                           s["pressure"].copy(), s["youngs"].copy()))
     if dist:
         dist.barrier()
+    launched = ens.stats()["launches"]
     torch.cuda.synchronize()
     with ClockSampler(local) as clk:
         ens.step(args.steps)
@@ -377,8 +378,9 @@ def run_cs3d(args, world, rank, local):
     # whole job: node-steps summed over ranks, times the slowest rank's; the
     # end-to-end leg the same way, its copies summed
     ee = e2e or {"seconds": 0.0, "node_steps": 0.0, "h2d": 0.0, "d2h": 0.0}
-    (ms_max, e2e_s), (total_node_steps, e2e_ns, e2e_h2d, e2e_d2h) = reduce_over_ranks(
-        dist, "cuda", [ms, ee["seconds"]], [node_steps, ee["node_steps"], ee["h2d"], ee["d2h"]])
+    (ms_max, e2e_s), (total_node_steps, e2e_ns, e2e_h2d, e2e_d2h, launches) = reduce_over_ranks(
+        dist, "cuda", [ms, ee["seconds"]],
+        [node_steps, ee["node_steps"], ee["h2d"], ee["d2h"], stats["launches"] - launched])
     result = None
     if rank == 0:
         peak, peak_kind = _peaks()
@@ -415,8 +417,8 @@ def run_cs3d(args, world, rank, local):
             "step_roofline": {"achieved": NODE_BYTES * value / 1e9 / world, "frac": NODE_BYTES * value / 1e9 / world / peak},
             "kernels_ms": {k: round(v, 4) for k, v in prof},
             "profiled_step_ms": step_ms,
-            # every rank launches the same kernel sequence: the whole job's count
-            "gpu_launches": int(stats["launches_per_step"]) * args.steps * world,
+            # kernels of the timed steps, over all ranks
+            "gpu_launches": int(launches),
             "nl_rebuilds": stats["rebuilds"],
             "nl_rebuilds_div_rule": stats["rebuilds_div_rule"],
             "max_entries": stats["max_entries"],

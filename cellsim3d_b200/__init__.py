@@ -389,11 +389,11 @@ class Ensemble:
         return b.value
 
     def stats(self):
-        s = (C.c_longlong * 9)()
-        _lib.check(_lib.lib().cs3d_get_stats(self.h, s, 9), "cs3d_get_stats")
+        s = (C.c_longlong * 11)()
+        _lib.check(_lib.lib().cs3d_get_stats(self.h, s, 11), "cs3d_get_stats")
         return {"steps": s[0], "rebuilds": s[1], "max_entries": s[2], "max_cand": s[3], "launches_per_step": s[4],
                 "max_halo": s[5], "lists_built": s[6], "rebuilds_div_rule": s[7],
-                "full_searches": s[8]}
+                "full_searches": s[8], "launches": s[9], "list_fallbacks": s[10]}
 
 
 class Simulation(Ensemble):

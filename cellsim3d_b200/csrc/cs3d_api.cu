@@ -49,6 +49,7 @@ struct cs3d_ctx {
     std::vector<InstState> hst;    // the instances' states as last read
     std::vector<char> buf;         // small transfers
     cudaGraphExec_t graph[2][2][2][3] = {};  // [parity][division][integrate first][S2 mode: 0, fused 1, fused last 2]
+    long long graph_launches[2][2][2][3] = {};  // kernels of each
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // asynchronous read-back (cs3d_get_state_async): a copy stream, two
     // device staging slots and their events
@@ -57,7 +58,8 @@ struct cs3d_ctx {
     cudaEvent_t aready[2] = {nullptr, nullptr}, adone[2] = {nullptr, nullptr};
     bool apending[2] = {false, false};
     float last_ms = 0.f;
-    long long launches_per_step = 0;
+    long long launches_per_step = 0;   // of the last step (1: in a launch with others)
+    long long launches = 0;            // kernels launched by cs3d_step calls
     unsigned last_err_bits = 0;
 };
 
@@ -520,6 +522,7 @@ int get_graph(cs3d_ctx *c, int par, bool div, bool k1, int fuse, cudaGraphExec_t
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         int rc = launch_step(c, par, div, k1, fuse);
+        c->graph_launches[par][div ? 1 : 0][k1 ? 1 : 0][fuse] = c->launches_per_step;
         cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
         if (rc) { if (e == cudaSuccess) cudaGraphDestroy(graph); return rc; }
         CK(e);
@@ -528,6 +531,7 @@ int get_graph(cs3d_ctx *c, int par, bool div, bool k1, int fuse, cudaGraphExec_t
         CK(e);
     }
     *out = g;
+    c->launches_per_step = c->graph_launches[par][div ? 1 : 0][k1 ? 1 : 0][fuse];
     return CS3D_OK;
 }
 
@@ -986,11 +990,13 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
             if (k1) {
                 k_integrate<<<c->grid_s2, SLOTS, 0, c->stream>>>(c->d);
                 CK(cudaGetLastError());
+                c->launches += 1;
                 k1 = false;
             }
             bool fits = true;
             if ((rc = launch_steps(c, s, m, last, &fits))) return rc;
             if (!fits) { --k; continue; }   // the same step again, by the sequence
+            c->launches += 1;
             c->host_step = s + m - 1;
             k1 = c->any_com;
             c->prekicked = last && !c->any_com;
@@ -1013,6 +1019,7 @@ int cs3d_step(cs3d_ctx *c, int n_steps)
             if ((rc = get_graph(c, par, div, k1, fuse, &g))) return rc;
             CK(cudaGraphLaunch(g, c->stream));
         }
+        c->launches += c->launches_per_step;
         c->host_step = s;
         k1 = fuse == 0;
         c->prekicked = fuse == 2;
@@ -1385,7 +1392,8 @@ int cs3d_get_stats(cs3d_ctx *c, long long *stats, int n)
     std::vector<InstState> st(c->n_inst);
     CK(cudaMemcpyAsync(st.data(), c->d.st, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    long long v[9] = {c->host_step, 0, 0, 0, c->launches_per_step, 0, 0, 0, 0};
+    constexpr int N = 11;
+    long long v[N] = {c->host_step, 0, 0, 0, c->launches_per_step, 0, 0, 0, 0, c->launches, 0};
     for (auto &q : st) v[5] = std::max<long long>(v[5], q.max_halo);
     for (auto &q : st) {
         v[1] += q.rebuilds;
@@ -1394,8 +1402,9 @@ int cs3d_get_stats(cs3d_ctx *c, long long *stats, int n)
         v[6] += q.built;
         v[7] += q.rebuilds_div;
         v[8] += q.searches;
+        v[10] += q.fallbacks;
     }
-    for (int k = 0; k < n && k < 9; ++k) stats[k] = v[k];
+    for (int k = 0; k < n && k < N; ++k) stats[k] = v[k];
     return CS3D_OK;
 }
 

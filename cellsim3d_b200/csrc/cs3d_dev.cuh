@@ -71,6 +71,7 @@ struct InstState {
     int n_large, n_giant;  // cells in its list (d.large): large ones, and those of no class
     int built;             // cells whose lists were built (cumulative)
     int searches;          // of those, the ones for which all cells were looked at
+    int fallbacks;         // and the ones built with the smaller radius of whole builds in a partial one
     int rebuilds;
     int rebuilds_div;      // of those, the ones only the rule for dividing instances called for
     float syscm[3];        // the reference's system centre of mass as of its last

@@ -2385,7 +2385,10 @@ __device__ __forceinline__ void nb_lists(const Dev &d, ListSmem &sm)
         bool full = st->rebuild == 2;
         while (!nb_cell(d, a, node, epoch, full, sm)) {
             full = true;
-            if (t == 0) st->force_rebuild = 1;
+            if (t == 0) {
+                st->force_rebuild = 1;
+                atomicAdd(&st->fallbacks, 1);
+            }
         }
         deal.advance();
     }

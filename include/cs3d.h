@@ -408,15 +408,19 @@ int cs3d_last_error(cs3d_ctx *ctx, int inst, uint32_t *bits);
 
 /* Counters of this library's neighbour lists (no counterpart in the
  * reference): [0] steps, [1] neighbour-list rebuilds, [2] max entries per node
- * seen, [3] max candidate cells per cell seen, [4] kernel launches per step
- * (1 where the steps share one launch),
+ * seen, [3] max candidate cells per cell seen, [4] kernel launches of the
+ * last step (1 where the steps share one launch),
  * [5] max distinct contact-candidate nodes (of other cells) per cell seen
  * (counted only with CS3D_OPT_HALO_STATS, else 0),
  * [6] cell neighbour lists built (cumulative), [7] of the rebuilds [1], those
  * that only the rule for dividing instances called for (more than one cell in
  * 16 divided in the step, with no other cause), [8] of the lists [6], those for
  * which all cells of the instance were looked at (a cell far larger than the
- * mesh at rest, or one with more than 192 others in reach). */
+ * mesh at rest, or one with more than 192 others in reach), [9] kernels that
+ * cs3d_step calls launched (cumulative), [10] of the lists [6], those that a
+ * build around a division made with the radius of a whole build, because the
+ * one it needs gave a node more entries or a cell more candidates than they
+ * have room for. */
 int cs3d_get_stats(cs3d_ctx *ctx, long long *stats, int n);
 
 /* Profiling pass: n_steps steps launched kernel by kernel (not as a graph)

@@ -280,6 +280,7 @@ def test_partial_build_with_more_candidates_than_slots(mesh):
         sim.load_state(st["X"], st["Y"], st["Z"], v, v * 0, v * 0, n_cells=n)
         sim.step(4)
         got.append((sim.state(), sim.events(), sim.forces()))
+        assert (sim.stats()["list_fallbacks"] > 0) == (skin == 0.1)
         sim.close()
     (a, ea, fa), (b, eb, fb) = got
     assert np.array_equal(ea, eb) and ea.tolist() == [[1, 1, n]]
@@ -412,4 +413,64 @@ def test_barrier_limit_option_is_checked(mesh):
     for bad in (-1, 1 << 32):
         with pytest.raises(cs.CS3DError):
             sim.set_option(cs.OPT_SYNC_POLLS, bad)
+    sim.close()
+
+
+def _multiprocessors():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("over", [{}, {"correct_com": 1}, {"add_rands": 1, "rand_scale_factor": 0.1, "rand_seed": 5}])
+@pytest.mark.parametrize("at", [1, 8, "limit", "limit + 1", 300])
+def test_kernels_of_a_step(mesh, over, at):
+    """Which path takes the steps, by the kernels that they launch: one launch
+    for up to 256 steps of a context with at most a cell for each
+    multiprocessor (the first half kick apart, of every launch with the
+    centre-of-mass correction), the sequence of a step beyond; the same for two
+    instances, whose cells add up."""
+    cells = {"limit": _multiprocessors(), "limit + 1": _multiprocessors() + 1}.get(at, at)
+    one = cells <= _multiprocessors()
+    p, st = _growing(cells, growth_rate=0.0, **over)
+    topo = cs.build_topology(cs.mesh_from_arrays(mesh), st["X"][:192], st["Y"][:192], st["Z"][:192])
+    half = cells // 2
+    for parts in ([cells], [half, cells - half]) if half else ([cells],):
+        ens = cs.Ensemble([p] * len(parts), topo, parts)
+        first = 0
+        for k, n in enumerate(parts):
+            ens.load_state(k, *[st[q][first * 192:(first + n) * 192] for q in "XYZ"], n_cells=n)
+            first += n
+        com = bool(over.get("correct_com"))
+        ens.step(300)
+        s = ens.stats()
+        sequence = 5 + (3 if com else 0)   # half kick, centre and shift
+        assert s["launches_per_step"] == (1 if one else sequence)
+        want = 2 + (2 if com else 1) if one else 300 * sequence + (0 if com else 1)
+        assert s["launches"] == want
+        ens.step(2)
+        assert ens.stats()["launches"] - want == (1 + com if one else 2 * sequence)
+        ens.close()
+
+
+def test_growth_out_of_the_one_kernel_path(mesh):
+    """A context that outgrows the one-kernel steps goes on with the sequence, between two launches and between two calls."""
+    n = _multiprocessors() // 2 + 1
+    p, st = _growing(n)
+    sim = _sim(p, st, mesh, capacity=4 * n)
+    sim.step(2)
+    assert sim.n_cells() > _multiprocessors()
+    assert sim.stats()["launches_per_step"] == 1 and sim.stats()["launches"] == 2
+    sim.step(1)
+    assert sim.stats()["launches_per_step"] == 7 and sim.stats()["launches"] == 9
+    sim.close()
+
+
+@pytest.mark.parametrize("skin,some", [(0.1, False), (0.35, True)])
+def test_wide_skin_takes_the_fallback(mesh, skin, some):
+    """The colony of test_partial_builds_do_not_change_results: at a skin of 0.35 some lists are built with the smaller radius."""
+    p, st = _growing(64)
+    sim = _sim(p, st, mesh, capacity=512)
+    sim.set_option(cs.OPT_SKIN, int(round(skin * 1e6)))
+    sim.step(1200)
+    assert (sim.stats()["list_fallbacks"] > 0) == some
     sim.close()
