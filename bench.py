@@ -410,7 +410,7 @@ def run_cs3d(args, world, rank, local):
                          "unit": "GB/s", "frac": achieved / peak,
                          "traffic": S1_TRAFFIC_PER_NODE * n_nodes if args.workload == "packed100k" else None,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_s1 launch "
-                                           "on 30k cells, scaled by nodes (profiles/k_s1_packed30k.md)",
+                                           "on 30k cells, scaled by nodes",
                          "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                          else peak_kind,
                          "algorithmic_bytes_per_node": NODE_BYTES},
