@@ -108,7 +108,7 @@ void free_all(cs3d_ctx *c)
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
 }
 
-// Host copies of the mesh tables: packed neighbours, R0 and 1/R0, theta0
+// Host copies of the mesh tables: packed neighbours, 1/R0, theta0
 // with its FP64 cosine and sine, and the arm table: for node i and each of
 // its neighbours n, the index n*3 + k of the arm force that the angles at
 // vertex n send to i (k = the slot of i in n's neighbour list; the two
@@ -116,7 +116,7 @@ void free_all(cs3d_ctx *c)
 // src/propagate.cu:63-78).
 struct TopoTables {
     double2 cs0[3 * SLOTS];
-    float4 r0[SLOTS], th[SLOTS];
+    float4 th[SLOTS];
     uint4 arm[SLOTS];
     double r0i[3 * SLOTS];
     uint32_t nnp[SLOTS];
@@ -130,7 +130,6 @@ Topo topo_pointers(TopoTables *t)
 {
     Topo T;
     T.nnpack = t->nnp;
-    T.r0 = t->r0;
     T.th0 = t->th;
     T.cs0 = t->cs0;
     T.r0i = t->r0i;
@@ -190,7 +189,6 @@ int topo_tables(const cs3d_topology *t, TopoTables &o)
         int a = t->nn[i], b = t->nn[192 + i], cc = t->nn[384 + i];
         if (a < 0 || a >= NODES || b < 0 || b >= NODES || cc < 0 || cc >= NODES) return CS3D_E_ARG;
         o.nnp[i] = (uint32_t)a | ((uint32_t)b << 8) | ((uint32_t)cc << 16) | ((uint32_t)(uint8_t)(int8_t)t->sign[i] << 24);
-        o.r0[i] = make_float4(t->r0[i], t->r0[192 + i], t->r0[384 + i], 0.f);
         o.th[i] = make_float4(t->theta0[3 * i], t->theta0[3 * i + 1], t->theta0[3 * i + 2], 0.f);
         for (int k = 0; k < 3; ++k) {
             const double th = (double)t->theta0[3 * i + k];

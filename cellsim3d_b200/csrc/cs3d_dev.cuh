@@ -90,7 +90,6 @@ struct DivEntry {
 // Static mesh tables in global memory (7 KB, L1/L2 resident).
 struct Topo {
     uint32_t *nnpack;   // [192] nn0 | nn1<<8 | nn2<<16 | (sign&0xff)<<24
-    float4 *r0;         // [192] equilibrium lengths to nn0..2
     float4 *th0;        // [192] aij, ajk, aik
     double2 *cs0;       // [192*3] (cos, sin) of aij, ajk, aik in FP64
     double *r0i;        // [192*3] 1/R0 in FP64
