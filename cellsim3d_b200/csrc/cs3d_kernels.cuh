@@ -812,7 +812,7 @@ __device__ __forceinline__ void geom_box(const GeomScratch &gs, float4 &lo, floa
     }
 }
 
-// sqrt(x) to within an ulp: the approximate inverse root, refined once (to 1e-12),
+// sqrt(x) to half an ulp: the approximate inverse root, refined once (to 1e-12),
 // then Heron's step by the exact remainder.  Zero, values that the approximation
 // does not reach and those that are no finite numbers take the full root.
 __device__ __forceinline__ double sqrt_full(double x)

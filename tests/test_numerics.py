@@ -77,3 +77,72 @@ def test_one_newton_step_on_1e6_seeds():
         worst_c = max(worst_c, abs(float((Fr(float(r1)) - c) / c)))
     assert worst_r < 2e-12, worst_r
     assert worst_c < 2e-12, worst_c
+
+
+def _fma32(a, b, c):
+    """fma of float32 arrays: the product is exact in float64; where the float64
+    sum lies at a tie of float32 (its rounding may have moved it there), the
+    exact sum decides."""
+    p = a.astype(np.float64) * b.astype(np.float64)
+    s = p + c.astype(np.float64)
+    out = s.astype(np.float32)
+    bits = s.view(np.uint64) & np.uint64((1 << 29) - 1)
+    for k in np.flatnonzero(bits == np.uint64(1 << 28)):
+        exact = Fr(float(p[k])) + Fr(float(c[k]))
+        near = [np.nextafter(out[k], np.float32(d)) for d in (-np.inf, np.inf)] + [out[k]]
+        dist = [abs(Fr(float(v)) - exact) for v in near]
+        best = min(dist)
+        ties = [v for v, d in zip(near, dist) if d == best]
+        out[k] = ties[0] if len(ties) == 1 else next(v for v in ties if not int(np.float32(v).view(np.uint32)) & 1)
+    return out
+
+
+def test_bin_quotient_is_the_ieee_quotient_for_every_significand():
+    """x / 2.9 of the grid bins (div_dl): the product with the rounded
+    reciprocal corrected once by the remainder, against the IEEE division over
+    all 2^23 significands of one binade (the operations scale with the exponent)
+    and both signs."""
+    dl = np.float32(2.9)
+    r = np.float32(1.0) / dl
+    x = (np.arange(1 << 23, dtype=np.uint32) + np.uint32(0x3f800000)).view(np.float32)
+    for x in (x, -x):
+        q = x * r
+        e = _fma32(-q, np.full_like(q, dl), x)
+        assert np.array_equal(_fma32(e, np.full_like(q, r), q), x / dl)
+        assert (q != x / dl).any()   # the correction is not idle
+
+
+def test_division_by_180_is_the_correctly_rounded_quotient():
+    """t / 180 of the centres of mass (div_nodes): the sums of 180 float
+    coordinates, in float64."""
+    rng = random.Random(180)
+    r, n = 1.0 / 180.0, 0
+    for _ in range(6000):
+        t = float(F(rng.choice([1.0, -1.0])) * F(180.0 * 10.0 ** rng.uniform(-6, 5)))
+        if rng.random() < 0.5:
+            t = float(np.float32(t))
+        q = float(F(t) * F(r))
+        q2 = fma(fma(-q, 180.0, t), r, q)
+        assert q2 == rn(Fr(t) / 180), t
+        n += q != q2
+    assert n > 0
+
+
+def test_square_root_of_the_triangle_areas():
+    """sqrt_full: an inverse root of relative error 2e-12 (the seed after its
+    Newton step) times x, and Heron's step by the exact remainder.  The error
+    before the last rounding is the square of the seed's, so that the result is
+    within half an ulp, 2^-53 relative, and a millionth of that."""
+    from decimal import Decimal, getcontext
+    getcontext().prec = 60
+    rng = random.Random(11)
+    worst = 0.0
+    for _ in range(3000):
+        x = 10.0 ** rng.uniform(-270, 270) if rng.random() < 0.3 else 10.0 ** rng.uniform(-12, 8)
+        t = _decimal_rsqrt(x)
+        r = float(t * (1 + Fr(rng.choice([2e-12, -2e-12, rng.uniform(-2e-12, 2e-12)]))))
+        s = float(F(x) * F(r))
+        got = fma(float(F(0.5) * F(r)), fma(-s, s, x), s)
+        root = Fr(Decimal(x).sqrt())
+        worst = max(worst, abs(float((Fr(got) - root) / root)))
+    assert worst <= 2.0 ** -53 * (1 + 1e-6), worst * 2.0 ** 53
