@@ -475,9 +475,10 @@ int launch_step(cs3d_ctx *c, int par, bool div, bool k1 = true, int fuse = 0, co
 }
 
 // Systems of up to one cell for each SM take their steps in k_steps (us a step,
-// this kernel against the launch sequence: 1 growing cell 17.5 / 26.1, 8 cells
-// 27.8 / 34.7, 64 39.0 / 43.2, 150 47.2 / 49.4, 300 56.7 / 56.4; beyond that
-// its fixed four CTAs an SM cost more than the launches).
+// this kernel against the launch sequence: 1 growing cell 16.1 / 22.9, 8 cells
+// 26.3 / 30.1, 64 36.0 / 39.0, 150 44.0 / 44.1, 300 52.7 / 51.0; 148 packed ones
+// 21.1 / 22.3); beyond that the fixed four CTAs an SM cost growing systems more
+// than the launches.
 bool in_one_kernel(const cs3d_ctx *c) { return c->grid_steps > 0 && c->n_now <= c->nsm; }
 // After a launch the host looks at the cell counts again.
 constexpr int STEPS_PER_LAUNCH = 256;

@@ -271,7 +271,11 @@ int cs3d_create_ensemble(int n_inst, const cs3d_params *params, const cs3d_topol
  * V*, pressure and youngs may be NULL (zeros, min_pressure, stiffness1 --
  * the reference's defaults, src/GPUbounce.cu:449-451, :867-871, :617-620).
  * The initial centre of mass, grid and first force evaluation
- * (src/GPUbounce.cu:739-763, :978-1004) run before the next step or read. */
+ * (src/GPUbounce.cu:739-763, :978-1004) run before the next step or read.
+ * The arrays are free to change when the call returns.  Up to 256 KB it does
+ * not wait for the device, so that an error of the device from the copy or from
+ * earlier work is returned by the next call that does: every step and every read of
+ * an array.  The RANMAR state stays as it is. */
 int cs3d_load_state(cs3d_ctx *ctx, int inst, int n_cells, const float *X, const float *Y,
                     const float *Z, const float *VX, const float *VY, const float *VZ,
                     const float *pressure, const float *youngs);
@@ -279,7 +283,8 @@ int cs3d_load_state(cs3d_ctx *ctx, int inst, int n_cells, const float *X, const 
 /* Replace the RANMAR state of instance inst (e.g. after host-side draws
  * for random placement).  The reference keeps one RANMAR state per process
  * in file-scope variables (src/marsaglia.h:50-51); an ensemble has one per
- * instance, so it is set and read through these two calls. */
+ * instance, so it is set and read through these two calls.  cs3d_set_rng does
+ * not wait for the device (as cs3d_load_state). */
 int cs3d_set_rng(cs3d_ctx *ctx, int inst, const cs3d_rng *rng);
 /* Current RANMAR state of instance inst (the stream the divisions draw from). */
 int cs3d_get_rng(cs3d_ctx *ctx, int inst, cs3d_rng *rng);
@@ -306,7 +311,8 @@ int cs3d_set_skin_schedule(cs3d_ctx *ctx, int n, const int *min_cells, const flo
  * error bit (see cs3d_last_error). */
 int cs3d_step(cs3d_ctx *ctx, int n_steps);
 
-/* Read back instance inst.  Any output pointer may be NULL.  Replaces the
+/* Read back instance inst.  Any output pointer may be NULL; the cell count alone
+ * is known on the host and does not wait for the device.  Replaces the
  * device-to-host copies before a trajectory frame and the force file,
  * src/GPUbounce.cu:1447-1449 and :1458-1471. */
 int cs3d_get_state(cs3d_ctx *ctx, int inst, int *n_cells, float *X, float *Y, float *Z,
