@@ -442,6 +442,11 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
                 }
                 ss.res[0][lane] = k;
                 ss.res[1][lane] = ex; ss.res[2][lane] = ey; ss.res[3][lane] = ez;
+                // a pair with a node that is no number counts for the friction only
+                // and must not get into F: k = 0 times 0 (the owner leaving out pairs
+                // with k = 0 makes the steps of 8 cells 1.3 % slower, zeros chosen
+                // before the stores S1 of packed cells 1 %)
+                if (r2 != r2) ss.res[1][lane] = ss.res[2][lane] = ss.res[3][lane] = 0.0;
                 // velocity differences of floats are exact in FP64
                 ss.res[4][lane] = (double)vo.x - vj.x;
                 ss.res[5][lane] = (double)vo.y - vj.y;
@@ -455,14 +460,10 @@ __device__ __forceinline__ int sweep_s1(const Dev &d, const InstParams &P, const
                 mine &= mine - 1u;
                 if (nd < MAXD) dl[(size_t)nd * SLOTS] = (uint16_t)ss.item[b + q];
                 ++nd;
-                // 0 also where the pair is a dissipative one only: at the cut-off,
-                // or with a node that is no number, which must not get into F
                 const double k = ss.res[0][q];
-                if (k != 0.0) {
-                    FX = fma(k, ss.res[1][q], FX);
-                    FY = fma(k, ss.res[2][q], FY);
-                    FZ = fma(k, ss.res[3][q], FZ);
-                }
+                FX = fma(k, ss.res[1][q], FX);
+                FY = fma(k, ss.res[2][q], FY);
+                FZ = fma(k, ss.res[3][q], FZ);
                 vsum.x += ss.res[4][q]; vsum.y += ss.res[5][q]; vsum.z += ss.res[6][q];
             }
             __syncwarp();
@@ -636,7 +637,7 @@ __device__ __forceinline__ void assign_hash_slices(const Dev &d)
             if (st->rebuild) {
                 bits = 6;
                 while ((1ll << bits) < 2ll * st->n) ++bits;
-                for (int q = 0; q < LEVELS * 3; ++q) st->hmax[q / 3][q % 3] = 0u;
+                for (int q = 0; q <= st->top; ++q) st->hmax[q][0] = st->hmax[q][1] = st->hmax[q][2] = 0u;
                 st->top = st->n_large = st->n_giant = 0;
                 size = 1 << bits;
             }
@@ -2158,42 +2159,47 @@ __device__ __forceinline__ void cells_in_reach(const Dev &d, const InstParams &P
         if (cell_near(d, P, a, lo, hi, full, da, c, d.nbox[2 * c], d.nbox[2 * c + 1])) take(c);
     };
     const float r = list_radius(P, full, da, st->ds) * BOX_REACH;
-    const int top = st->top;
-    for (int k = 0; k <= top; ++k) {
-        if (st->hmax[k][0] == 0u) continue;   // no cells
-        // the centre of a box in reach lies within r + its half extent of this
-        // box; a thousandth more covers the rounding of the bounds
-        const float inv = class_inv(P.inv_bin, k);
-        const float ex = (r + __uint_as_float(st->hmax[k][0])) * 1.001f, ey = (r + __uint_as_float(st->hmax[k][1])) * 1.001f,
-                    ez = (r + __uint_as_float(st->hmax[k][2])) * 1.001f;
-        const int x0 = bin_coord(lo.x - ex, inv), y0 = bin_coord(lo.y - ey, inv), z0 = bin_coord(lo.z - ez, inv);
-        const long long nx = bin_coord(hi.x + ex, inv) - x0 + 1ll, ny = bin_coord(hi.y + ey, inv) - y0 + 1ll,
-                        nz = bin_coord(hi.z + ez, inv) - z0 + 1ll;
-        // A cell whose nodes are all NaN along an axis has no box (lo 1e30, hi
-        // -1e30) and reaches nothing: the bins of its ranges come out negative,
-        // and their product wraps to some 1e9.
-        if (nx <= 0 || ny <= 0 || nz <= 0) return;
-        if (nx > 64 || ny > 64 || nz > 64 || nx * ny * nz > 4096) {   // far larger than the class
-            if (t == 0) atomicAdd(&sm.n, MAXB + 1);
-            return;
-        }
-        const int nyz = (int)(ny * nz), nb = (int)nx * nyz;
-        for (int q = t; q < nb; q += SLOTS) {
-            const int ix = x0 + q / nyz, iy = y0 + (q % nyz) / (int)nz, iz = z0 + q % (int)nz;
-            const unsigned long long h = d.bins[bin_slot(*st, k, ix, iy, iz)];
-            int c = (unsigned)(h >> 32) == epoch ? (int)(unsigned)h : -1;
-            while (c >= 0) {
-                const int nxt = d.bnext[c];
-                const float4 l = d.nbox[2 * c], g = d.nbox[2 * c + 1];
-                // bins share table entries: only the cells of this very bin
-                if (cell_near(d, P, a, lo, hi, full, da, c, l, g) && box_bin(l.x, g.x, inv) == ix &&
-                    box_bin(l.y, g.y, inv) == iy && box_bin(l.z, g.z, inv) == iz && (top == 0 || box_level(l, g, P.inv_bin) == k))
-                    take(c);
-                c = nxt;
+    const int top = st->top, nl = min(st->n_large, MAXL), ng = st->n_giant;
+    // largest half extents of the class
+    unsigned hx = st->hmax[0][0], hy = st->hmax[0][1], hz = st->hmax[0][2];
+    for (int k = 0;;) {
+        if (hx != 0u) {   // some cells
+            // the centre of a box in reach lies within r + its half extent of this
+            // box; a thousandth more covers the rounding of the bounds
+            const float inv = class_inv(P.inv_bin, k);
+            const float ex = (r + __uint_as_float(hx)) * 1.001f, ey = (r + __uint_as_float(hy)) * 1.001f,
+                        ez = (r + __uint_as_float(hz)) * 1.001f;
+            const int x0 = bin_coord(lo.x - ex, inv), y0 = bin_coord(lo.y - ey, inv), z0 = bin_coord(lo.z - ez, inv);
+            const long long nx = bin_coord(hi.x + ex, inv) - x0 + 1ll, ny = bin_coord(hi.y + ey, inv) - y0 + 1ll,
+                            nz = bin_coord(hi.z + ez, inv) - z0 + 1ll;
+            // A cell whose nodes are all NaN along an axis has no box (lo 1e30, hi
+            // -1e30) and reaches nothing: the bins of its ranges come out negative,
+            // and their product wraps to some 1e9.
+            if (nx <= 0 || ny <= 0 || nz <= 0) return;
+            if (nx > 64 || ny > 64 || nz > 64 || nx * ny * nz > 4096) {   // far larger than the class
+                if (t == 0) atomicAdd(&sm.n, MAXB + 1);
+                return;
+            }
+            const int nyz = (int)(ny * nz), nb = (int)nx * nyz;
+            for (int q = t; q < nb; q += SLOTS) {
+                const int ix = x0 + q / nyz, iy = y0 + (q % nyz) / (int)nz, iz = z0 + q % (int)nz;
+                const unsigned long long h = d.bins[bin_slot(*st, k, ix, iy, iz)];
+                int c = (unsigned)(h >> 32) == epoch ? (int)(unsigned)h : -1;
+                while (c >= 0) {
+                    const int nxt = d.bnext[c];
+                    const float4 l = d.nbox[2 * c], g = d.nbox[2 * c + 1];
+                    // bins share table entries: only the cells of this very bin
+                    if (cell_near(d, P, a, lo, hi, full, da, c, l, g) && box_bin(l.x, g.x, inv) == ix &&
+                        box_bin(l.y, g.y, inv) == iy && box_bin(l.z, g.z, inv) == iz &&
+                        (top == 0 || box_level(l, g, P.inv_bin) == k))
+                        take(c);
+                    c = nxt;
+                }
             }
         }
+        if (++k > top) break;
+        hx = st->hmax[k][0]; hy = st->hmax[k][1]; hz = st->hmax[k][2];
     }
-    const int nl = min(st->n_large, MAXL), ng = st->n_giant;
     for (int q = t; q < nl; q += SLOTS) take_if_near(d.large[P.base + q]);
     for (int q = t; q < ng; q += SLOTS) take_if_near(d.large[P.base + P.cap - 1 - q]);
 }
